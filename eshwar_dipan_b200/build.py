@@ -23,10 +23,14 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 INC = ["-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 
 HOST_C = ["gp_host.c", "gp_host_io.c"]
-# (file, extra nvcc flags): the FP64 unit stays without FMA contraction so the
-# plain step is bit-identical to the reference; the FP32 storage form may fuse.
-CUDA = [("gp_device.cu", ["--fmad=false"]), ("gp_batch32.cu", ["--fmad=true"]),
-        ("gp_adjoint.cu", ["--fmad=false"])]
+# (object, file, extra nvcc flags): the FP64 units stay without FMA contraction
+# so the plain step is bit-identical to the reference; the FP32 storage form may
+# fuse.  The step kernels compile once per field type and system size.
+SIZES = [(2, 1), (3, 1), (4, 1), (2, 2), (3, 2), (4, 2)]
+CUDA = [("gp_device.cu.o", "gp_device.cu", ["--fmad=false"]), ("gp_adjoint.cu.o", "gp_adjoint.cu", ["--fmad=false"])]
+CUDA += [("gp_kernels_%s_%d_%d.o" % (r, n, k), "gp_kernels.cu",
+          ["--fmad=%s" % fmad, "-DGP_R=" + r, "-DGP_N=%d" % n, "-DGP_K=%d" % k])
+         for r, fmad in (("double", "false"), ("float", "true")) for n, k in reversed(SIZES)]
 
 
 def _run(cmd, verbose):
@@ -59,8 +63,8 @@ def build(verbose=False, ptxas_info=False):
                   "-Wno-unused-function", *INC, "-c", src, "-o", obj], verbose)
         objs.append(obj)
     jobs = []
-    for f, flags in CUDA:
-        src, obj = os.path.join(CSRC, f), os.path.join(BUILD, f + ".o")
+    for o, f, flags in CUDA:
+        src, obj = os.path.join(CSRC, f), os.path.join(BUILD, o)
         if _stale(obj, [src] + headers) or ptxas_info:
             cmd = [NVCC, *ARCH, "-lineinfo", "-O3", *flags, "-std=c++17", "-Xcompiler", "-fPIC",
                    "-Xcompiler", "-ffp-contract=off", *INC, "-c", src, "-o", obj]
@@ -69,7 +73,7 @@ def build(verbose=False, ptxas_info=False):
             jobs.append(cmd)
         objs.append(obj)
     # the CUDA translation units are independent: compile them side by side
-    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
         for r in pool.map(lambda c: _run(c, verbose), jobs):
             if ptxas_info and r.stderr:
                 sys.stderr.write(r.stderr)

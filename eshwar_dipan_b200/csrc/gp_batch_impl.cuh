@@ -1,8 +1,8 @@
 /*
  * gp_batch_impl.cuh -- launchers of the batched kernels for one field type.
- * Included by gp_device.cu (FP64, compiled without FMA contraction so that it
- * stays bit-identical to the reference) and gp_batch32.cu (FP32 storage form,
- * compiled with FMA contraction).  Each exposes a BatchLaunch table.
+ * Instantiated by gp_kernels.cu, one translation unit per field type and
+ * system size (FP64 without FMA contraction, so that it stays bit-identical to
+ * the reference; the FP32 storage form with it); each gives a BatchLaunch table.
  */
 #pragma once
 #include <cuda_runtime.h>
@@ -200,20 +200,15 @@ struct BatchKernels {
   }
 };
 
-template <typename R>
-bool batch_launch_table(int N, int K, bool A, BatchLaunch *out) {
-#define GP_CASE(n, k)                                                                                   \
-  if (N == n && K == k) {                                                                               \
-    *out = A ? BatchKernels<R, n, k, true>::table() : BatchKernels<R, n, k, false>::table();            \
-    return true;                                                                                        \
-  }
-  GP_CASE(2, 1) GP_CASE(3, 1) GP_CASE(4, 1) GP_CASE(2, 2) GP_CASE(3, 2) GP_CASE(4, 2)
-#undef GP_CASE
-  return false;
-}
-
 }  // namespace gpd
 
-/* defined in gp_device.cu (FP64) and gp_batch32.cu (FP32) */
-bool gp_batch_launch_f64(int N, int K, bool aniso, gpd::BatchLaunch *out);
-bool gp_batch_launch_f32(int N, int K, bool aniso, gpd::BatchLaunch *out);
+/* The launch tables by field type and system size: gp_kernels.cu, one
+ * translation unit per (type, NUMPHASES, components), so that they compile
+ * side by side. */
+#define GP_TABLE_NAME2(r, n, k) gp_batch_table_##r##_##n##_##k
+#define GP_TABLE_NAME(r, n, k) GP_TABLE_NAME2(r, n, k)
+#define GP_FOR_SIZES(X, r) X(r, 2, 1) X(r, 3, 1) X(r, 4, 1) X(r, 2, 2) X(r, 3, 2) X(r, 4, 2)
+#define GP_DECLARE_TABLE(r, n, k) gpd::BatchLaunch GP_TABLE_NAME(r, n, k)(bool aniso);
+GP_FOR_SIZES(GP_DECLARE_TABLE, double)
+GP_FOR_SIZES(GP_DECLARE_TABLE, float)
+#undef GP_DECLARE_TABLE

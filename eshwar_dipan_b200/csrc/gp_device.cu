@@ -7,7 +7,7 @@
  *  - gp_batch: simulations of different sizes and parameters stepped together
  *    by two kernels per step (bulk tiles, then interface tiles from a device
  *    work list), in FP64 (bit-identical to the reference step) or in the FP32
- *    storage form (gp_batch32.cu); steps are replayed as CUDA graphs of
+ *    storage form (both in gp_kernels.cu); steps are replayed as CUDA graphs of
  *    GP_GRAPH_STEPS steps.
  *  - gp_ctx: one simulation, a batch of one.
  *  - gp_step_noalloc: one FP64 step on caller-owned buffers, two-pass kernels
@@ -247,10 +247,21 @@ bool pick(int N, int K, bool A, Kern *out) {
 
 }  // namespace
 
-bool gp_batch_launch_f64(int N, int K, bool aniso, gpd::BatchLaunch *out) {
-  return gpd::batch_launch_table<double>(N, K, aniso, out);
+/* the launch table of a system size; false where no kernel exists */
+static bool batch_launch(gp_precision prec, int N, int K, bool aniso, gpd::BatchLaunch *out) {
+#define GP_CASE(r, n, k)                    \
+  if (N == n && K == k) {                   \
+    *out = GP_TABLE_NAME(r, n, k)(aniso);   \
+    return true;                            \
+  }
+  if (prec == GP_FP64) {
+    GP_FOR_SIZES(GP_CASE, double)
+  } else {
+    GP_FOR_SIZES(GP_CASE, float)
+  }
+#undef GP_CASE
+  return false;
 }
-
 
 struct gp_batch;
 
@@ -1011,9 +1022,7 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
                                        "Function_anisotropy from simulation 0", s);
     }
   }
-  bool ok = prec == GP_FP64 ? gp_batch_launch_f64(b->N, b->K, b->aniso != 0, &b->L)
-                            : gp_batch_launch_f32(b->N, b->K, b->aniso != 0, &b->L);
-  if (!ok) {
+  if (!batch_launch(prec, b->N, b->K, b->aniso != 0, &b->L)) {
     delete b;
     return bfail(nullptr, GP_EINVAL, "gp_batch_create: no kernel for N=%d K=%d", b->N, b->K);
   }
