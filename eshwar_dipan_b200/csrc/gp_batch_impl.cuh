@@ -12,31 +12,44 @@
 
 namespace gpd {
 
+/* What one step's kernels are launched with.  mul: every simulation's spacings
+ * are powers of two (x/dx == x*(1/dx)); diag: every phase's off-diagonal D, c_mu
+ * and A are zero and no E is -0 (those terms are left out); tg: some simulation is
+ * non-isothermal; solo: a batch of one's StepArgs (host memory), or NULL. */
+struct StepLaunch {
+  cudaStream_t stream;
+  int grid;
+  bool mul, diag, tg;
+  const void *solo;
+  const SimDesc *sims;
+  const void *consts;
+  const int4 *blist, *glist;
+  const TensorMapSlot *tmaps;   /* per simulation and state buffer the maps MAP_MU and MAP_ALL */
+  int buf;                      /* the buffer `state` is */
+  const void *state;
+  void *next;
+  TileFlags *flag_out;
+  int *ctr;
+  int ndone;                    /* the CTAs of this step's kernels together */
+  StatBufs st;
+};
+
 struct BatchLaunch {
-  /* occupancy of the bulk and interface kernels (blocks per SM) */
-  cudaError_t (*prepare)(int *blocks_per_sm_bulk, int *blocks_per_sm_general);
-  /* one step: bulk tiles + interface list, then the interface tiles */
-  /* flag_out: the flags of the buffer the step writes (copied into the bulk entries) */
+  /* set up the kernels a batch with these launch options takes (mul, diag, tg and
+   * solo of l) and give the blocks per SM of its kf_bulk, kf_general and kf_step */
+  cudaError_t (*prepare)(const StepLaunch &l, int *bulk, int *general, int *step);
+  /* the bulk and interface lists of a step; flag_out: the flags of the buffer it
+   * writes (copied into the bulk entries) */
   cudaError_t (*classify)(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
-                          const TileFlags *flag_in, const TileFlags *flag_out, int *glist, int4 *blist, int *ctr);
-  /* mul: every simulation's spacings are powers of two (x/dx == x*(1/dx)) */
-  /* ndone: the CTAs of this step's kf_bulk and kf_general together */
-  /* tmaps: per simulation two tensor maps of its mu planes (state buffer 0
-   * and 1); buf: the buffer `state` is; diag: every phase's off-diagonal D,
-   * c_mu and A are zero and no E is -0 (the bulk kernel leaves those terms
-   * out) */
-  cudaError_t (*bulk)(int grid, bool mul, bool diag, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
-                      const int4 *blist, const TensorMapSlot *tmaps, int buf, const void *state, void *next,
-                      TileFlags *flag_out, int *ctr, int ndone, StatBufs st);
+                          const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist, int4 *blist, int *ctr);
+  cudaError_t (*bulk)(const StepLaunch &l);
+  cudaError_t (*general)(const StepLaunch &l);
   /* bulk and interface tiles in one launch (kf_step; not for a sums step) */
-  cudaError_t (*step)(int grid, bool mul, bool diag, cudaStream_t s, const SimDesc *sims, const void *consts,
-                      const int *tsim, const int4 *blist, const int *glist, const TensorMapSlot *tmaps, int buf,
-                      const void *state, void *next, TileFlags *flag_out, int *ctr, int ndone, StatBufs st);
-  /* blocks per SM of kf_step */
-  int (*step_occupancy)();
-  cudaError_t (*general)(int grid, bool mul, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
-                         const void *state, void *next, TileFlags *flag_out, const int *glist, int *ctr, int ndone,
-                         StatBufs st);
+  cudaError_t (*step)(const StepLaunch &l);
+  /* the StepArgs of a batch of one (FP32: none, every batch takes the same kernels,
+   * since another kernel's fused multiply-adds could round differently) */
+  size_t solo_bytes;
+  void (*solo_fill)(void *dst, const void *consts, const SimDesc *sd);
   cudaError_t (*flags)(int ntiles, cudaStream_t s, const SimDesc *sims, const int *tsim, const void *state,
                        TileFlags *flags);
   /* one smoothing sweep of a simulation (tcc: its temperature rows, or NULL) */
@@ -57,101 +70,104 @@ struct BatchLaunch {
 template <typename R, int N, int K, bool A>
 struct BatchKernels {
   static constexpr size_t bulk_smem = bulk_smem_bytes<R, K>();
-  static constexpr size_t step_smem =
-      sizeof(GenSmem<R, N, K>) > bulk_smem ? sizeof(GenSmem<R, N, K>) : bulk_smem;
-  template <bool MUL, bool DIAG>
-  static cudaError_t step_attr() {
-    return cudaFuncSetAttribute(kf_step<R, N, K, A, MUL, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)step_smem);
+  static constexpr size_t item_smem = sizeof(TileSmem<R, N, K, A>);
+  static constexpr size_t step_smem = item_smem > bulk_smem ? item_smem : bulk_smem;
+  /* Kernel variants: MUL only where it can differ (FP32 always multiplies), DIAG
+   * only where there are off-diagonal terms, SOLO in FP64 only; a non-isothermal
+   * batch takes the TG kernels, which read each simulation's constants from global
+   * memory.  f(kernel) is called with the one a launch takes. */
+  static constexpr bool DIV = sizeof(R) == 8, SOLO = sizeof(R) == 8;
+  static const StepArgs<R, true> &solo_of(const StepLaunch &l) {
+    return *reinterpret_cast<const StepArgs<R, true> *>(l.solo);
   }
-  static int step_occupancy() {
-    int n = 0;
-    if (step_attr<true, false>() != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kf_step<R, N, K, A, true, false>, NT, step_smem) !=
-            cudaSuccess)
-      return 0;
-    return n;
+  static void solo_fill(void *dst, const void *consts, const SimDesc *sd) {
+    StepArgs<R, true> *a = reinterpret_cast<StepArgs<R, true> *>(dst);
+    a->c = *reinterpret_cast<const Consts<R> *>(consts);
+    a->sd = *sd;
   }
-  static cudaError_t step(int grid, bool mul, bool diag, cudaStream_t s, const SimDesc *sims, const void *consts,
-                          const int *tsim, const int4 *blist, const int *glist, const TensorMapSlot *tmaps, int buf,
-                          const void *state, void *next, TileFlags *flag_out, int *ctr, int ndone, StatBufs st) {
-#define GP_STEP(MUL, DIAG)                                                                                      \
-  kf_step<R, N, K, A, MUL, DIAG><<<grid, NT, step_smem, s>>>(sims, (const Consts<R> *)consts, tsim, blist, glist,  \
-                                                             tmaps, buf, (const R *)state, (R *)next, flag_out, ctr, \
-                                                             ndone, st)
-    if (diag) {
-      if (mul) GP_STEP(true, true);
-      else GP_STEP(false, true);
+  template <bool MUL, bool DIAG, typename F>
+  static void with_step_md(const StepLaunch &l, F &&f) {
+    if (l.tg) f(kf_step<R, N, K, A, MUL, true, false, false>, StepArgs<R, false>{});
+    else if (SOLO && l.solo) f(kf_step<R, N, K, A, MUL, false, SOLO, DIAG>, pick_args(l));
+    else f(kf_step<R, N, K, A, MUL, false, false, DIAG>, StepArgs<R, false>{});
+  }
+  static decltype(auto) pick_args(const StepLaunch &l) {
+    if constexpr (SOLO) return (solo_of(l));
+    else return StepArgs<R, false>{};
+  }
+  template <typename F>
+  static void with_step(const StepLaunch &l, F &&f) {
+    constexpr bool KD = K > 1;
+    if (DIV && !l.mul) {
+      if (KD && l.diag) with_step_md<!DIV, KD>(l, f);
+      else with_step_md<!DIV, false>(l, f);
     } else {
-      if (mul) GP_STEP(true, false);
-      else GP_STEP(false, false);
+      if (KD && l.diag) with_step_md<true, KD>(l, f);
+      else with_step_md<true, false>(l, f);
     }
-#undef GP_STEP
+  }
+  template <bool MUL, typename F>
+  static void with_general_m(const StepLaunch &l, F &&f) {
+    if (l.tg) f(kf_general<R, N, K, A, MUL, true, false>, StepArgs<R, false>{});
+    else if (SOLO && l.solo) f(kf_general<R, N, K, A, MUL, false, SOLO>, pick_args(l));
+    else f(kf_general<R, N, K, A, MUL, false, false>, StepArgs<R, false>{});
+  }
+  template <typename F>
+  static void with_general(const StepLaunch &l, F &&f) {
+    if (DIV && !l.mul) with_general_m<!DIV>(l, f);
+    else with_general_m<true>(l, f);
+  }
+  template <bool MUL, typename F>
+  static void with_bulk_m(const StepLaunch &l, bool sums, F &&f) {
+    constexpr bool KD = K > 1;
+    /* the sums step (last of a call) takes every term: same results */
+    if (sums) f(kf_bulk<R, N, K, true, MUL, false>);
+    else if (KD && l.diag) f(kf_bulk<R, N, K, false, MUL, KD>);
+    else f(kf_bulk<R, N, K, false, MUL, false>);
+  }
+  template <typename F>
+  static void with_bulk(const StepLaunch &l, bool sums, F &&f) {
+    if (DIV && !l.mul) with_bulk_m<!DIV>(l, sums, f);
+    else with_bulk_m<true>(l, sums, f);
+  }
+  static cudaError_t step(const StepLaunch &l) {
+    with_step(l, [&](auto k, const auto &args) {
+      k<<<l.grid, NTI, step_smem, l.stream>>>(args, l.sims, (const Consts<R> *)l.consts, l.blist, l.glist, l.tmaps, l.buf,
+                                              (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
+    });
     return cudaGetLastError();
   }
-  template <bool SUMS, bool MUL, bool DIAG>
-  static cudaError_t bulk_attr() {
-    return cudaFuncSetAttribute(kf_bulk<R, N, K, SUMS, MUL, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)bulk_smem);
+  static cudaError_t bulk(const StepLaunch &l) {
+    with_bulk(l, l.st.want_sums != 0, [&](auto k) {
+      k<<<l.grid, NTI, bulk_smem, l.stream>>>(l.sims, (const Consts<R> *)l.consts, l.blist, l.tmaps, l.buf,
+                                              (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
+    });
+    return cudaGetLastError();
   }
-  static cudaError_t prepare(int *bb, int *bg) {
-    cudaError_t e = cudaFuncSetAttribute(kf_general<R, N, K, A, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(GenSmem<R, N, K>));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kf_general<R, N, K, A, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(GenSmem<R, N, K>));
-    if (e == cudaSuccess) e = bulk_attr<false, false, false>();
-    if (e == cudaSuccess) e = bulk_attr<false, true, false>();
-    if (e == cudaSuccess) e = bulk_attr<false, false, true>();
-    if (e == cudaSuccess) e = bulk_attr<false, true, true>();
-    if (e == cudaSuccess) e = bulk_attr<true, false, false>();
-    if (e == cudaSuccess) e = bulk_attr<true, true, false>();
-    if (e == cudaSuccess) e = step_attr<false, false>();
-    if (e == cudaSuccess) e = step_attr<true, false>();
-    if (e == cudaSuccess) e = step_attr<false, true>();
-    if (e == cudaSuccess) e = step_attr<true, true>();
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bb, kf_bulk<R, N, K, false, true, false>, NT, bulk_smem);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bg, kf_general<R, N, K, A, true>, NT,
-                                                         sizeof(GenSmem<R, N, K>));
+  static cudaError_t general(const StepLaunch &l) {
+    with_general(l, [&](auto k, const auto &args) {
+      k<<<l.grid, NTI, item_smem, l.stream>>>(args, l.sims, (const Consts<R> *)l.consts, l.tmaps, l.buf,
+                                              (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.ctr, l.ndone, l.st);
+    });
+    return cudaGetLastError();
+  }
+  static cudaError_t prepare(const StepLaunch &l, int *bb, int *bg, int *bs) {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto k, size_t smem, int *blocks) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess && blocks) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, NTI, smem);
+    };
+    with_bulk(l, false, [&](auto k) { set(k, bulk_smem, bb); });
+    with_bulk(l, true, [&](auto k) { set(k, bulk_smem, nullptr); });
+    with_general(l, [&](auto k, const auto &) { set(k, item_smem, bg); });
+    with_step(l, [&](auto k, const auto &) { set(k, step_smem, bs); });
+    return e;
   }
   static cudaError_t classify(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts,
-                              const int *tsim, const TileFlags *flag_in, const TileFlags *flag_out, int *glist,
+                              const int *tsim, const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist,
                               int4 *blist, int *ctr) {
     kf_classify<R><<<(ntiles + NTC - 1) / NTC, NTC, 0, s>>>(sims, (const Consts<R> *)consts, tsim, ntiles, flag_in, flag_out, glist,
                                                          blist, ctr);
-    return cudaGetLastError();
-  }
-  static cudaError_t bulk(int grid, bool mul, bool diag, cudaStream_t s, const SimDesc *sims, const void *consts,
-                          const int *tsim, const int4 *blist, const TensorMapSlot *tmaps, int buf,
-                          const void *state, void *next, TileFlags *flag_out, int *ctr, int ndone, StatBufs st) {
-#define GP_BULK(SUMS, MUL, DIAG)                                                                               \
-  kf_bulk<R, N, K, SUMS, MUL, DIAG><<<grid, NT, bulk_smem, s>>>(sims, (const Consts<R> *)consts, tsim, blist, tmaps,  \
-                                                          buf, (const R *)state, (R *)next, flag_out, ctr, ndone, st)
-    /* the sums step (last of a call) takes every term: same results */
-    if (st.want_sums) {
-      if (mul) GP_BULK(true, true, false);
-      else GP_BULK(true, false, false);
-    } else if (diag) {
-      if (mul) GP_BULK(false, true, true);
-      else GP_BULK(false, false, true);
-    } else {
-      if (mul) GP_BULK(false, true, false);
-      else GP_BULK(false, false, false);
-    }
-#undef GP_BULK
-    return cudaGetLastError();
-  }
-  static cudaError_t general(int grid, bool mul, cudaStream_t s, const SimDesc *sims, const void *consts,
-                             const int *tsim, const void *state, void *next, TileFlags *flag_out, const int *glist,
-                             int *ctr, int ndone, StatBufs st) {
-    if (mul)
-      kf_general<R, N, K, A, true><<<grid, NT, sizeof(GenSmem<R, N, K>), s>>>(
-          sims, (const Consts<R> *)consts, tsim, (const R *)state, (R *)next, flag_out, glist, ctr, ndone, st);
-    else
-      kf_general<R, N, K, A, false><<<grid, NT, sizeof(GenSmem<R, N, K>), s>>>(
-          sims, (const Consts<R> *)consts, tsim, (const R *)state, (R *)next, flag_out, glist, ctr, ndone, st);
     return cudaGetLastError();
   }
   static cudaError_t flags(int ntiles, cudaStream_t s, const SimDesc *sims, const int *tsim, const void *state,
@@ -188,7 +204,8 @@ struct BatchKernels {
     t.classify = classify;
     t.bulk = bulk;
     t.step = step;
-    t.step_occupancy = step_occupancy;
+    t.solo_bytes = SOLO ? sizeof(StepArgs<R, true>) : 0;
+    t.solo_fill = solo_fill;
     t.general = general;
     t.flags = flags;
     t.smooth = smooth;

@@ -68,6 +68,10 @@ gpd::Consts<R> make_consts(const gp_derived &d) {
   c.dx = (R)d.dx; c.dy = (R)d.dy; c.dt = (R)d.dt; c.eps = (R)d.eps; c.inv_eps = (R)d.inv_eps;
   c.tau = (R)d.tau; c.c16pi2 = (R)d.c16pi2; c.jat_obst = (R)d.jat_obst; c.jat_well = (R)d.jat_well;
   c.well_half = (R)d.well_half;
+  {
+    auto plain = [](double v) { return fabs(v) >= 0x1p-60 && fabs(v) < 0x1p60; };
+    c.quick_span = plain(d.dx) && plain(d.dy) ? gpd::QUICK_SPAN : 0u;
+  }
   c.mul_dx = f64 ? pow2(d.dx) : 1;
   c.mul_dy = f64 ? pow2(d.dy) : 1;
   c.inv_dx = (R)(1.0 / d.dx);
@@ -331,6 +335,7 @@ struct gp_batch {
   std::vector<gp_derived> derived;
   std::vector<gpd::SimDesc> desc;
   int dev, nsm, grid_b, grid_g, grid_s;   /* grid_s: kf_step (0: bulk and interface kernels apart) */
+  std::vector<char> solo;       /* a batch of one: its StepArgs (the step kernels' parameter) */
   bool mul;                     /* every simulation's dx and dy are powers of two (or FP32) */
   bool diag;                    /* off-diagonal D, c_mu, A all zero and no E is -0, in every simulation */
   int mbar_tries;               /* kf_bulk's polls of a box barrier before it reports an error */
@@ -348,10 +353,10 @@ struct gp_batch {
   int *d_tsim, *d_seg0, *d_segn;
   void *state[2];               /* ping-pong: every simulation's N phi then K mu planes */
   gpd::TileFlags *flags[2];     /* per tile and state buffer: one-hot phase of the tile and its edge bands */
-  int *glist;                   /* interface tiles of the current step */
+  int4 *glist;                  /* interface tiles of the current step */
   int4 *blist;                  /* bulk tiles of the current step (entries written by kf_classify) */
   int *counters;                /* gpd::CTR_* */
-  gpd::TensorMapSlot *tmaps;    /* [nsims][2]: TMA maps of each simulation's mu planes in state[0], state[1] */
+  gpd::TensorMapSlot *tmaps;    /* [nsims][2][MAP_KINDS]: TMA maps of each simulation's planes in state[0], state[1] */
   int cur;
   long long *ext;               /* running extremes per simulation [nsims][2(N+K)] */
   bool tgrad;                   /* some simulation is non-isothermal: temperature rows each step */
@@ -406,6 +411,7 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   st.round_step = (const unsigned *)(b->counters + gpd::CTR_STEP);
   st.mbar_tries = b->mbar_tries;
   st.tma_extra = b->tma_extra;
+  st.diag = b->diag ? 1 : 0;
   st.dphi_out = b->dphi_out;
   st.bch_max = b->shape.bch_max;
   st.mixed = b->shape.mixed ? 1 : 0;
@@ -420,24 +426,41 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   if (b->tgrad) BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
   BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
                    b->redir_in ? b->redir_have : b->flags[out], b->glist, b->blist, b->counters));
+  gpd::StepLaunch l;
+  l.stream = b->stream;
+  l.mul = b->mul;
+  l.diag = b->diag;
+  l.tg = b->tgrad;
+  l.solo = b->solo.empty() ? nullptr : b->solo.data();
+  l.sims = b->d_desc;
+  l.consts = b->d_consts;
+  l.blist = b->blist;
+  l.glist = b->glist;
+  l.tmaps = tmaps;
+  l.buf = tbuf;
+  l.state = sin;
+  l.next = sout;
+  l.flag_out = b->flags[out];
+  l.ctr = b->counters;
+  l.st = st;
   if (!want_sums && b->grid_s > 0 && b->shape.fused && (!ev || ev[3] == nullptr)) {
     /* one launch for both kinds of tile; ev (with ev[3] null): events after
      * the classification and after the step */
     if (ev) BK(cudaEventRecord(ev[1], b->stream));
-    BK(b->L.step(b->grid_s, b->mul, b->diag, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->blist, b->glist,
-                 tmaps, tbuf, sin, sout, b->flags[out], b->counters, b->grid_s, st));
+    l.grid = l.ndone = b->grid_s;
+    BK(b->L.step(l));
     if (ev) BK(cudaEventRecord(ev[2], b->stream));
     b->cur = out;
     b->steps++;
     return GP_OK;
   }
   /* kf_bulk then kf_general; the last CTA of the two resets the lists */
-  const int nd = b->grid_b + b->grid_g;
-  BK(b->L.bulk(b->grid_b, b->mul, b->diag, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->blist, tmaps, tbuf,
-               sin, sout, b->flags[out], b->counters, nd, st));
+  l.ndone = b->grid_b + b->grid_g;
+  l.grid = b->grid_b;
+  BK(b->L.bulk(l));
   if (ev) BK(cudaEventRecord(ev[1], b->stream));
-  BK(b->L.general(b->grid_g, b->mul, b->stream, b->d_desc, b->d_consts, b->d_tsim, sin, sout,
-                  b->flags[out], b->glist, b->counters, nd, st));
+  l.grid = b->grid_g;
+  BK(b->L.general(l));
   if (ev) BK(cudaEventRecord(ev[2], b->stream));
   b->cur = out;
   b->steps++;
@@ -484,7 +507,7 @@ static int batch_fold_stats(gp_batch *b, gp_stats *out) {
   return GP_OK;
 }
 
-/* The error flag of the step kernels (a TMA box of kf_bulk that did not
+/* The error flag of the step kernels (a TMA box that did not
  * arrive within its poll limit): read, clear, report. */
 static int batch_check_error(gp_batch *b) {
   int e = 0;
@@ -492,7 +515,7 @@ static int batch_check_error(gp_batch *b) {
   BK(cudaStreamSynchronize(b->stream));
   if (e) {
     BK(cudaMemsetAsync(b->counters + gpd::CTR_ERR, 0, sizeof e, b->stream));
-    return bfail(b, GP_ETIMEOUT, "kf_bulk: a tile's mu did not arrive within the wait limit; the state is not valid");
+    return bfail(b, GP_ETIMEOUT, "the step kernels: a tile's staged fields did not arrive within the wait limit; the state is not valid");
   }
   return GP_OK;
 }
@@ -890,33 +913,38 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_tiled_fn() {
   return fn;
 }
 
-/* The TMA maps of kf_bulk: per simulation and state buffer, the K mu planes
- * as a 3-D tensor {pitch, mx, K} (strides one row, one plane) read in boxes
- * of {BW, SH, K}; coordinates outside the tensor read zeros. */
-/* The tensor map of simulation s's K mu planes in a state buffer whose
- * simulation-s planes start at `state` (the bulk tiles' TMA boxes). */
-static int encode_mu_map(gp_batch *b, int s, void *state, gpd::TensorMapSlot *out) {
+/* The tensor maps (MAP_MU, MAP_ALL) of simulation s's planes in a state buffer
+ * where they start at `state`, into out[0..MAP_KINDS): the planes as a 3-D tensor
+ * {pitch, mx, planes} (strides one row, one plane); coordinates outside it read
+ * zeros. */
+static int encode_maps(gp_batch *b, int s, void *state, gpd::TensorMapSlot *out) {
   PFN_cuTensorMapEncodeTiled_v12000 fn = encode_tiled_fn();
   if (!fn) return bfail(b, GP_ECUDA, "cuTensorMapEncodeTiled is not available");
   const bool f64 = b->elem == 8;
-  const cuuint32_t bw = f64 ? gpd::BulkGeom<double, 1>::BW : gpd::BulkGeom<float, 1>::BW;
   const gpd::SimDesc &sd = b->desc[s];
-  void *base = (char *)state + (size_t)((long long)b->N * sd.g.plane) * b->elem;
-  const cuuint64_t dims[3] = {(cuuint64_t)sd.g.pitch, (cuuint64_t)sd.g.mx, (cuuint64_t)b->K};
-  const cuuint64_t strides[2] = {(cuuint64_t)sd.g.pitch * b->elem, (cuuint64_t)sd.g.plane * b->elem};
-  const cuuint32_t box[3] = {bw, (cuuint32_t)gpd::SH, (cuuint32_t)b->K};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn((CUtensorMap *)out, f64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-                  base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return bfail(b, GP_ECUDA, "cuTensorMapEncodeTiled failed (%d) for simulation %d", (int)r, s);
+  for (int kind = 0; kind < gpd::MAP_KINDS; kind++) {
+    const bool all = kind == gpd::MAP_ALL;
+    const int first = all ? 0 : b->N, planes = all ? b->N + b->K : b->K;
+    const cuuint32_t bw = all ? (f64 ? gpd::ItemGeom<double>::BW : gpd::ItemGeom<float>::BW)
+                              : (f64 ? gpd::BulkGeom<double, 1>::BW : gpd::BulkGeom<float, 1>::BW);
+    void *base = (char *)state + (size_t)((long long)first * sd.g.plane) * b->elem;
+    const cuuint64_t dims[3] = {(cuuint64_t)sd.g.pitch, (cuuint64_t)sd.g.mx, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)sd.g.pitch * b->elem, (cuuint64_t)sd.g.plane * b->elem};
+    const cuuint32_t box[3] = {bw, (cuuint32_t)(all ? gpd::FR : gpd::SH), (cuuint32_t)planes};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn((CUtensorMap *)(out + kind), f64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                    3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return bfail(b, GP_ECUDA, "cuTensorMapEncodeTiled failed (%d) for simulation %d", (int)r, s);
+  }
   return GP_OK;
 }
 
-static int encode_mu_maps(gp_batch *b, gpd::TensorMapSlot *out) {
+static int encode_all_maps(gp_batch *b, gpd::TensorMapSlot *out) {
   for (int s = 0; s < b->nsims; s++)
     for (int p = 0; p < 2; p++) {
-      const int rc = encode_mu_map(b, s, (char *)b->state[p] + (size_t)b->desc[s].off_state * b->elem, &out[2 * s + p]);
+      const int rc = encode_maps(b, s, (char *)b->state[p] + (size_t)b->desc[s].off_state * b->elem,
+                                 out + (2 * s + p) * gpd::MAP_KINDS);
       if (rc != GP_OK) return rc;
     }
   return GP_OK;
@@ -1072,6 +1100,10 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
     }
   }
   b->ntiles = nt;
+  if (nsims == 1 && b->L.solo_bytes) {
+    b->solo.resize(b->L.solo_bytes);
+    b->L.solo_fill(b->solo.data(), consts.data(), &b->desc[0]);
+  }
   for (int s = 0; s < nsims; s++) {
     /* kf_bulk packs a tile's row and column into 15 and 16 bits */
     const gpd::SimDesc &sd = b->desc[s];
@@ -1108,8 +1140,21 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
     b->tma_extra = (unsigned)std::max(0, std::min(4096, atoi(v)));
     if (b->tma_extra) b->mbar_tries = 256;
   }
-  int bpb = 1, bpg = 1;
-  e = b->L.prepare(&bpb, &bpg);
+  b->tgrad = false;
+  b->shift = false;
+  for (int s = 0; s < nsims; s++) {
+    b->tgrad |= b->derived[s].tgrad != 0;
+    b->shift |= b->derived[s].shift != 0;
+  }
+  int bpb = 1, bpg = 1, bps = 0;
+  {
+    gpd::StepLaunch l;
+    l.mul = b->mul;
+    l.diag = b->diag;
+    l.tg = b->tgrad;
+    l.solo = b->solo.empty() ? nullptr : b->solo.data();
+    e = b->L.prepare(l, &bpb, &bpg, &bps);
+  }
   if (e != cudaSuccess) {
     rc = bfail(b, GP_ECUDA, "gp_batch_create: %s", cudaGetErrorString(e));
     gp_batch_destroy(b);
@@ -1117,11 +1162,7 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
   }
   b->grid_b = std::min(nt, b->nsm * std::max(1, bpb));
   b->grid_g = b->nsm * std::max(1, bpg);
-  /* the single-launch step when it keeps the bulk kernel's occupancy */
-  {
-    const int bps = b->L.step_occupancy();
-    b->grid_s = (bps >= bpb && getenv("GP_SPLIT_KERNELS") == nullptr) ? b->nsm * bps : 0;
-  }
+  b->grid_s = (bps > 0 && getenv("GP_SPLIT_KERNELS") == nullptr) ? b->nsm * bps : 0;
   /* launch shapes: the first graph chunks of the first batch of its kind time
    * each candidate; later batches of that kind take its choice (GP_NO_TUNING:
    * the first candidate, untimed) */
@@ -1160,7 +1201,7 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
   BALLOC(b->state[1], (size_t)off * b->elem);
   BALLOC(b->flags[0], 2 * sizeof(gpd::TileFlags) * (size_t)nt);
   b->flags[1] = b->flags[0] + nt;
-  BALLOC(b->glist, sizeof(int) * (size_t)nt);
+  BALLOC(b->glist, sizeof(int4) * (size_t)nt);
   BALLOC(b->blist, sizeof(int4) * (size_t)nt);
   BALLOC(b->d_desc, sizeof(gpd::SimDesc) * nsims);
   BALLOC(b->d_consts, csz * nsims);
@@ -1171,20 +1212,14 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
   BALLOC(b->partials, sizeof(double) * (size_t)ns * nt);
   BALLOC(b->sums_sim, sizeof(double) * (size_t)ns * nsims);
   BALLOC(b->counters, gpd::CTR_COUNT * sizeof(int));
-  BALLOC(b->tmaps, sizeof(gpd::TensorMapSlot) * 2 * (size_t)nsims);
-  b->tgrad = false;
-  b->shift = false;
-  for (int s = 0; s < nsims; s++) {
-    b->tgrad |= b->derived[s].tgrad != 0;
-    b->shift |= b->derived[s].shift != 0;
-  }
+  BALLOC(b->tmaps, sizeof(gpd::TensorMapSlot) * 2 * gpd::MAP_KINDS * (size_t)nsims);
   BALLOC(b->spos, sizeof(int) * (size_t)nsims);
   if (b->shift) b->tune_next = b->ncand;   /* the first chunks end at the frame checks: no tuning */
   BALLOC(b->trows, sizeof(double) * (size_t)std::max(offT, 1));
   BALLOC(b->dyn, sizeof(gpd::SimDyn) * (size_t)nsims);
 #undef BALLOC
-  std::vector<gpd::TensorMapSlot> tm(2 * (size_t)nsims);
-  if (encode_mu_maps(b, tm.data()) != GP_OK) {
+  std::vector<gpd::TensorMapSlot> tm(2 * gpd::MAP_KINDS * (size_t)nsims);
+  if (encode_all_maps(b, tm.data()) != GP_OK) {
     rc = GP_ECUDA;
     gp_batch_destroy(b);
     return rc;
@@ -1545,6 +1580,11 @@ int gp_set_stat_rows(gp_ctx *c, long x0, long x1) {
   CK(cudaMemcpyAsync(b->d_desc, b->desc.data(), sizeof(gpd::SimDesc) * b->desc.size(), cudaMemcpyHostToDevice,
                      b->stream));
   CK(cudaStreamSynchronize(b->stream));
+  /* the step kernels take the rows from their parameter: captured steps hold the old ones */
+  std::vector<char> consts(b->consts_bytes);
+  CK(cudaMemcpy(consts.data(), b->d_consts, b->consts_bytes, cudaMemcpyDeviceToHost));
+  if (!b->solo.empty()) b->L.solo_fill(b->solo.data(), consts.data(), &sd);
+  batch_drop_graphs(b);
   return GP_OK;
 }
 
@@ -1611,7 +1651,7 @@ struct AdjBufs {
          *pbar = nullptr, *final_state = nullptr;
   double *rblk = nullptr;   /* two reverse blocks: adjoint of a state, adjoint of its delta-phi, list counters */
   double *dtape = nullptr;  /* delta-phi of every step, written by the forward pass (whole-tape mode) */
-  gpd::TensorMapSlot *smaps = nullptr;   /* whole-tape mode: the tensor map of each slot's mu planes */
+  gpd::TensorMapSlot *smaps = nullptr;   /* whole-tape mode: the tensor maps of each slot's planes */
   int2 *cells = nullptr;    /* cells of a reverse pass that take the dual passes */
   int *ncells = nullptr;
   gpd::TileFlags *unknown = nullptr;   /* whole-tape mode: "unknown" flags of every tile (redir_have) */
@@ -1721,13 +1761,14 @@ int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) {
   if (dtape) AALLOC(m.dtape, Sd * (size_t)T);
 #undef AALLOC
   if (dtape) {
-    std::vector<gpd::TensorMapSlot> hm((size_t)T);
+    std::vector<gpd::TensorMapSlot> hm(gpd::MAP_KINDS * (size_t)T);
     for (long t = 0; t < T; t++)
-      if ((rc = encode_mu_map(b, 0, m.snap + S * (size_t)t, &hm[(size_t)t])) != GP_OK) return fail(c, rc, "%s", b->err);
-    if (cudaMalloc((void **)&m.smaps, sizeof(gpd::TensorMapSlot) * (size_t)T) != cudaSuccess ||
+      if ((rc = encode_maps(b, 0, m.snap + S * (size_t)t, &hm[gpd::MAP_KINDS * (size_t)t])) != GP_OK)
+        return fail(c, rc, "%s", b->err);
+    if (cudaMalloc((void **)&m.smaps, sizeof(gpd::TensorMapSlot) * hm.size()) != cudaSuccess ||
         cudaMalloc((void **)&m.unknown, sizeof(gpd::TileFlags) * (size_t)b->ntiles) != cudaSuccess)
       return fail(c, GP_ENOMEM, "gp_adjoint: cudaMalloc of the slot maps failed");
-    CK(cudaMemcpyAsync(m.smaps, hm.data(), sizeof(gpd::TensorMapSlot) * (size_t)T, cudaMemcpyHostToDevice, b->stream));
+    CK(cudaMemcpyAsync(m.smaps, hm.data(), sizeof(gpd::TensorMapSlot) * hm.size(), cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemsetAsync(m.unknown, 0xfe, sizeof(gpd::TileFlags) * (size_t)b->ntiles, b->stream));
     /* the interface tiles write the delta-phi of their cells and rings; every
      * other cell of every step keeps this +0.0 */
@@ -1873,7 +1914,7 @@ int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) {
           for (long t = t0; t < t1; t++) {
             b->redir_in = slot_ptr((int)t);
             b->redir_out = t + 1 < T ? slot_ptr((int)t + 1) : m.final_state;
-            b->redir_map = m.smaps + t;
+            b->redir_map = m.smaps + gpd::MAP_KINDS * t;
             b->redir_have = m.unknown;
             b->dphi_out = m.dtape + Sd * (size_t)t;
             const int r = batch_step_once(b, 0, nullptr);

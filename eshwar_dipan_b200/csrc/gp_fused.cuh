@@ -17,11 +17,10 @@
  *              next tile's mu in flight (one TMA box) while one is stepped.  Bulk
  *              tiles read and write mu only (phi is rewritten only when the
  *              output buffer does not already hold the same one-hot tile).
- *  kf_general  persistent CTAs over the interface list.  Stages phi with a
- *              two-cell halo and mu with one, computes delta-phi on the tile
- *              plus its one-cell ring in shared memory (the ring is recomputed
- *              by each neighbour instead of going through HBM), then the mu
- *              update and the phi commit, and the tile's new flag.
+ *  kf_general  persistent CTAs over the interface list (gp_iface.cuh): delta-phi
+ *              on a tile plus its one-cell ring in shared memory (the ring is
+ *              recomputed by each neighbour instead of going through HBM), then
+ *              the mu update and the phi commit, and the tile's new flags.
  *
  * The arithmetic of each cell is the reference's, in its order (FP64 results
  * are bit-identical to the reference step); the FP32 form differs only where
@@ -31,14 +30,11 @@
 #include <climits>
 #include <type_traits>
 
+#include "gp_iface.cuh"
+#include "gp_iface32.cuh"
 #include "gp_tiles.cuh"
 
 namespace gpd {
-
-constexpr int W2 = TY + 4, H2 = TX + 4, S2 = W2 * H2;   /* phi with a two-cell halo */
-constexpr int RXF = (TX + 3) * (TY + 2);                 /* x-faces around the ring cells */
-constexpr int RYF = (TX + 2) * (TY + 3);                 /* y-faces around the ring cells */
-#define L2I(i, j) ((i) * W2 + (j))
 
 constexpr signed char FLAG_MIXED = -1, FLAG_UNKNOWN = -2;
 
@@ -103,28 +99,11 @@ __device__ __forceinline__ float ulpf(float v) {
  * four two-cell-deep edge bands (top = first two rows, bot = last two rows,
  * left/right = first/last two columns, over the tile's cells inside the
  * domain): the phase p whose exact one-hot phi every cell of the region holds,
- * FLAG_MIXED, or FLAG_UNKNOWN.  8 bytes, read as one word. */
+ * FLAG_MIXED, or FLAG_UNKNOWN.  8 bytes, read as one word.  The bottom and
+ * right bands are read only where a tile follows (the tile is then full). */
 struct __align__(8) TileFlags {
   signed char whole, top, bot, left, right, pad0, pad1, pad2;
 };
-
-struct RemapTab2 {
-  int row[H2], col[W2];
-};
-
-/* rows/columns of the two-cell phi halo (origin x0-2, y0-2) after the remap;
- * -1 outside [-2, m+1] (not needed by any delta-phi ring cell). */
-template <typename R>
-__device__ __forceinline__ void remap_tab2(RemapTab2 &t, const Consts<R> &D, const Grid &g, int x0, int y0) {
-  const int u = threadIdx.x;
-  if (u < H2) {
-    const int x = x0 - 2 + u;
-    t.row[u] = (x >= -2 && x <= g.mx + 1) ? remap(x, g.mx, D.bc_x[0][0], D.bc_x[0][1]) * g.pitch : -1;
-  } else if (u < H2 + W2) {
-    const int y = y0 - 2 + (u - H2);
-    t.col[u - H2] = (y >= -2 && y <= g.my + 1) ? remap(y, g.my, D.bc_y[0][0], D.bc_y[0][1]) : -1;
-  }
-}
 
 /* one-hot test on exact bits: phase index, or -1 */
 template <typename R, int N>
@@ -145,40 +124,34 @@ __device__ __forceinline__ int one_hot(const R *ph) {
   return (ones == 1 && zeros == N - 1) ? p : -1;
 }
 
-/* Flags of a tile from its new phi, one one-hot phase (or -1) per thread
- * (cell (tx, ty) of the tile, valid cells only; rows x cols cells are in the
- * domain).  Call with all threads; the result is valid in every thread. */
-__device__ __forceinline__ TileFlags tile_flags(bool valid, int p, int tx, int ty, int rows, int cols) {
-  __shared__ int s_lo[NT / 32][5], s_hi[NT / 32][5];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const bool in[5] = {true, tx < 2, tx >= rows - 2, ty < 2, ty >= cols - 2};
-  int lo[5], hi[5];
+/* Flag bits of one tile row (a warp, a lane per column) from the one-hot phase
+ * (or -1) of each lane's cell: bit p: every valid cell holds phase p; bit 8+p:
+ * those of the first two columns; bit 16+p: those of the last two.  Call with the
+ * whole warp. */
+template <int N>
+__device__ __forceinline__ unsigned row_flag_bits(bool valid, int oh) {
+  const unsigned v = __ballot_sync(0xffffffffu, valid);
+  unsigned r = 0;
 #pragma unroll
-  for (int r = 0; r < 5; r++) {
-    lo[r] = (valid && in[r]) ? p : INT_MAX;
-    hi[r] = (valid && in[r]) ? p : INT_MIN;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[r] = min(lo[r], __shfl_xor_sync(0xffffffffu, lo[r], o));
-      hi[r] = max(hi[r], __shfl_xor_sync(0xffffffffu, hi[r], o));
-    }
+  for (int p = 0; p < N; p++) {
+    const unsigned miss = v & ~__ballot_sync(0xffffffffu, oh == p);
+    r |= (miss ? 0u : 1u << p) | ((miss & 0x3u) ? 0u : 1u << (8 + p)) |
+         ((miss & 0xc0000000u) ? 0u : 1u << (16 + p));
   }
-  if (lane == 0) {
+  return r;
+}
+/* a tile's flags from its rows' bits; a row outside the domain holds every bit */
+__device__ __forceinline__ TileFlags flags_of_rows(const unsigned *w) {
+  unsigned all = w[0];
 #pragma unroll
-    for (int r = 0; r < 5; r++) { s_lo[wid][r] = lo[r]; s_hi[wid][r] = hi[r]; }
-  }
-  __syncthreads();
-  signed char f[5];
-#pragma unroll
-  for (int r = 0; r < 5; r++) {
-    int l2 = INT_MAX, h2 = INT_MIN;
-#pragma unroll
-    for (int w = 0; w < NT / 32; w++) { l2 = min(l2, s_lo[w][r]); h2 = max(h2, s_hi[w][r]); }
-    f[r] = (l2 >= 0 && l2 == h2) ? (signed char)l2 : FLAG_MIXED;
-  }
-  __syncthreads();
+  for (int r = 1; r < TX; r++) all &= w[r];
+  auto phase = [](unsigned bits) { return bits ? (signed char)(__ffs(bits) - 1) : FLAG_MIXED; };
   TileFlags t;
-  t.whole = f[0]; t.top = f[1]; t.bot = f[2]; t.left = f[3]; t.right = f[4];
+  t.whole = phase(all & 0xffu);
+  t.top = phase(w[0] & w[1] & 0xffu);
+  t.bot = phase(w[TX - 2] & w[TX - 1] & 0xffu);
+  t.left = phase((all >> 8) & 0xffu);
+  t.right = phase((all >> 16) & 0xffu);
   t.pad0 = t.pad1 = t.pad2 = 0;
   return t;
 }
@@ -238,519 +211,6 @@ __device__ __forceinline__ int bulk_phase(const Consts<R> &D, const Grid &g, con
 
 
 /* ------------------------------------------------------------------ */
-/* interface tiles                                                     */
-/* ------------------------------------------------------------------ */
-
-template <typename R, int N, int K>
-struct GenSmem {
-  R P[N][S2];              /* phi, two-cell halo, origin (x0-2, y0-2) */
-  R M[K][SS];              /* mu, one-cell halo, origin (x0-1, y0-1)  */
-  R DP[N][SS];             /* delta-phi of the ring region (same origin as M) */
-  unsigned char ACT[SS];   /* active phases of each ring cell (bit a) */
-  short LIST[SS];          /* ring cells with an active phase, in no particular order */
-  short FLIST[RXF + RYF];  /* anisotropy faces those cells read */
-  int nlist, nflist;
-  union {
-    R T[NP<N>::v][4][RXF + RYF];   /* anisotropy face terms of the ring region */
-    struct {
-      R CM[N][K][SS];      /* c_a,k(mu) per cell */
-      R H[N][SS];          /* h_a(phi) per cell */
-      R SP[N][SS];         /* s_phi of the obstacle anti-trapping (solid phases) */
-      R DD[K][K][SS];      /* D_kl per cell */
-      R JX[K][NXF], JY[K][NYF];
-      R FX[K][K][NXF], FY[K][K][NYF];
-    } u;
-  } w;
-  RemapTab2 rtp;
-  RemapTab rtm;
-};
-
-/* Anisotropy terms of one face of the ring region for all pairs: the same
- * arithmetic as face_terms (function_A_01.h:163-215 through functionQ.h and
- * anisotropy_01.h) on the two-cell-halo layout.  xface: face between P rows
- * i and i+1 at column j; else between columns j and j+1 of row i. */
-template <typename R, int N, typename CT>
-__device__ __forceinline__ void ring_face_terms(const CT &D, const R (*P)[S2], R (*T)[4][RXF + RYF],
-                                                bool xface, int i, int j, int fidx) {
-  R s[N], gr[N], c0[N], c1[N];
-#pragma unroll
-  for (int a = 0; a < N; a++) {
-    const R *S = P[a];
-    if (xface) {
-      R p0 = S[L2I(i, j)], p1 = S[L2I(i + 1, j)];
-      s[a] = R(0.5) * (p1 + p0);
-      gr[a] = divx(p1 - p0, D);
-      c0[a] = div2y(S[L2I(i, j + 1)] - S[L2I(i, j - 1)], D);
-      c1[a] = div2y(S[L2I(i + 1, j + 1)] - S[L2I(i + 1, j - 1)], D);
-    } else {
-      R p0 = S[L2I(i, j)], p1 = S[L2I(i, j + 1)];
-      s[a] = R(0.5) * (p1 + p0);
-      gr[a] = divy(p1 - p0, D);
-      c0[a] = R(0.5) * (divx(S[L2I(i + 1, j)] - S[L2I(i, j)], D) + divx(S[L2I(i, j)] - S[L2I(i - 1, j)], D));
-      c1[a] = R(0.5) * (divx(S[L2I(i + 1, j + 1)] - S[L2I(i, j + 1)], D) +
-                        divx(S[L2I(i, j + 1)] - S[L2I(i - 1, j + 1)], D));
-    }
-  }
-#pragma unroll
-  for (int a = 0; a < N; a++)
-#pragma unroll
-    for (int b = a + 1; b < N; b++) {
-      const int p = pidx<N>(a, b);
-      R Pab = s[a] * gr[b] - s[b] * gr[a];
-      R Pba = s[b] * gr[a] - s[a] * gr[b];
-      R tq = R(0.5) * (s[a] * (c0[b] + c1[b]) - s[b] * (c0[a] + c1[a]));
-      R q0, q1;
-      if (xface) rot2(D, D.rot[a][b], Pab, tq, q0, q1);
-      else rot2(D, D.rot[a][b], tq, Pab, q0, q1);
-      R acv = ac(q0, q1, D.dab[a][b]);
-      QPow<R> qp = qpow(q0, q1);
-      R rd;
-      if (D.rot_identity) {
-        rd = (xface ? dadq_c(q0, qp, D.dab16[a][b]) : dadq_c(q1, qp, D.dab16[a][b])) + R(0.0);
-      } else {
-        R d0 = dadq_c(q0, qp, D.dab16[a][b]), d1 = dadq_c(q1, qp, D.dab16[a][b]);
-        R r0, r1;
-        rot2(D, D.rinv[a][b], d0, d1, r0, r1);
-        rd = xface ? r0 : r1;
-      }
-      R ac2 = acv * acv, acq = acv * qp.q2;
-      T[p][0][fidx] = ac2 * Pab * (-s[b]);
-      T[p][1][fidx] = ac2 * Pba * (-s[a]);
-      T[p][2][fidx] = acq * rd * (-s[b]);
-      T[p][3][fidx] = acq * (R(0.0) - rd) * (-s[a]);
-    }
-}
-
-/* delta-phi of one ring cell (ring coordinates ri, rj; its phi at P row ri+1,
- * column rj+1) from the staged tile: calculate_divergence_phasefield_2D
- * (calculate_divergence_phasefield.h:4-62) in the same arithmetic as dphi_tile.
- * Not inlined: as a call of its own it gets its own register allocation, and
- * the interface tiles spill far less under the 128-register cap of two CTAs
- * per SM (FP64 ternary 3-phase: 732 bytes of spill stores inlined, about 200
- * not; FP32: none), which made whole steps 3-8 % faster. */
-template <typename R, int N, int K, bool ANISO, typename CT>
-__device__ __noinline__ void ring_dphi(const CT &D, const GenSmem<R, N, K> &sm, int ri, int rj,
-                                          unsigned mask, R *d, double Tpf) {
-  const int i = ri + 1, j = rj + 1, e = LI(ri, rj);
-  R ph[N];
-  bool act[N];
-#pragma unroll
-  for (int a = 0; a < N; a++) {
-    ph[a] = sm.P[a][L2I(i, j)];
-    act[a] = (mask >> a) & 1u;
-  }
-  if (!mask) {
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      d[a] = R(0.0);
-      if ((ph[a] + d[a]) < R(0.0)) d[a] += fabs(d[a] + ph[a]);
-    }
-    return;
-  }
-  R m[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) m[k] = sm.M[k][e];
-  R gcx[N], gcy[N];
-#pragma unroll
-  for (int a = 0; a < N; a++) {
-    const R *S = sm.P[a];
-    gcx[a] = R(0.5) * (divx(S[L2I(i + 1, j)] - S[L2I(i, j)], D) + divx(S[L2I(i, j)] - S[L2I(i - 1, j)], D));
-    gcy[a] = div2y(S[L2I(i, j + 1)] - S[L2I(i, j - 1)], D);
-  }
-  R psi[N];
-  if (D.tgrad) {
-    /* init_propertymatrices(T) at the cell's temperature before dpsi
-     * (calculate_divergence_phasefield.h:21-29) */
-    R E[N][K], Bt[N][K], Ct[N];
-    e_at<R, N, K>(D, Tpf, E);
-    bc_at<R, N, K>(D, Tpf, Bt, Ct);
-#pragma unroll
-    for (int b = 0; b < N; b++) {
-      R c[K], ps = R(0.0);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        c[k] = c_muE<R, K>(D, E[b], m, b, k);
-        ps -= m[k] * c[k];
-      }
-      ps += feBC<R, K>(D, Bt[b], Ct[b], c, b);
-      psi[b] = ps;
-    }
-  } else {
-#pragma unroll
-    for (int b = 0; b < N; b++) {
-      R c[K], ps = R(0.0);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        c[k] = c_mu<R, K>(D, m, b, k);
-        ps -= m[k] * c[k];
-      }
-      ps += fe<R, K>(D, c, b);
-      psi[b] = ps;
-    }
-  }
-  R cq0[NP<N>::v], cq1[NP<N>::v], cd0[NP<N>::v], cd1[NP<N>::v], cac[NP<N>::v], cq2[NP<N>::v];
-  if (ANISO) {
-#pragma unroll
-    for (int a = 0; a < N; a++)
-#pragma unroll
-      for (int b = a + 1; b < N; b++) {
-        const int p = pidx<N>(a, b);
-        R q0, q1;
-        rot2(D, D.rot[a][b], (ph[a] * gcx[b] - ph[b] * gcx[a]), (ph[a] * gcy[b] - ph[b] * gcy[a]), q0, q1);
-        QPow<R> qp = qpow(q0, q1);
-        cq0[p] = q0;
-        cq1[p] = q1;
-        cd0[p] = dadq_c(q0, qp, D.dab16[a][b]);
-        cd1[p] = dadq_c(q1, qp, D.dab16[a][b]);
-        cq2[p] = (q0 * q0 + q1 * q1 + R(0.0) * R(0.0));
-        cac[p] = ac(q0, q1, D.dab[a][b]);
-      }
-  }
-  const R tau = tau_of<R, N>(D, ph);
-  R lam[N], sl = R(0.0);
-  long nact = 0;
-  /* face indices of this cell in the ring face cache */
-  const int xf = i * (TY + 2) + (j - 1), xb = (i - 1) * (TY + 2) + (j - 1);
-  const int yr = RXF + (i - 1) * (TY + 3) + j, yl = RXF + (i - 1) * (TY + 3) + (j - 1);
-#pragma unroll
-  for (int a = 0; a < N; a++) {
-    if (!act[a]) continue;
-    R dA, div;
-    if (ANISO) {
-      R s1 = R(0.0), s2 = R(0.0), t1 = R(0.0), t2 = R(0.0);
-#pragma unroll
-      for (int b = 0; b < N; b++) {
-        if (b == a) continue;
-        const int p = a < b ? pidx<N>(a, b) : pidx<N>(b, a);
-        const R sg = R(0.0);
-        R q0 = a < b ? cq0[p] : sg - cq0[p], q1 = a < b ? cq1[p] : sg - cq1[p];
-        R d0 = a < b ? cd0[p] : sg - cd0[p], d1 = a < b ? cd1[p] : sg - cd1[p];
-        R w0, w1;
-        rot2(D, D.rot[a][b], gcx[b], gcy[b], w0, w1);
-        R sp1 = R(0.0), sp2 = R(0.0);
-        sp1 += q0 * w0;
-        sp1 += q1 * w1;
-        sp2 += (d0) * w0;
-        sp2 += (d1) * w1;
-        sp1 *= D.gamma[a][b] * (cac[p] * cac[p]);
-        sp2 *= D.gamma[a][b] * cac[p] * cq2[p];
-        s1 += sp1;
-        s2 += sp2;
-        const int o = a < b ? 0 : 1;
-        const R(*T)[RXF + RYF] = sm.w.T[p];
-        R d1v = divx((T[o][xf]) - (T[o][xb]), D);
-        d1v += divy((T[o][yr]) - (T[o][yl]), D);
-        d1v *= D.gamma[a][b];
-        t1 += d1v;
-        R d2v = divx(T[2 + o][xf] - T[2 + o][xb], D);
-        d2v += divy(T[2 + o][yr] - T[2 + o][yl], D);
-        d2v *= D.gamma[a][b];
-        t2 += d2v;
-      }
-      dA = R(2.0) * (s1 + s2);
-      div = (R(2.0) * (t1 + t2) + R(0.0));
-    } else {
-      R s = R(0.0), t = R(0.0);
-      const R *Sa = sm.P[a];
-#pragma unroll
-      for (int b = 0; b < N; b++) {
-        if (b == a) continue;
-        const R *Sb = sm.P[b];
-        R sp = R(0.0);
-        sp += (ph[a] * gcx[b] - ph[b] * gcx[a]) * gcx[b];
-        sp += (ph[a] * gcy[b] - ph[b] * gcy[a]) * gcy[b];
-        sp *= D.gamma[a][b];
-        s += sp;
-        R pa = Sa[L2I(i, j)], pb = Sb[L2I(i, j)];
-        R sxa = R(0.5) * (Sa[L2I(i + 1, j)] + pa), sxb = R(0.5) * (Sb[L2I(i + 1, j)] + pb);
-        R gxa = divx(Sa[L2I(i + 1, j)] - pa, D), gxb = divx(Sb[L2I(i + 1, j)] - pb, D);
-        R bxa = R(0.5) * (pa + Sa[L2I(i - 1, j)]), bxb = R(0.5) * (pb + Sb[L2I(i - 1, j)]);
-        R hxa = divx(pa - Sa[L2I(i - 1, j)], D), hxb = divx(pb - Sb[L2I(i - 1, j)], D);
-        R sya = R(0.5) * (Sa[L2I(i, j + 1)] + pa), syb = R(0.5) * (Sb[L2I(i, j + 1)] + pb);
-        R gya = divy(Sa[L2I(i, j + 1)] - pa, D), gyb = divy(Sb[L2I(i, j + 1)] - pb, D);
-        R lya = R(0.5) * (pa + Sa[L2I(i, j - 1)]), lyb = R(0.5) * (pb + Sb[L2I(i, j - 1)]);
-        R hya = divy(pa - Sa[L2I(i, j - 1)], D), hyb = divy(pb - Sb[L2I(i, j - 1)], D);
-        R dvg = divx((sxa * gxb - sxb * gxa) * (-sxb) - ((bxa * hxb - bxb * hxa) * (-bxb)), D);
-        dvg += divy((sya * gyb - syb * gya) * (-syb) - ((lya * hyb - lyb * hya) * (-lyb)), D);
-        dvg *= D.gamma[a][b];
-        t += dvg;
-      }
-      dA = R(2.0) * s;
-      div = R(2.0) * t;
-    }
-    R dpsi = R(0.0);
-#pragma unroll
-    for (int b = 0; b < N; b++) dpsi += psi[b] * dh<R, N>(ph, b, a);
-    lam[a] = D.eps * (-dA + div) - D.inv_eps * dwdphi<R, N>(D, ph, act, a, false) - dpsi;
-    sl += lam[a];
-    nact++;
-  }
-  if (nact) sl /= (R)nact;
-#pragma unroll
-  for (int a = 0; a < N; a++) d[a] = act[a] ? D.dt * (lam[a] - sl) / (tau * D.eps) : R(0.0);
-  project<R, N>(ph, act, d);
-}
-
-/* One interface tile (cells (x0+tx, y0+ty)): delta-phi on the tile and its
- * ring, then the concentration pass (calculate_fluxes_concentration_2D +
- * calculate_divergence_concentration_2D, calculate_fluxes_concentration.h:4-145,
- * calculate_divergence_concentration.h:4-153) and the phi commit, in the
- * arithmetic of update_tile's general path.  Returns the tile's new flags. */
-template <typename R, int N, int K, bool ANISO, typename CT>
-__device__ __forceinline__ TileFlags general_tile(const CT &D, const Grid &g, const R *__restrict__ phi,
-                                                    const R *__restrict__ mu, R *__restrict__ phin,
-                                                    R *__restrict__ mun, int x0, int y0, const StatBufs &st,
-                                                    long long ext_slot, long long slot, GenSmem<R, N, K> &sm,
-                                                    const double *__restrict__ tpf, const double *__restrict__ tcc) {
-  constexpr int L = N - 1;
-  const R cst = D.obstacle ? D.jat_obst : D.jat_well;
-
-  /* ---- stage phi (two-cell halo) and mu (one-cell halo) through the copy tables */
-  remap_tab2(sm.rtp, D, g, x0, y0);
-  remap_tab(sm.rtm, D, g, x0, y0, 1, -1, g.mx, -1, g.my);
-  __syncthreads();
-  for (int e = threadIdx.x; e < S2; e += NT) {
-    const int i = e / W2, j = e - i * W2;
-    const int r = sm.rtp.row[i], c = sm.rtp.col[j];
-    if (r >= 0 && c >= 0) {
-      const R *src = phi + (r + c);
-#pragma unroll
-      for (int a = 0; a < N; a++) sm.P[a][e] = __ldg(src + a * g.plane);
-    } else {
-#pragma unroll
-      for (int a = 0; a < N; a++) sm.P[a][e] = R(0.0);
-    }
-  }
-  for (int e = threadIdx.x; e < SS; e += NT) {
-    const int i = e / SW, j = e - i * SW;
-    const int r = sm.rtm.row[i], c = sm.rtm.col[j];
-    if (r >= 0 && c >= 0) {
-      const R *src = mu + (r + c);
-#pragma unroll
-      for (int k = 0; k < K; k++) sm.M[k][e] = __ldg(src + k * g.plane);
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; k++) sm.M[k][e] = R(0.0);
-    }
-  }
-  __syncthreads();
-
-  /* ---- active phases of the ring cells (interior plus ring: x <= mx, y <= my).
-   * A cell with no active phase gets its delta-phi here (no phase active:
-   * 0, then the projection's clamp of a negative phi; outside the needed
-   * region: 0); the others go on a list, so that the expensive delta-phi
-   * work is spread over every thread of the CTA wherever the active cells
-   * lie in the tile. */
-  for (int e = threadIdx.x; e < SS; e += NT) {
-    const int ri = e / SW, rj = e - ri * SW, i = ri + 1, j = rj + 1;
-    const bool vd = (x0 - 1 + ri <= g.mx) && (y0 - 1 + rj <= g.my);
-    unsigned mask = 0;
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      const R *S = sm.P[a];
-      R gxf = divx(S[L2I(i + 1, j)] - S[L2I(i, j)], D), gxb = divx(S[L2I(i, j)] - S[L2I(i - 1, j)], D);
-      R gyr = divy(S[L2I(i, j + 1)] - S[L2I(i, j)], D), gyl = divy(S[L2I(i, j)] - S[L2I(i, j - 1)], D);
-      R dv = divx(gxf - gxb, D);
-      dv += divy(gyr - gyl, D);
-      if (fabs(dv) > R(0.0)) mask |= 1u << a;
-    }
-    if (!vd) mask = 0;
-    sm.ACT[e] = (unsigned char)mask;
-    if (mask) {
-      sm.LIST[atomicAdd(&sm.nlist, 1)] = (short)e;
-    } else {
-#pragma unroll
-      for (int a = 0; a < N; a++) {
-        R d = R(0.0);
-        if (vd) {
-          const R ph = sm.P[a][L2I(i, j)];
-          if ((ph + d) < R(0.0)) d += fabs(d + ph);
-        }
-        sm.DP[a][e] = d;
-      }
-    }
-  }
-  __syncthreads();
-  const int nact = sm.nlist;
-  if (ANISO && nact > 0) {
-    /* only the faces of active ring cells are read by ring_dphi: list them,
-     * then compute them spread over the CTA */
-    for (int e = threadIdx.x; e < RXF + RYF; e += NT) {
-      bool need;
-      if (e < RXF) {
-        const int fi = e / (TY + 2), fj = e - fi * (TY + 2) + 1;
-        /* ring cells (fi-1, fj-1) and (fi, fj-1) */
-        need = (fi >= 1 && sm.ACT[LI(fi - 1, fj - 1)]) || (fi < SH && sm.ACT[LI(fi, fj - 1)]);
-      } else {
-        const int f = e - RXF, fi = f / (TY + 3) + 1, fj = f - (fi - 1) * (TY + 3);
-        /* ring cells (fi-1, fj-1) and (fi-1, fj) */
-        need = (fj >= 1 && sm.ACT[LI(fi - 1, fj - 1)]) || (fj < SW && sm.ACT[LI(fi - 1, fj)]);
-      }
-      if (need) sm.FLIST[atomicAdd(&sm.nflist, 1)] = (short)e;
-    }
-    __syncthreads();
-    const int nf = sm.nflist;
-    for (int q = threadIdx.x; q < nf; q += NT) {
-      const int e = sm.FLIST[q];
-      if (e < RXF) {
-        const int fi = e / (TY + 2), fj = e - fi * (TY + 2) + 1;
-        ring_face_terms<R, N>(D, sm.P, sm.w.T, true, fi, fj, e);
-      } else {
-        const int f = e - RXF, fi = f / (TY + 3) + 1, fj = f - (fi - 1) * (TY + 3);
-        ring_face_terms<R, N>(D, sm.P, sm.w.T, false, fi, fj, e);
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < nact; q += NT) {
-    const int e = sm.LIST[q];
-    const int ri = e / SW, rj = e - ri * SW;
-    R d[N];
-    ring_dphi<R, N, K, ANISO>(D, sm, ri, rj, sm.ACT[e], d, D.tgrad ? tpf[y0 - 1 + rj + 3] : 0.0);
-#pragma unroll
-    for (int a = 0; a < N; a++) sm.DP[a][e] = d[a];
-  }
-  __syncthreads();   /* the face-term cache is dead from here: its space holds the update's arrays */
-  if (st.dphi_out) {
-    /* the adjoint's tape: the delta-phi of the tile and of its ring cells
-     * (the domain's ring included), as the reverse sweep reads it */
-    for (int e = threadIdx.x; e < SS; e += NT) {
-      const int x = x0 - 1 + e / SW, y = y0 - 1 + e % SW;
-      if (x <= g.mx && y <= g.my) {
-#pragma unroll
-        for (int a = 0; a < N; a++)
-          st.dphi_out[a * g.dplane + (long long)(x + 1) * g.dpitch + (y + 1)] = (double)sm.DP[a][e];
-      }
-    }
-  }
-  if (threadIdx.x == 0) {
-    sm.nlist = 0;    /* for the CTA's next tile */
-    sm.nflist = 0;
-  }
-
-#define PR(a, e) sm.P[a][L2I((e) / SW + 1, (e) % SW + 1)]
-  /* ---- per-cell quantities of the ring region */
-  for (int e = threadIdx.x; e < SS; e += NT) {
-    R p[N], mm[K];
-#pragma unroll
-    for (int a = 0; a < N; a++) p[a] = PR(a, e);
-#pragma unroll
-    for (int k = 0; k < K; k++) mm[k] = sm.M[k][e];
-    R Ec[N][K];
-    /* the ghosted column of ring cell e (cells past my+1 are not needed: clamped) */
-    if (D.tgrad) e_at<R, N, K>(D, tcc[min(y0 - 1 + e % SW + 3, g.my + 5)], Ec);
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      R hv = h<R, N>(p, a);
-      sm.w.u.H[a][e] = hv;
-#pragma unroll
-      for (int k = 0; k < K; k++)
-        sm.w.u.CM[a][k][e] = D.tgrad ? c_muE<R, K>(D, Ec[a], mm, a, k) : c_mu<R, K>(D, mm, a, k);
-      if (a < L)
-        sm.w.u.SP[a][e] =
-            (p[a] * (R(1.0) - p[a]) > R(0.0)) ? p[a] * (R(1.0) - hv) / (sqrt(p[a] * (R(1.0) - p[a]))) : R(0.0);
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-      for (int l = 0; l < K; l++) sm.w.u.DD[k][l][e] = Dcell<R, N, K>(D, p, k, l);
-  }
-  __syncthreads();
-
-#define PRIJ(a, i, j) sm.P[a][L2I((i) + 1, (j) + 1)]
-  /* ---- faces of the tile: anti-trapping current and diffusion flux products */
-  for (int e = threadIdx.x; e < NXF + NYF; e += NT) {
-    const bool xface = e < NXF;
-    int fi, fj, i1, j1, fidx;
-    if (xface) { fi = e / TY; fj = e - fi * TY + 1; i1 = fi + 1; j1 = fj; fidx = e; }
-    else { int f = e - NXF; fi = f / (TY + 1) + 1; fj = f - (fi - 1) * (TY + 1); i1 = fi; j1 = fj + 1; fidx = f; }
-    const int c0 = LI(fi, fj), c1 = LI(i1, j1);
-    R gr[N], cn[N];
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      if (xface) {
-        gr[a] = divx(PRIJ(a, i1, j1) - PRIJ(a, fi, fj), D);
-        cn[a] = R(0.5) * (div2y(PRIJ(a, fi, fj + 1) - PRIJ(a, fi, fj - 1), D) +
-                          div2y(PRIJ(a, i1, fj + 1) - PRIJ(a, i1, fj - 1), D));
-      } else {
-        gr[a] = divy(PRIJ(a, i1, j1) - PRIJ(a, fi, fj), D);
-        R gc0 = R(0.5) * (divx(PRIJ(a, fi + 1, fj) - PRIJ(a, fi, fj), D) + divx(PRIJ(a, fi, fj) - PRIJ(a, fi - 1, fj), D));
-        R gc1 = R(0.5) * (divx(PRIJ(a, fi + 1, j1) - PRIJ(a, i1, j1), D) + divx(PRIJ(a, i1, j1) - PRIJ(a, fi - 1, j1), D));
-        cn[a] = R(0.5) * (gc0 + gc1);
-      }
-    }
-    R jat[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) jat[k] = R(0.0);
-    /* calculate_fluxes_concentration.h:65: no y-current where gidy is 0 or MESH_Y-2 */
-    const bool yskip = !xface && ((y0 - 1 + fj) + 3 == g.my - 2);
-    R nl = R(-1.0);
-#pragma unroll
-    for (int a = 0; a < L; a++) {
-      const R s2 = cn[a] * cn[a] + gr[a] * gr[a];
-      if (s2 != R(0.0) && !yskip) {
-        const R ng = sqrt(s2);
-        if (nl < R(0.0)) nl = sqrt(cn[L] * cn[L] + gr[L] * gr[L]);
-        R sp = gr[a] * gr[L];
-        sp += cn[a] * cn[L];
-        if (nl > R(0.0)) sp /= (nl * ng);
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-          R cl1 = sm.w.u.CM[L][k][c1], cl0 = sm.w.u.CM[L][k][c0];
-          R cs1 = sm.w.u.CM[a][k][c1], cs0 = sm.w.u.CM[a][k][c0];
-          R bracket;
-          if (D.obstacle)
-            bracket = sm.w.u.SP[a][c1] * (cl1 - cs1) * sm.DP[a][c1] + sm.w.u.SP[a][c0] * (cl0 - cs0) * sm.DP[a][c0];
-          else
-            bracket = (cl1 - cs1) * sm.DP[a][c1] + (cl0 - cs0) * sm.DP[a][c0];
-          jat[k] += D.atf[a][k] * fabs(sp) * (D.obstacle ? R(0.5) : D.well_half) * bracket * gr[a] / ng;
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      if (xface) sm.w.u.JX[k][fidx] = jat[k];
-      else sm.w.u.JY[k][fidx] = jat[k];
-#pragma unroll
-      for (int l = 0; l < K; l++) {
-        R dm = (sm.w.u.DD[k][l][c1] + sm.w.u.DD[k][l][c0]) * R(0.5);
-        R gm = xface ? divx(sm.M[l][c1] - sm.M[l][c0], D) : divy(sm.M[l][c1] - sm.M[l][c0], D);
-        if (xface) sm.w.u.FX[k][l][fidx] = dm * gm;
-        else sm.w.u.FY[k][l][fidx] = dm * gm;
-      }
-    }
-  }
-  __syncthreads();
-
-  /* ---- per cell: mu update, phi commit */
-  const int tx = threadIdx.x / TY, ty = threadIdx.x - (threadIdx.x / TY) * TY;
-  const int x = x0 + tx, y = y0 + ty, i = tx + 1, j = ty + 1, c = LI(i, j);
-  const bool valid = (x < g.mx) && (y < g.my);
-  R ph[N], dp[N], m[K], nph[N], nm[K];
-  double dmu[K];
-  int oh = -1;
-  if (valid) {
-#pragma unroll
-    for (int a = 0; a < N; a++) { ph[a] = PRIJ(a, i, j); dp[a] = sm.DP[a][c]; }
-#pragma unroll
-    for (int k = 0; k < K; k++) m[k] = sm.M[k][c];
-    commit_cell<R, N, K>(D, sm.w.u.FX, sm.w.u.FY, sm.w.u.JX, sm.w.u.JY, sm.w.u.CM, sm.w.u.H, i, j, x, y, ph, dp, m,
-                         nph, nm, dmu, st, D.tgrad ? tcc[y + 3] : 0.0);
-    const long long o = (long long)x * g.pitch + y;
-#pragma unroll
-    for (int a = 0; a < N; a++) phin[a * g.plane + o] = nph[a];
-#pragma unroll
-    for (int k = 0; k < K; k++) mun[k * g.plane + o] = nm[k];
-    oh = one_hot<R, N>(nph);
-  }
-#undef PRIJ
-#undef PR
-  block_stats<R, N, K>(D, valid && stat_row(g, x), nph, nm, dp, dmu, st, ext_slot, slot,
-                       (D.tgrad && valid) ? tcc[y + 3] : 0.0);
-  return tile_flags(valid, oh, tx, ty, min(TX, g.mx - x0), min(TY, g.my - y0));
-}
-
-/* ------------------------------------------------------------------ */
 /* kernels                                                             */
 /* ------------------------------------------------------------------ */
 
@@ -789,23 +249,27 @@ __device__ __forceinline__ void step_finish(int *ctr, int ndone) {
 /* One thread per tile: the bulk test, then the tile goes on the bulk list
  * or the interface list; one atomic per warp and list.  A bulk entry holds
  * everything kf_bulk needs to start the tile: {t | phase << 28, simulation |
- * flag of the output buffer << 24, tile row << 16 | tile column, 0}.  Small CTAs (NTC threads) spread the flag reads over every SM. */
+ * flag of the output buffer << 24, tile row << 16 | tile column, 0}; an interface
+ * entry {t, simulation, tile row << 16 | tile column, 1 when the tile is full and
+ * its two-cell halo lies inside the domain (staged by one TMA box)}.  Small CTAs
+ * (NTC threads) spread the flag reads over every SM. */
 constexpr int NTC = 64;
 template <typename R>
 __global__ void __launch_bounds__(NTC) kf_classify(const SimDesc *__restrict__ sims,
                                                   const Consts<R> *__restrict__ consts, const int *__restrict__ tsim,
                                                   int ntiles, const TileFlags *__restrict__ flag_in,
                                                   const TileFlags *__restrict__ flag_outbuf,
-                                                  int *__restrict__ glist, int4 *__restrict__ blist,
+                                                  int4 *__restrict__ glist, int4 *__restrict__ blist,
                                                   int *__restrict__ ctr) {
   const int t = blockIdx.x * NTC + threadIdx.x, lane = threadIdx.x & 31;
-  int p = -1, s = 0, by = 0, bx = 0;
+  int p = -1, s = 0, by = 0, bx = 0, inside = 0;
   if (t < ntiles) {
     s = __ldg(tsim + t);
     const SimDesc &sd = sims[s];
     const int lt = t - sd.tile0;
     by = lt / sd.tiles_x;
     bx = lt - by * sd.tiles_x;
+    inside = by > 0 && by * TX + TX + 2 <= sd.g.mx && bx > 0 && bx * TY + TY + 2 <= sd.g.my;
     /* a non-isothermal simulation steps every tile as an interface tile
      * (whose pure-phase cells take the bulk update at their temperature) */
     if (!consts[s].tgrad) p = bulk_phase<R>(consts[s], sd.g, flag_in, sd.tile0, sd.tiles_x, by, bx);
@@ -824,7 +288,8 @@ __global__ void __launch_bounds__(NTC) kf_classify(const SimDesc *__restrict__ s
     if (p >= 0)
       blist[bb + __popc(mb & below)] =
           make_int4(t | (p << 28), s | (((int)flag_outbuf[t].whole & 0xff) << 24), (by << 16) | bx, 0);
-    else glist[bg + __popc(mg & below)] = t;
+    else
+      glist[bg + __popc(mg & below)] = make_int4(t, s, (by << 16) | bx, inside);
   }
 }
 
@@ -872,13 +337,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int tri
 /* x/dx and y/dy of the bulk kernel: a multiplication by the reciprocal when
  * the spacing is a power of two (MUL, chosen at launch), else the division */
 template <bool MUL, typename R>
-__device__ __forceinline__ R bdiv(R v, R inv, R d) {
+__device__ __forceinline__ R bdiv(R v, R inv, R d, unsigned span) {
   if constexpr (MUL) return v * inv;
-  else return v / d;
+  else return quick_div(v, d, inv, span);
 }
 
-/* A tensor map (CUtensorMap, 128 bytes) of the K mu planes of one simulation
- * in one state buffer: dimensions {pitch, mx, K}, box {BW, SH, K}. */
+/* Tensor maps (CUtensorMap, 128 bytes), two per simulation and state buffer:
+ * MAP_MU of the K mu planes, dimensions {pitch, mx, K}, box {BulkGeom::BW, SH, K}
+ * (bulk tiles); MAP_ALL of the N + K planes, box {ItemGeom::BW, FR, N + K}
+ * (interface items). */
+enum { MAP_MU = 0, MAP_ALL = 1, MAP_KINDS = 2 };
 struct alignas(64) TensorMapSlot {
   unsigned long long w[16];
 };
@@ -910,12 +378,16 @@ struct alignas(128) BulkWarpSmem {
   unsigned long long bar[BulkGeom<R, K>::NST];
   BulkEntry meta[BulkGeom<R, K>::NST];
 };
-/* dynamic shared memory of kf_bulk (the base is rounded up to 128 bytes in
- * the kernel) */
+/* dynamic shared memory of kf_bulk */
 template <typename R, int K>
 constexpr size_t bulk_smem_bytes() {
-  return (NT / 32) * sizeof(BulkWarpSmem<R, K>) + 128;
+  return (NTI / 32) * sizeof(BulkWarpSmem<R, K>);
 }
+/* The step kernels' dynamic shared memory (TMA boxes want 128-byte alignment).
+ * Named in every function that uses it, so that its accesses are shared-memory
+ * loads and stores: through a pointer argument, or a base rounded up as an
+ * integer, they were generic ones with 64-bit address arithmetic. */
+extern __shared__ __align__(128) unsigned char step_smem_base[];
 
 /* The FP64 bulk update of one cell (stage row i, column j) of phase p with
  * every term of the K x K matrices: the expressions of a non-DIAG kernel in
@@ -929,9 +401,10 @@ __device__ __forceinline__ void bulk_cell_full_f64(const double *__restrict__ st
   constexpr int BW = BulkGeom<double, K>::BW;
   const Consts<double> &D = *Dp;
   const double idx = D.inv_dx, idy = D.inv_dy, ddx = D.dx, ddy = D.dy, dt = D.dt;
+  const unsigned qs = D.quick_span;
   const double cst = D.obstacle ? D.jat_obst : D.jat_well;
-  double divjat = bdiv<MUL>((0.0 - 0.0) * cst, idx, ddx);
-  divjat += bdiv<MUL>((0.0 - 0.0) * cst, idy, ddy);
+  double divjat = bdiv<MUL>((0.0 - 0.0) * cst, idx, ddx, qs);
+  divjat += bdiv<MUL>((0.0 - 0.0) * cst, idy, ddy, qs);
 #define BM(l, r, c) st[((l) * SH + (r)) * BW + (c)]
   double cn[K];
 #pragma unroll
@@ -941,12 +414,12 @@ __device__ __forceinline__ void bulk_cell_full_f64(const double *__restrict__ st
     for (int l = 0; l < K; l++) {
       const double Dv = D.Dbulk[p][k][l];
       const double dm = (Dv + Dv) * 0.5, c = BM(l, i, j);
-      const double fx = dm * bdiv<MUL>(BM(l, i + 1, j) - c, idx, ddx);
-      const double bx_ = dm * bdiv<MUL>(c - BM(l, i - 1, j), idx, ddx);
-      const double fy = dm * bdiv<MUL>(BM(l, i, j + 1) - c, idy, ddy);
-      const double by_ = dm * bdiv<MUL>(c - BM(l, i, j - 1), idy, ddy);
-      divflux += bdiv<MUL>(fx - bx_, idx, ddx);
-      divflux += bdiv<MUL>(fy - by_, idy, ddy);
+      const double fx = dm * bdiv<MUL>(BM(l, i + 1, j) - c, idx, ddx, qs);
+      const double bx_ = dm * bdiv<MUL>(c - BM(l, i - 1, j), idx, ddx, qs);
+      const double fy = dm * bdiv<MUL>(BM(l, i, j + 1) - c, idy, ddy, qs);
+      const double by_ = dm * bdiv<MUL>(c - BM(l, i, j - 1), idy, ddy, qs);
+      divflux += bdiv<MUL>(fx - bx_, idx, ddx, qs);
+      divflux += bdiv<MUL>(fy - by_, idy, ddy, qs);
     }
     double cm = 0.0;   /* c_mu (functionF_01.h:30-37) */
 #pragma unroll
@@ -976,18 +449,18 @@ __device__ __forceinline__ void bulk_cell_full_f64(const double *__restrict__ st
  * (atomic max/min) when the warp moves to another simulation or finishes;
  * bulk tiles cannot move the phi extremes (their phi is 0 or 1, inside the
  * initial [0, 1]).  A stage whose bytes do not arrive within the poll limit
- * sets ctr[CTR_ERR]; the warp then stops taking tiles. */
+ * sets ctr[CTR_ERR]; the warp then stops taking tiles.  A call of its own: inlined
+ * beside the interface code it made both spill. */
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
-__device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
-                                           const int *__restrict__ tsim, const int4 *__restrict__ blist,
+__device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
+                                           const int4 *__restrict__ blist,
                                            const TensorMapSlot *__restrict__ tmaps, int buf,
                                            const R *__restrict__ state, R *__restrict__ next,
-                                           TileFlags *__restrict__ flag_out, int *__restrict__ ctr, StatBufs st,
-                                           unsigned char *smraw) {
+                                           TileFlags *__restrict__ flag_out, int *__restrict__ ctr,
+                                           const StatBufs st) {
   using G = BulkGeom<R, K>;
   constexpr int NS = 2 * N + 2 * K + 1, NST = G::NST, CO = G::CO;
-  unsigned char *sbase = (unsigned char *)(((size_t)smraw + 127) & ~(size_t)127);
-  BulkWarpSmem<R, K> &ws = reinterpret_cast<BulkWarpSmem<R, K> *>(sbase)[threadIdx.x >> 5];
+  BulkWarpSmem<R, K> &ws = reinterpret_cast<BulkWarpSmem<R, K> *>(step_smem_base)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nbulk = *(const volatile int *)(ctr + CTR_BULK);
 
@@ -1025,7 +498,7 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
    * entry r of the chunk in half h; B's entries are loaded when it is taken,
    * one 16-byte load per lane, and used one tile later. */
   constexpr int BCH = 16;
-  const int nwarps = gridDim.x * (NT / 32);
+  const int nwarps = gridDim.x * (NTI / 32);
   int q_item = 0, q_s = 0, q_xy = 0;   /* q_s: simulation | output flag << 24; q_xy: tile row << 16 | column */
   auto grab = [&](int half, int &start, int &n) {
     int v = 0, c = 0;
@@ -1077,7 +550,7 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
       ws.meta[b] = en;
       const unsigned bar = smem_addr(&ws.bar[b]);
       mbar_expect_tx(bar, G::BOX_BYTES + st.tma_extra);
-      tma_load_3d(smem_addr(&ws.st[b]), tmaps + 2 * en.s + buf, en.y0 - 1 - CO, en.x0 - 1, 0, bar);
+      tma_load_3d(smem_addr(&ws.st[b]), tmaps + (2 * en.s + buf) * MAP_KINDS + MAP_MU, en.y0 - 1 - CO, en.x0 - 1, 0, bar);
     }
   };
 
@@ -1086,6 +559,7 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
   Grid g = {};
   long long off_state = 0;
   int cur_key = -1;
+  unsigned qs = 0;
   R idx = R(0), idy = R(0), ddx = R(1), ddy = R(1), dt = R(0), divjat = R(0);
   /* the K x K constants of a phase: diffusive flux factor, c_mu, A and
    * dmu/dc */
@@ -1152,12 +626,12 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
     }
     if (cur_key != s * 16 + p) {
       cur_key = s * 16 + p;
-      idx = D.inv_dx; idy = D.inv_dy; ddx = D.dx; ddy = D.dy; dt = D.dt;
+      idx = D.inv_dx; idy = D.inv_dy; ddx = D.dx; ddy = D.dy; dt = D.dt; qs = D.quick_span;
       const R cst = D.obstacle ? D.jat_obst : D.jat_well;
       /* the anti-trapping divergence of a bulk cell: no phi gradient, the
        * same value for every cell */
-      divjat = bdiv<MUL>((R(0.0) - R(0.0)) * cst, idx, ddx);
-      divjat += bdiv<MUL>((R(0.0) - R(0.0)) * cst, idy, ddy);
+      divjat = bdiv<MUL>((R(0.0) - R(0.0)) * cst, idx, ddx, qs);
+      divjat += bdiv<MUL>((R(0.0) - R(0.0)) * cst, idy, ddy, qs);
 #pragma unroll
       for (int k = 0; k < K; k++) {
         E[k] = D.E[p][k];
@@ -1282,7 +756,7 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
         for (int l = 0; l < K; l++) {
           const double2 pp = *reinterpret_cast<const double2 *>(&sg.M[l][r0][c]);
           P[l] = *reinterpret_cast<const double2 *>(&sg.M[l][r0 + 1][c]);
-          const R g0 = bdiv<MUL>(P[l].x - pp.x, idx, ddx), g1 = bdiv<MUL>(P[l].y - pp.y, idx, ddx);
+          const R g0 = bdiv<MUL>(P[l].x - pp.x, idx, ddx, qs), g1 = bdiv<MUL>(P[l].y - pp.y, idx, ddx, qs);
 #pragma unroll
           for (int k = 0; k < K; k++)
             if (!DIAG || l == k) FXP[k][l] = make_double2(mc.dm[k][l] * g0, mc.dm[k][l] * g1);
@@ -1301,16 +775,16 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
               Pn[k] = *reinterpret_cast<const double2 *>(&sg.M[k][i + 1][c]);
               const R L = sg.M[k][i][c - 1], Rn = sg.M[k][i][c + 2];
               const R dm = mc.dm[k][k];
-              const R fx0 = dm * bdiv<MUL>(Pn[k].x - P[k].x, idx, ddx);
-              const R fx1 = dm * bdiv<MUL>(Pn[k].y - P[k].y, idx, ddx);
-              const R fl = dm * bdiv<MUL>(P[k].x - L, idy, ddy);
-              const R fm = dm * bdiv<MUL>(P[k].y - P[k].x, idy, ddy);
-              const R fr = dm * bdiv<MUL>(Rn - P[k].y, idy, ddy);
+              const R fx0 = dm * bdiv<MUL>(Pn[k].x - P[k].x, idx, ddx, qs);
+              const R fx1 = dm * bdiv<MUL>(Pn[k].y - P[k].y, idx, ddx, qs);
+              const R fl = dm * bdiv<MUL>(P[k].x - L, idy, ddy, qs);
+              const R fm = dm * bdiv<MUL>(P[k].y - P[k].x, idy, ddy, qs);
+              const R fr = dm * bdiv<MUL>(Rn - P[k].y, idy, ddy, qs);
               R a0 = R(0.0), a1 = R(0.0);
-              a0 += bdiv<MUL>(fx0 - FXP[k][k].x, idx, ddx);
-              a0 += bdiv<MUL>(fm - fl, idy, ddy);
-              a1 += bdiv<MUL>(fx1 - FXP[k][k].y, idx, ddx);
-              a1 += bdiv<MUL>(fr - fm, idy, ddy);
+              a0 += bdiv<MUL>(fx0 - FXP[k][k].x, idx, ddx, qs);
+              a0 += bdiv<MUL>(fm - fl, idy, ddy, qs);
+              a1 += bdiv<MUL>(fx1 - FXP[k][k].y, idx, ddx, qs);
+              a1 += bdiv<MUL>(fr - fm, idy, ddy, qs);
               FXP[k][k] = make_double2(fx0, fx1);
               /* c_mu, the bulk update and Mu (functionF_01.h:19-37) of the
                * pure phase, diagonal terms only */
@@ -1329,11 +803,11 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
             for (int l = 0; l < K; l++) {
               Pn[l] = *reinterpret_cast<const double2 *>(&sg.M[l][i + 1][c]);
               const R L = sg.M[l][i][c - 1], Rn = sg.M[l][i][c + 2];
-              gx0[l] = bdiv<MUL>(Pn[l].x - P[l].x, idx, ddx);
-              gx1[l] = bdiv<MUL>(Pn[l].y - P[l].y, idx, ddx);
-              gl[l] = bdiv<MUL>(P[l].x - L, idy, ddy);
-              gm[l] = bdiv<MUL>(P[l].y - P[l].x, idy, ddy);
-              gr[l] = bdiv<MUL>(Rn - P[l].y, idy, ddy);
+              gx0[l] = bdiv<MUL>(Pn[l].x - P[l].x, idx, ddx, qs);
+              gx1[l] = bdiv<MUL>(Pn[l].y - P[l].y, idx, ddx, qs);
+              gl[l] = bdiv<MUL>(P[l].x - L, idy, ddy, qs);
+              gm[l] = bdiv<MUL>(P[l].y - P[l].x, idy, ddy, qs);
+              gr[l] = bdiv<MUL>(Rn - P[l].y, idy, ddy, qs);
             }
             R df0[K], df1[K];
 #pragma unroll
@@ -1344,10 +818,10 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
                 const R dm = mc.dm[k][l];
                 const R fx0 = dm * gx0[l], fx1 = dm * gx1[l];
                 const R fl = dm * gl[l], fm = dm * gm[l], fr = dm * gr[l];
-                a0 += bdiv<MUL>(fx0 - FXP[k][l].x, idx, ddx);
-                a0 += bdiv<MUL>(fm - fl, idy, ddy);
-                a1 += bdiv<MUL>(fx1 - FXP[k][l].y, idx, ddx);
-                a1 += bdiv<MUL>(fr - fm, idy, ddy);
+                a0 += bdiv<MUL>(fx0 - FXP[k][l].x, idx, ddx, qs);
+                a0 += bdiv<MUL>(fm - fl, idy, ddy, qs);
+                a1 += bdiv<MUL>(fx1 - FXP[k][l].y, idx, ddx, qs);
+                a1 += bdiv<MUL>(fr - fm, idy, ddy, qs);
                 FXP[k][l] = make_double2(fx0, fx1);
               }
               df0[k] = a0;
@@ -1522,9 +996,8 @@ __device__ __forceinline__ void bulk_tiles(const SimDesc *__restrict__ sims, con
  * afterwards: its stage barriers are invalidated (every box it issued has
  * completed or been waited for). */
 template <typename R, int K>
-__device__ __forceinline__ void bulk_release_warp(unsigned char *smraw) {
-  unsigned char *sbase = (unsigned char *)(((size_t)smraw + 127) & ~(size_t)127);
-  BulkWarpSmem<R, K> &ws = reinterpret_cast<BulkWarpSmem<R, K> *>(sbase)[threadIdx.x >> 5];
+__device__ __forceinline__ void bulk_release_warp() {
+  BulkWarpSmem<R, K> &ws = reinterpret_cast<BulkWarpSmem<R, K> *>(step_smem_base)[threadIdx.x >> 5];
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
     for (int q = 0; q < BulkGeom<R, K>::NST; q++)
@@ -1534,99 +1007,496 @@ __device__ __forceinline__ void bulk_release_warp(unsigned char *smraw) {
 }
 
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
-__global__ void __launch_bounds__(NT, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
-                                                 const int *__restrict__ tsim, const int4 *__restrict__ blist,
-                                                 const TensorMapSlot *__restrict__ tmaps, int buf,
-                                                 const R *__restrict__ state, R *__restrict__ next,
-                                                 TileFlags *__restrict__ flag_out, int *__restrict__ ctr,
-                                                 int ndone, StatBufs st) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, tsim, blist, tmaps, buf, state, next, flag_out, ctr, st, smraw);
+__global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk(
+    const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist,
+    const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
+    TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
   step_finish(ctr, ndone);
 }
 
-/* Interface tiles of one step: the CTA takes tiles from the interface list
- * until it is empty.  Each simulation's constants are copied into shared
- * memory when the CTA moves to it.  Not inlined: the step kernel and the
- * interface-only kernel share one copy of this code. */
-template <typename R, int N, int K, bool ANISO, bool MUL>
-__device__ __noinline__ void general_tiles(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
-                                           const int *__restrict__ tsim, const R *__restrict__ state,
-                                           R *__restrict__ next, TileFlags *__restrict__ flag_out,
-                                           const int *__restrict__ glist, int *__restrict__ ctr, StatBufs st,
-                                           unsigned char *smraw) {
-  GenSmem<R, N, K> &sm = *reinterpret_cast<GenSmem<R, N, K> *>(smraw);
-  __shared__ Consts<R> sc;
-  __shared__ int s_item;
-  const int nlist = *(volatile int *)(ctr + CTR_LIST);
-  int cur_sim = -1;
-  if (threadIdx.x == 0) {   /* the tile's list counters (reset again after each tile) */
-    sm.nlist = 0;
-    sm.nflist = 0;
-  }
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(ctr + CTR_HEAD, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= nlist) break;
-    const int t = __ldg(glist + item);
-    const int s = __ldg(tsim + t);
-    if (s != cur_sim) {
-      load_consts(sc, consts + s);
-      cur_sim = s;
-      __syncthreads();
-    }
-    const SimDesc sd = sims[s];
-    const int lt = t - sd.tile0, by = lt / sd.tiles_x, bx = lt - by * sd.tiles_x;
-    const R *ph = state + sd.off_state;
-    R *nx = next + sd.off_state;
-    using CT = typename std::conditional<MUL, ConstsMul<R>, Consts<R>>::type;
-    const double *tpf = st.trows ? st.trows + sd.off_T : nullptr;
-    const double *tcc = tpf ? tpf + (sd.g.my + 6) : nullptr;
-    const TileFlags f = general_tile<R, N, K, ANISO>(static_cast<const CT &>(sc), sd.g, ph, ph + (long long)N * sd.g.plane, nx,
-                                                       nx + (long long)N * sd.g.plane, by * TX, bx * TY, st, s, t,
-                                                       sm, tpf, tcc);
-    if (threadIdx.x == 0) flag_out[t] = f;
-    __syncthreads();
-  }
+/* an interface tile's shared memory */
+template <typename R, int N, int K>
+struct TileSmem32 : ItemCommon<R, N, K> {
+  ItemSmem32<R, N, K> t;
+};
+template <typename R, int N, int K, bool ANISO>
+using TileSmem = typename std::conditional<sizeof(R) == 8, ItemSmem<R, N, K, ANISO>, TileSmem32<R, N, K>>::type;
+
+/* What a step kernel needs of a batch of one, as a kernel parameter: constants
+ * and layout then come from the constant bank, as operands of the arithmetic.
+ * Batches of several simulations read them from global memory (SOLO false). */
+template <typename R, bool SOLO>
+struct StepArgs {};
+template <typename R>
+struct StepArgs<R, true> {
+  Consts<R> c;
+  SimDesc sd;
+};
+template <typename R, bool SOLO>
+__device__ __forceinline__ const Consts<R> &pick_consts(const StepArgs<R, SOLO> &args, const Consts<R> *sc) {
+  if constexpr (SOLO) return args.c;
+  else return *sc;
 }
 
-template <typename R, int N, int K, bool ANISO, bool MUL>
-__global__ void __launch_bounds__(NT, (N <= 3 ? 2 : 1)) kf_general(const SimDesc *__restrict__ sims,
-                                                 const Consts<R> *__restrict__ consts, const int *__restrict__ tsim,
-                                                 const R *__restrict__ state, R *__restrict__ next,
-                                                 TileFlags *__restrict__ flag_out, const int *__restrict__ glist,
-                                                 int *__restrict__ ctr, int ndone, StatBufs st) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  general_tiles<R, N, K, ANISO, MUL>(sims, consts, tsim, state, next, flag_out, glist, ctr, st, smraw);
+/* Interface tiles of one step: the CTA takes tiles from the interface list
+ * until it is empty, the next one's box in flight while one is stepped.  TG: some
+ * simulation is non-isothermal.  A box whose bytes do not arrive within the poll
+ * limit sets ctr[CTR_ERR]; the CTA then stops taking tiles. */
+template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
+__device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, const SimDesc *__restrict__ sims,
+                                              const Consts<R> *__restrict__ consts,
+                                              const TensorMapSlot *__restrict__ tmaps, int buf,
+                                              const R *__restrict__ state, R *__restrict__ next,
+                                              TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                              int *__restrict__ ctr, const StatBufs &st) {
+  using CT = typename std::conditional<MUL, ConstsMul<R>, Consts<R>>::type;
+  using IG = ItemGeom<R>;
+  constexpr int CO = IG::CO, NWI = NTI / 32;
+  constexpr unsigned BOX_BYTES = (unsigned)((N + K) * FR * IG::BW * sizeof(R));
+  const int nlist = *(volatile int *)(ctr + CTR_LIST);
+  if (nlist == 0) return;
+  using SM = TileSmem<R, N, K, ANISO>;
+  SM &sm = *reinterpret_cast<SM *>(step_smem_base);
+  __shared__ __align__(16) unsigned char sc_raw[SOLO ? 16 : sizeof(Consts<R>)];
+  Consts<R> *const scp = reinterpret_cast<Consts<R> *>(sc_raw);
+  const CT &D = static_cast<const CT &>(pick_consts<R, SOLO>(args, scp));
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  /* thread 0: note an entry in slot c and start its box */
+  auto issue = [&](const int4 &en, int c) {
+    sm.ent[c] = en;
+    if (en.x >= 0 && en.w) {
+      const unsigned bar = smem_addr(&sm.bar[c]);
+      mbar_expect_tx(bar, BOX_BYTES + st.tma_extra);
+      tma_load_3d(smem_addr(&sm.F[c]), tmaps + (2 * en.y + buf) * MAP_KINDS + MAP_ALL, (en.z & 0xffff) * TY - 2 - CO,
+                  (en.z >> 16) * TX - 2, 0, bar);
+    }
+  };
+  if (tid == 0) {
+    mbar_init(smem_addr(&sm.bar[0]), 1);
+    mbar_init(smem_addr(&sm.bar[1]), 1);
+    fence_barrier_init();
+    fence_proxy_async_smem();
+    if constexpr (sizeof(R) == 8) sm.n_test = sm.n_act = sm.n_task = sm.n_extra = sm.n_j = 0;
+    else sm.t.nlist = sm.t.nflist = 0;
+    const int i = atomicAdd(ctr + CTR_HEAD, 1);
+    issue(i < nlist ? __ldg(glist + i) : make_int4(-1, 0, 0, 0), 0);
+  }
+  int cur_sim = -1;
+  unsigned parity = 0;   /* bit c: the phase of slot c's barrier its next box completes */
+  Grid g = {};
+  long long off_state = 0;
+  const double *tpf = nullptr, *tcc = nullptr;
+  __syncthreads();
+#pragma unroll 1
+  for (int cur = 0;; cur ^= 1) {
+    const int4 en = sm.ent[cur];
+    if (en.x < 0) break;
+    const int t = en.x, s = SOLO ? 0 : en.y, x0 = (en.z >> 16) * TX, y0 = (en.z & 0xffff) * TY;
+    int nxt = 0;
+    if (tid == 0) nxt = atomicAdd(ctr + CTR_HEAD, 1);   /* used after the next barrier */
+    if (s != cur_sim) {
+      cur_sim = s;
+      if constexpr (!SOLO) {
+        const int *src = reinterpret_cast<const int *>(consts + s);
+        int *dst = reinterpret_cast<int *>(scp);
+        for (int w = tid; w < (int)(sizeof(Consts<R>) / sizeof(int)); w += NTI) dst[w] = __ldg(src + w);
+      }
+      if (tid < 2 * (N + K)) {
+        const long long o = st.ext ? *(volatile long long *)(st.ext + (long long)s * (2 * (N + K)) + tid) : 0;
+        sm.ext[tid] = __longlong_as_double(o < 0 ? o ^ 0x7fffffffffffffffLL : o);
+      }
+      if constexpr (SOLO) {
+        g = args.sd.g;
+        off_state = args.sd.off_state;
+      } else {
+        const SimDesc sd = sims[s];
+        g = sd.g;
+        off_state = sd.off_state;
+        if (TG && st.trows) {
+          tpf = st.trows + sd.off_T;
+          tcc = tpf + (g.my + 6);
+        }
+      }
+      __syncthreads();
+    }
+    R(&F)[N + K][FR][IG::BW] = sm.F[cur];
+    bool ok = true;
+    if (en.w) {
+      ok = mbar_wait(smem_addr(&sm.bar[cur]), (parity >> cur) & 1u, st.mbar_tries);
+      parity ^= 1u << cur;
+    } else {
+      /* rows and columns of the frame after the boundary remap of phi and mu;
+       * -1 where no needed cell lies (phi: [-2, m+1], mu: [-1, m]) */
+      if (tid < 2 * (FR + FC)) {
+        const int f = tid / (FR + FC), u = tid - f * (FR + FC), reach = 2 - f;
+        if (u < FR) {
+          const int x = x0 - 2 + u;
+          sm.row[f][u] = (x >= -reach && x < g.mx + reach) ? remap(x, g.mx, D.bc_x[f][0], D.bc_x[f][1]) * g.pitch : -1;
+        } else {
+          const int y = y0 - 2 + (u - FR);
+          sm.col[f][u - FR] = (y >= -reach && y < g.my + reach) ? remap(y, g.my, D.bc_y[f][0], D.bc_y[f][1]) : -1;
+        }
+      }
+      __syncthreads();
+      const R *src = state + off_state;
+      for (int q = tid; q < FR * FC; q += NTI) {
+        const int i = q / FC, j = q - i * FC;
+        const int r = sm.row[0][i], c = sm.col[0][j], rm = sm.row[1][i], cm = sm.col[1][j];
+#pragma unroll
+        for (int a = 0; a < N; a++) F[a][i][j + CO] = (r >= 0 && c >= 0) ? __ldg(src + a * g.plane + (r + c)) : R(0.0);
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          F[N + k][i][j + CO] = (rm >= 0 && cm >= 0) ? __ldg(src + (N + k) * g.plane + (rm + cm)) : R(0.0);
+      }
+      fence_proxy_async_smem();   /* before a later box overwrites this slot */
+      __syncthreads();
+    }
+
+    const int tx = wid, ty = lane, x = x0 + tx, y = y0 + ty;
+    const bool valid = x < g.mx && y < g.my;
+    R dp[N], nph[N], nm[K];
+    double dmu[K];
+    const double Tc = (TG && D.tgrad && valid) ? tcc[y + 3] : 0.0;
+    if constexpr (sizeof(R) == 4) {
+      if (!__syncthreads_and(ok)) {
+        if (tid == 0) atomicExch(ctr + CTR_ERR, 1);
+        break;   /* no other box is in flight */
+      }
+      int4 nent = make_int4(-1, 0, 0, 0);
+      if (tid == 0 && nxt < nlist) nent = __ldg(glist + nxt);
+      tile32<R, N, K, ANISO>(D, g, F, x0, y0, st, sm.t, tpf, tcc, dp, nph, nm, dmu, [&]() {
+        if (tid == 0) issue(nent, cur ^ 1);   /* the other slot was last read a tile ago */
+      });
+    } else {
+    /* ---- ring cells, a warp per row and one for the last two columns: a constant
+     * 5-point stencil has no active phase (delta-phi is 0, or the projection's clamp
+     * of a negative phi), the others are listed; D; whether the fields are of
+     * ordinary size (left-out terms are then +-0) */
+    bool tame = true;
+    for (int rt = wid; rt < RR + 1; rt += NWI) {
+      const int ri = rt < RR ? rt : lane >> 1, rj = rt < RR ? lane : 32 + (lane & 1);
+      const bool in = rt < RR || lane < 2 * RR;
+      const int i = ri + 1, j = rj + 1, e = RI(ri, rj);
+      const bool vd = in && (x0 - 1 + ri <= g.mx) && (y0 - 1 + rj <= g.my);
+      bool nu = false;
+      R p[N];
+#pragma unroll
+      for (int a = 0; a < N; a++) p[a] = R(0.0);
+      if (vd) {
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          p[a] = F[a][i][j + CO];
+          tame = tame && fabs(p[a]) < R(1e18);
+          nu = nu || !(F[a][i + 1][j + CO] == p[a] && F[a][i - 1][j + CO] == p[a] && F[a][i][j + 1 + CO] == p[a] &&
+                       F[a][i][j - 1 + CO] == p[a]);
+        }
+#pragma unroll
+        for (int k = 0; k < K; k++) tame = tame && fabs(F[N + k][i][j + CO]) < R(1e18);
+        /* (a constant stencil between phases is listed too, for its anti-trapping weights) */
+#pragma unroll
+        for (int a = 0; a < N - 1; a++) nu = nu || !(p[a] == R(0.0) || p[a] == R(1.0));
+      }
+      if (in) {
+        if (!nu) {
+          sm.ACT[e] = 0;
+#pragma unroll
+          for (int a = 0; a < N; a++) {
+            R d = R(0.0);
+            if ((p[a] + d) < R(0.0)) d += fabs(d + p[a]);
+            sm.DP[a][e] = d;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < K; k++)
+#pragma unroll
+          for (int l = 0; l < K; l++) {
+            if (k != l && st.diag) continue;
+            R v = R(0.0);
+#pragma unroll
+            for (int b = 0; b < N; b++)
+#pragma unroll
+              for (int n = 0; n < K; n++)
+                if (n == k || !st.diag) v += D.DC[b][k][l][n] * p[b];
+            sm.DD[k][l][e] = v;
+          }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, nu);
+      if (lane == 0) {
+        if (rt < RR) sm.NU[rt] = m;
+        else sm.NUX = m;
+      }
+      if (m) {
+        int b = 0;
+        if (lane == 0) b = atomicAdd(&sm.n_test, __popc(m));
+        b = __shfl_sync(0xffffffffu, b, 0);
+        if (nu) sm.TEST[b + __popc(m & ((1u << lane) - 1u))] = (short)e;
+      }
+    }
+    tame = __syncthreads_and(ok && tame);
+    if (!tame) {
+      if (!__syncthreads_and(ok)) {
+        if (tid == 0) atomicExch(ctr + CTR_ERR, 1);
+        break;   /* no other box is in flight */
+      }
+      if (K > 1 && st.diag) {   /* the off-diagonal D left out above */
+        for (int e = tid; e < RS; e += NTI) {
+          R p[N];
+#pragma unroll
+          for (int a = 0; a < N; a++) p[a] = F[a][e / RC + 1][e % RC + 1 + CO];
+#pragma unroll
+          for (int k = 0; k < K; k++)
+#pragma unroll
+            for (int l = 0; l < K; l++) sm.DD[k][l][e] = Dcell<R, N, K>(D, p, k, l);
+        }
+        __syncthreads();
+      }
+    }
+    const bool dg = st.diag && tame;
+    int4 nent = make_int4(-1, 0, 0, 0);
+    if (tid == 0 && nxt < nlist) nent = __ldg(glist + nxt);
+
+    /* ---- listed cells: active phases */
+    const int ntest = sm.n_test;
+    for (int q0 = 32 * wid; q0 < ntest; q0 += NTI) {
+      const int q = q0 + lane;
+      unsigned mask = 0;
+      int e = 0;
+      if (q < ntest) {
+        e = sm.TEST[q];
+        const int ri = e / RC, rj = e - ri * RC, i = ri + 1, j = rj + 1;
+        R p[N];
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          p[a] = F[a][i][j + CO];
+          const R xp = F[a][i + 1][j + CO], xm = F[a][i - 1][j + CO], yp = F[a][i][j + 1 + CO],
+                  ym = F[a][i][j - 1 + CO];
+          /* a phase that is zero on the stencil is not active */
+          if (N > 2 && p[a] == R(0.0) && xp == R(0.0) && xm == R(0.0) && yp == R(0.0) && ym == R(0.0)) continue;
+          R dv = divx(divx(xp - p[a], D) - divx(p[a] - xm, D), D);
+          dv += divy(divy(yp - p[a], D) - divy(p[a] - ym, D), D);
+          if (fabs(dv) > R(0.0)) mask |= 1u << a;
+        }
+        sm.ACT[e] = (unsigned char)mask;
+        if (!mask) {
+#pragma unroll
+          for (int a = 0; a < N; a++) {
+            R d = R(0.0);
+            if ((p[a] + d) < R(0.0)) d += fabs(d + p[a]);
+            sm.DP[a][e] = d;
+          }
+        }
+        if (D.obstacle) {
+          /* a solid between 0 and 1 that is not active (the active ones' weights come with the lambdas) */
+#pragma unroll 1
+          for (int a = 0; a < N - 1; a++) {
+            const R pa = F[a][i][j + CO];
+            if (!((mask >> a) & 1u) && pa * (R(1.0) - pa) > R(0.0)) sm.SP[a][e] = item_sphi<R, N, K>(F, i, j, a);
+          }
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, mask != 0);
+      if (m) {
+        unsigned ma[N];
+        int nt = 0, b = 0, bt = 0;
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          ma[a] = __ballot_sync(0xffffffffu, (mask >> a) & 1u);
+          nt += __popc(ma[a]);
+        }
+        if (lane == 0) {
+          b = atomicAdd(&sm.n_act, __popc(m));
+          bt = atomicAdd(&sm.n_task, nt);
+        }
+        b = __shfl_sync(0xffffffffu, b, 0);
+        bt = __shfl_sync(0xffffffffu, bt, 0);
+        const unsigned below = (1u << lane) - 1u;
+        if (mask) sm.LIST[b + __popc(m & below)] = (short)e;
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          if ((mask >> a) & 1u) sm.TASK[bt + __popc(ma[a] & below)] = (short)(e | (a << 10));
+          bt += __popc(ma[a]);
+        }
+      }
+    }
+    /* ---- faces next to a cell with a varying stencil, a warp per row of faces */
+    for (int q = wid; q < 2 * TX + 1; q += NWI) {
+      const int r = q <= TX ? q : q - TX;   /* ring row; x-faces lie between it and the next one */
+      const unsigned long long a = sm.NU[r] | (unsigned long long)((sm.NUX >> (2 * r)) & 3u) << 32;
+      unsigned long long w;
+      if (q <= TX) {
+        const unsigned long long c = sm.NU[r + 1] | (unsigned long long)((sm.NUX >> (2 * r + 2)) & 3u) << 32;
+        w = ((a | c) >> 1) & 0xffffffffull;
+      } else {
+        w = (a | (a >> 1)) & 0x1ffffffffull;
+      }
+      const unsigned lo = (unsigned)w;
+      int b = 0;
+      if (lane == 0) {
+        sm.JW[q] = w;
+        if (w) b = atomicAdd(&sm.n_j, __popcll(w));
+      }
+      if (w) {
+        b = __shfl_sync(0xffffffffu, b, 0);
+        const int f = q <= TX ? q * TY : JXF + (q - TX - 1) * (TY + 1);
+        if ((lo >> lane) & 1u) sm.JLIST[b + __popc(lo & ((1u << lane) - 1u))] = (short)(f + lane);
+        if (lane == 0 && (w >> 32)) sm.JLIST[b + __popc(lo)] = (short)(f + TY);
+      }
+    }
+    __syncthreads();
+    const int nact = sm.n_act, ntask = sm.n_task;
+    if (tid == 0) issue(nent, cur ^ 1);   /* the other slot was last read a tile ago */
+    if (ANISO && nact > 0) {
+      /* the faces of active cells, each once: forward x and right y of every
+       * cell, and the backward ones whose other cell is not active */
+      for (int q0 = 32 * wid; q0 < nact; q0 += NTI) {
+        const int q = q0 + lane;
+        bool bx_ = false, by_ = false;
+        int ri = 0, rj = 0;
+        if (q < nact) {
+          const int e = sm.LIST[q];
+          ri = e / RC;
+          rj = e - ri * RC;
+          sm.FLIST[q] = (short)((ri + 1) * RC + rj);
+          sm.FLIST[nact + q] = (short)(IXF + ri * (TY + 3) + rj + 1);
+          bx_ = ri == 0 || !sm.ACT[e - RC];
+          by_ = rj == 0 || !sm.ACT[e - 1];
+        }
+        const unsigned mx_ = __ballot_sync(0xffffffffu, bx_), my_ = __ballot_sync(0xffffffffu, by_);
+        int b = 0;
+        if (lane == 0) b = atomicAdd(&sm.n_extra, __popc(mx_) + __popc(my_));
+        b = 2 * nact + __shfl_sync(0xffffffffu, b, 0);
+        const unsigned below = (1u << lane) - 1u;
+        if (bx_) sm.FLIST[b + __popc(mx_ & below)] = (short)(ri * RC + rj);
+        if (by_) sm.FLIST[b + __popc(mx_) + __popc(my_ & below)] = (short)(IXF + ri * (TY + 3) + rj);
+      }
+      __syncthreads();
+      const int nf = 2 * nact + sm.n_extra;
+      for (int q = tid; q < nf; q += NTI) item_face<R, N, K, ANISO>(D, F, sm, sm.FLIST[q]);
+      __syncthreads();
+    }
+    {
+      /* lambda of each active (cell, phase), and on the threads after them the
+       * anti-trapping weights of the active cells' solids */
+      const int t32 = (ntask + 31) & ~31, all = D.obstacle ? t32 + nact : ntask;
+      for (int q = tid; q < all; q += NTI) {
+        if (q < ntask) {
+          const int v = sm.TASK[q], e = v & 1023;
+          item_lambda<R, N, K, ANISO, TG>(D, F, sm, e, v >> 10, tame, dg,
+                                          TG && D.tgrad ? tpf[y0 - 1 + e % RC + 3] : 0.0);
+        } else if (q >= t32) {
+          const int e = sm.LIST[q - t32], ri = e / RC, rj = e - ri * RC;
+          const unsigned act = sm.ACT[e];
+#pragma unroll 1
+          for (int a = 0; a < N - 1; a++) {
+            const R p = F[a][ri + 1][rj + 1 + CO];
+            if (((act >> a) & 1u) && p * (R(1.0) - p) > R(0.0)) sm.SP[a][e] = item_sphi<R, N, K>(F, ri + 1, rj + 1, a);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    const int nj = sm.n_j;
+    for (int q = tid; q < nact; q += NTI) item_dphi<R, N, K, ANISO>(D, F, sm, sm.LIST[q]);
+    __syncthreads();
+    if (tid == 0) sm.n_test = sm.n_act = sm.n_task = sm.n_extra = sm.n_j = 0;   /* for the next tile */
+    if (st.dphi_out) {
+      /* the adjoint's tape: the delta-phi of the tile and of its ring cells
+       * (the domain's ring included), as the reverse sweep reads it */
+      for (int e = tid; e < RS; e += NTI) {
+        const int x = x0 - 1 + e / RC, y = y0 - 1 + e % RC;
+        if (x <= g.mx && y <= g.my) {
+#pragma unroll
+          for (int a = 0; a < N; a++)
+            st.dphi_out[a * g.dplane + (long long)(x + 1) * g.dpitch + (y + 1)] = (double)sm.DP[a][e];
+        }
+      }
+    }
+    if (nj > 0) {
+      for (int q = tid; q < nj; q += NTI)
+        item_current<R, N, K, ANISO, TG>(D, F, sm, sm.JLIST[q], y0, g.my, dg, tcc);
+      __syncthreads();
+    }
+
+    /* ---- per cell: mu update, phi commit */
+    if (valid) {
+      R ph[N], m[K];
+#pragma unroll
+      for (int a = 0; a < N; a++) {
+        ph[a] = F[a][tx + 2][ty + 2 + CO];
+        dp[a] = sm.DP[a][RI(tx + 1, ty + 1)];
+      }
+#pragma unroll
+      for (int k = 0; k < K; k++) m[k] = F[N + k][tx + 2][ty + 2 + CO];
+      item_commit<R, N, K, ANISO, TG>(D, F, sm, tx, ty, x, y, tame, dg, ph, dp, m, nph, nm, dmu, Tc);
+    }
+    }
+    int oh = -1;
+    if (valid) {
+      R *out = next + off_state + (long long)x * g.pitch + y;
+#pragma unroll
+      for (int a = 0; a < N; a++) out[a * g.plane] = nph[a];
+#pragma unroll
+      for (int k = 0; k < K; k++) out[(N + k) * g.plane] = nm[k];
+      oh = one_hot<R, N>(nph);
+      if (st.ext && stat_row(g, x)) item_extremes<R, N, K>(sm.ext, nph, nm, st, s);
+    }
+    {
+      const unsigned b = row_flag_bits<N>(valid, oh);
+      if (lane == 0) sm.fm[cur][wid] = b;
+    }
+    if (st.want_sums) item_sums<R, N, K, TG>(D, valid && stat_row(g, x), nph, nm, dp, dmu, st, t, Tc);
+    __syncthreads();   /* the tile's shared memory is free, its rows' flag bits are written */
+    if (tid == 32) flag_out[t] = flags_of_rows(sm.fm[cur]);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(&sm.bar[0])) : "memory");
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(&sm.bar[1])) : "memory");
+  }
+  __syncthreads();
+}
+
+/* CTAs of the interface code an SM holds: what its shared memory leaves, at most two (128 registers a thread) */
+template <typename R, int N, int K, bool ANISO>
+constexpr int item_ctas() {
+  constexpr size_t need = sizeof(TileSmem<R, N, K, ANISO>) + 128 + sizeof(Consts<R>) + 2048;
+  constexpr int n = (int)(228 * 1024 / need);
+  return n < 1 ? 1 : (n > 2 ? 2 : n);
+}
+
+template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
+__global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
+    const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
+    const Consts<R> *__restrict__ consts, const TensorMapSlot *__restrict__ tmaps, int buf,
+    const R *__restrict__ state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
+    const int4 *__restrict__ glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
   step_finish(ctr, ndone);
 }
 
 /* One step in one persistent launch: each CTA takes interface tiles while
  * the interface list lasts, then its warps take bulk tiles, so the two kinds
- * of work share the SMs and the step ends with one tail instead of two. */
-template <typename R, int N, int K, bool ANISO, bool MUL, bool DIAG>
-__global__ void __launch_bounds__(NT, (N <= 3 ? 2 : 1)) kf_step(const SimDesc *__restrict__ sims,
-                                                 const Consts<R> *__restrict__ consts, const int *__restrict__ tsim,
-                                                 const int4 *__restrict__ blist, const int *__restrict__ glist,
-                                                 const TensorMapSlot *__restrict__ tmaps, int buf,
-                                                 const R *__restrict__ state, R *__restrict__ next,
-                                                 TileFlags *__restrict__ flag_out, int *__restrict__ ctr,
-                                                 int ndone, StatBufs st) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  if (st.mixed && (blockIdx.x & 1)) {
-    /* bulk tiles first, then whatever is left of the interface list: the two
-     * kinds of work share every SM from the start of the step */
-    bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, tsim, blist, tmaps, buf, state, next, flag_out, ctr, st,
-                                          smraw);
-    bulk_release_warp<R, K>(smraw);
-    __syncthreads();   /* the bulk stages' shared memory becomes the interface tile's */
-    general_tiles<R, N, K, ANISO, MUL>(sims, consts, tsim, state, next, flag_out, glist, ctr, st, smraw);
-  } else {
-    general_tiles<R, N, K, ANISO, MUL>(sims, consts, tsim, state, next, flag_out, glist, ctr, st, smraw);
-    __syncthreads();   /* the interface tiles' shared memory becomes the bulk stages */
-    bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, tsim, blist, tmaps, buf, state, next, flag_out, ctr, st,
-                                          smraw);
+ * of work share the SMs and the step ends with one tail instead of two.  In a
+ * mixed shape the odd CTAs take them the other way round: the two kinds of work
+ * then share every SM from the start of the step. */
+template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO, bool DIAG>
+__global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
+    const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
+    const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist, const int4 *__restrict__ glist,
+    const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
+    TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  const int bulk_pass = st.mixed && (blockIdx.x & 1) ? 0 : 1;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    if (pass == bulk_pass) {
+      bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
+      bulk_release_warp<R, K>();
+    } else {
+      general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr,
+                                                   st);
+    }
+    __syncthreads();   /* the pass's shared memory becomes the next one's */
   }
   step_finish(ctr, ndone);
 }
@@ -1777,16 +1647,16 @@ __global__ void __launch_bounds__(NT) ks_shift(const SimDesc *__restrict__ sims,
 }
 
 /* Flags of every tile of a state buffer from its phi (after an upload,
- * smoothing or gp_batch_set). */
+ * smoothing or gp_batch_set); a warp per tile row. */
 template <typename R, int N>
 __global__ void __launch_bounds__(NT) kf_flags(const SimDesc *__restrict__ sims, const int *__restrict__ tsim,
                                                const R *__restrict__ state, TileFlags *__restrict__ flags) {
+  __shared__ unsigned s_w[TX];
   const int t = blockIdx.x;
   const SimDesc sd = sims[__ldg(tsim + t)];
   const int lt = t - sd.tile0, by = lt / sd.tiles_x, bx = lt - by * sd.tiles_x;
-  const int tx = threadIdx.x / TY, ty = threadIdx.x - (threadIdx.x / TY) * TY;
-  const int x = by * TX + tx, y = bx * TY + ty;
-  const bool valid = (x < sd.g.mx) && (y < sd.g.my);
+  const int w = threadIdx.x / TY, lane = threadIdx.x - w * TY, x = by * TX + w, y = bx * TY + lane;
+  const bool valid = x < sd.g.mx && y < sd.g.my;
   int oh = -1;
   if (valid) {
     R ph[N];
@@ -1794,8 +1664,10 @@ __global__ void __launch_bounds__(NT) kf_flags(const SimDesc *__restrict__ sims,
     for (int a = 0; a < N; a++) ph[a] = __ldg(state + sd.off_state + a * sd.g.plane + (long long)x * sd.g.pitch + y);
     oh = one_hot<R, N>(ph);
   }
-  const TileFlags f = tile_flags(valid, oh, tx, ty, min(TX, sd.g.mx - by * TX), min(TY, sd.g.my - bx * TY));
-  if (threadIdx.x == 0) flags[t] = f;
+  const unsigned b = row_flag_bits<N>(valid, oh);
+  if (lane == 0) s_w[w] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) flags[t] = flags_of_rows(s_w);
 }
 
 }  // namespace gpd

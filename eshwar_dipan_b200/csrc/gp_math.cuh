@@ -19,10 +19,12 @@ namespace gpd {
  * meaning), plus FP64 copies of cmu (dc/dmu of each phase, for the inversion
  * of the FP32 form) and of its inverse muc (dmu/dc of each phase: 2A on the
  * diagonal, A off it; the FP32 form's bulk update). */
+constexpr unsigned QUICK_SPAN = 1800;   /* exponents of quick_div's dividends, from 2^-900 on */
 template <typename R>
 struct Consts {
   R dx, dy, dt, eps, inv_eps, tau, c16pi2, jat_obst, jat_well, well_half;
   R inv_dx, inv_dy, inv_2dy;   /* used instead of dividing when mul_dx/mul_dy are set */
+  unsigned quick_span;         /* quick_div's range of dividends: QUICK_SPAN, or 0 for an extreme spacing */
   int mul_dx, mul_dy;          /* FP64: dx (dy) is a power of two, so x*(1/dx) == x/dx exactly */
   int obstacle, well, aniso, inv_mode, rot_identity;
   int bc_x[2][2], bc_y[2][2];
@@ -294,7 +296,10 @@ __device__ __forceinline__ void project(const R *ph, const bool *act, R *d) {
     for (int b = 0; b < N; b++)
       if (act[b] && ((ph[b] + d[b]) > R(0.0)) && ((ph[b] + d[b]) < R(1.0))) {
         if (fabs(sum_phib) > R(0.0)) d[b] -= Dphi * (ph[b]) / (sum_phib);
-        else d[b] -= Dphi / (R)(count);
+        /* count 0: a phase just lifted to 0 that rounding left above it.  The
+         * reference divides by it; the FP32 form, where it happens to phi of
+         * 1e-18 beside 1.0, leaves the phase as lifted */
+        else if (sizeof(R) == 8 || count > 0) d[b] -= Dphi / (R)(count);
       }
   }
   int hit = -1;
@@ -302,10 +307,13 @@ __device__ __forceinline__ void project(const R *ph, const bool *act, R *d) {
   for (int a = 0; a < N; a++)
     if (hit < 0 && act[a] && (ph[a] + d[a]) > R(1.0)) hit = a;
   if (hit >= 0) {
-    d[hit] = (R(1.0) - ph[hit]);
+    /* d[hit] = 1 - ph[hit], the other active phases -ph (by compile-time
+     * indices: the arrays stay in registers) */
 #pragma unroll
-    for (int b = 0; b < N; b++)
-      if (act[b] && b != hit) d[b] = -ph[b];
+    for (int b = 0; b < N; b++) {
+      if (b == hit) d[b] = (R(1.0) - ph[b]);
+      else if (act[b]) d[b] = -ph[b];
+    }
   }
 }
 

@@ -72,12 +72,41 @@ __device__ __forceinline__ int remap(int v, int m, int tlo, int thi) {
   return src - 3;
 }
 
+/* v / d for a divisor known in advance, r = RN(1/d): the correctly rounded
+ * quotient in five multiply-adds (Markstein, "Computation of elementary functions
+ * on the IBM RISC System/6000 processor", 1990, theorem on q' = RN(q + r * RN(v - d q)):
+ * with r correctly rounded and q within one ulp of the quotient, q' is the
+ * correctly rounded quotient).  The first pass brings v * r (off by up to 1.5 ulp)
+ * within that; v outside [2^-900, 2^900) and not zero, where a product could
+ * leave the normal range, takes the division, and so does every v when d is
+ * outside [2^-60, 2^60) (span 0 instead of QUICK_SPAN, set on the host).  The interface tile of a 1.5-spaced grid spent half its time in
+ * these divisions. */
+/* out of line: inlined at every division it doubled the code of the tile */
+static __device__ __noinline__ double slow_div(double v, double d) { return v / d; }
+__device__ __forceinline__ double quick_div(double v, double d, double r, unsigned span) {
+  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+  double q = v * r;
+  if (e - 123u < span) {
+    q = __fma_rn(__fma_rn(-q, d, v), r, q);
+    q = __fma_rn(__fma_rn(-q, d, v), r, q);
+  } else if (v != 0.0) {
+    q = slow_div(v, d);
+  }
+  return q;
+}
+__device__ __forceinline__ float quick_div(float v, float d, float, unsigned) { return v / d; }
 template <typename R>
-__device__ __forceinline__ R divx(R v, const Consts<R> &D) { return D.mul_dx ? v * D.inv_dx : v / D.dx; }
+__device__ __forceinline__ R divx(R v, const Consts<R> &D) {
+  return D.mul_dx ? v * D.inv_dx : quick_div(v, D.dx, D.inv_dx, D.quick_span);
+}
 template <typename R>
-__device__ __forceinline__ R divy(R v, const Consts<R> &D) { return D.mul_dy ? v * D.inv_dy : v / D.dy; }
+__device__ __forceinline__ R divy(R v, const Consts<R> &D) {
+  return D.mul_dy ? v * D.inv_dy : quick_div(v, D.dy, D.inv_dy, D.quick_span);
+}
 template <typename R>
-__device__ __forceinline__ R div2y(R v, const Consts<R> &D) { return D.mul_dy ? v * D.inv_2dy : v / (R(2.0) * D.dy); }
+__device__ __forceinline__ R div2y(R v, const Consts<R> &D) {
+  return D.mul_dy ? v * D.inv_2dy : quick_div(v, R(2.0) * D.dy, D.inv_2dy, D.quick_span);
+}
 
 /* The same constants when every spacing is known to be a power of two (or
  * the field type is float): the divisions are multiplications by the exact
@@ -444,6 +473,7 @@ struct StatBufs {
   int mixed;           /* kf_step: odd CTAs take bulk tiles first, then interface tiles */
   const double *trows; /* non-isothermal simulations: per simulation the temperature of each ghosted column y
                           as the phase-field pass reads it, then as the concentration pass reads it */
+  int diag;            /* every phase's off-diagonal D, c_mu and A are zero and no E is -0 */
   unsigned tma_extra;  /* bytes a box's barrier expects beyond the box: 0, or more to test the give-up path */
   double *dphi_out;    /* NULL, or (a batch of one) the step's delta-phi of every interface tile and its ring in
                           the delta-phi layout (Grid dpitch/dplane); cells no interface tile covers are left as
@@ -603,6 +633,54 @@ __device__ __forceinline__ void block_stats(const Consts<R> &D, bool valid, cons
   }
 }
 
+/* dmu = (dc/dmu)^-1 dc in FP64 by the simulation's inversion mode, and mu + dmu
+ * into m64 (calculate_divergence_concentration.h:96-140) */
+template <typename R, int K, typename CT>
+__device__ __forceinline__ void solve_dmu(const CT &D, double (&dcdmu)[K][K], const double (&dc)[K], double (&m64)[K],
+                                          double *dmu) {
+#pragma unroll
+  for (int k = 0; k < K; k++) dmu[k] = 0.0;
+  if (D.inv_mode == GP_INV_BINARY) {
+    double i00 = 1.0 / dcdmu[0][0];
+    dmu[0] = dc[0] * i00;
+    m64[0] += dmu[0];
+  } else if (D.inv_mode == GP_INV_TERNARY && K == 2) {
+    double det = dcdmu[0][0] * dcdmu[K - 1][K - 1] - dcdmu[0][K - 1] * dcdmu[K - 1][0];
+    double iv[K][K];
+    iv[0][0] = dcdmu[K - 1][K - 1] / det;
+    iv[K - 1][K - 1] = dcdmu[0][0] / det;
+    iv[0][K - 1] = -dcdmu[0][K - 1] / det;
+    iv[K - 1][0] = -dcdmu[K - 1][0] / det;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      dmu[k] = 0.0;
+#pragma unroll
+      for (int l = 0; l < K; l++) dmu[k] += iv[k][l] * dc[l];
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) m64[k] = dmu[k] + m64[k];
+  } else if (D.inv_mode == GP_INV_DILUTE) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double ikk = 1.0 / dcdmu[k][k];
+      dmu[k] = dc[k] * ikk;
+      m64[k] += dmu[k];
+    }
+  } else {
+    double iv[K][K];
+    matinv_div<double, K>(dcdmu, iv);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double s = 0;
+#pragma unroll
+      for (int l = 0; l < K; l++) s = s + iv[k][l] * dc[l];
+      dmu[k] = s;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) m64[k] = dmu[k] + m64[k];
+  }
+}
+
 /* mu update and phi commit of one tile cell from the tile's face fluxes
  * (calculate_divergence_concentration.h:24-140): divergences, then the bulk
  * branch (mu = Mu_a(c_a(mu) + dc)) or the interface branch (dmu = (dc/dmu)^-1 dc,
@@ -696,46 +774,8 @@ __device__ __forceinline__ void commit_cell(const CT &D, const R (&FX)[K][K][NXF
     }
     double m64[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) { m64[k] = (double)m[k]; dmu[k] = 0.0; }
-    if (D.inv_mode == GP_INV_BINARY) {
-      double i00 = 1.0 / dcdmu[0][0];
-      dmu[0] = dc[0] * i00;
-      m64[0] += dmu[0];
-    } else if (D.inv_mode == GP_INV_TERNARY && K == 2) {
-      double det = dcdmu[0][0] * dcdmu[K - 1][K - 1] - dcdmu[0][K - 1] * dcdmu[K - 1][0];
-      double iv[K][K];
-      iv[0][0] = dcdmu[K - 1][K - 1] / det;
-      iv[K - 1][K - 1] = dcdmu[0][0] / det;
-      iv[0][K - 1] = -dcdmu[0][K - 1] / det;
-      iv[K - 1][0] = -dcdmu[K - 1][0] / det;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        dmu[k] = 0.0;
-#pragma unroll
-        for (int l = 0; l < K; l++) dmu[k] += iv[k][l] * dc[l];
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) m64[k] = dmu[k] + m64[k];
-    } else if (D.inv_mode == GP_INV_DILUTE) {
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        double ikk = 1.0 / dcdmu[k][k];
-        dmu[k] = dc[k] * ikk;
-        m64[k] += dmu[k];
-      }
-    } else {
-      double iv[K][K];
-      matinv_div<double, K>(dcdmu, iv);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        double s = 0;
-#pragma unroll
-        for (int l = 0; l < K; l++) s = s + iv[k][l] * dc[l];
-        dmu[k] = s;
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) m64[k] = dmu[k] + m64[k];
-    }
+    for (int k = 0; k < K; k++) m64[k] = (double)m[k];
+    solve_dmu<R, K>(D, dcdmu, dc, m64, dmu);
     if constexpr (sizeof(R) == 8) {
 #pragma unroll
       for (int k = 0; k < K; k++) nm[k] = (R)m64[k];
