@@ -52,7 +52,9 @@ struct BatchLaunch {
   void (*solo_fill)(void *dst, const void *consts, const SimDesc *sd);
   cudaError_t (*flags)(int ntiles, cudaStream_t s, const SimDesc *sims, const int *tsim, const void *state,
                        TileFlags *flags);
-  /* one smoothing sweep of a simulation (tcc: its temperature rows, or NULL) */
+  /* FP64: the listed tiles of a sweep (blocks: its blocks per SM when not NULL, no launch) */
+  cudaError_t (*sweep)(const StepLaunch &l, int *blocks);
+  /* FP32: one smoothing sweep of a simulation (tcc: its temperature rows, or NULL) */
   cudaError_t (*smooth)(cudaStream_t s, const void *consts, const void *phi, const void *mu, void *phin,
                         void *mun, Grid g, const double *tcc);
   /* moving frame: interface position into pos[s] (zeroed by the caller),
@@ -175,12 +177,26 @@ struct BatchKernels {
     kf_flags<R, N><<<ntiles, NT, 0, s>>>(sims, tsim, (const R *)state, fl);
     return cudaGetLastError();
   }
+  static cudaError_t sweep(const StepLaunch &l, int *blocks) {
+    if constexpr (sizeof(R) == 8) {
+      if (blocks) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, ks_tiles<R, N, K, A>, NT, 0);
+      ks_tiles<R, N, K, A><<<l.grid, NT, 0, l.stream>>>(l.sims, (const Consts<R> *)l.consts, (const R *)l.state,
+                                                        (R *)l.next, l.flag_out, l.glist, l.st.trows, l.ctr, l.ndone);
+      return cudaGetLastError();
+    } else {
+      return cudaErrorNotSupported;
+    }
+  }
   static cudaError_t smooth(cudaStream_t s, const void *consts, const void *phi, const void *mu, void *phin,
                             void *mun, Grid g, const double *tcc) {
-    dim3 grid((g.my + 127) / 128, g.mx);
-    k_smooth<R, N, K, A><<<grid, 128, 0, s>>>((const Consts<R> *)consts, (const R *)phi, (const R *)mu, (R *)phin,
-                                              (R *)mun, g, tcc);
-    return cudaGetLastError();
+    if constexpr (sizeof(R) == 4) {
+      dim3 grid((g.my + 127) / 128, g.mx);
+      k_smooth<R, N, K, A><<<grid, 128, 0, s>>>((const Consts<R> *)consts, (const R *)phi, (const R *)mu, (R *)phin,
+                                                (R *)mun, g, tcc);
+      return cudaGetLastError();
+    } else {
+      return cudaErrorNotSupported;
+    }
   }
   static cudaError_t shift_pos(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
                                const void *state, int *pos) {
@@ -208,6 +224,7 @@ struct BatchKernels {
     t.solo_fill = solo_fill;
     t.general = general;
     t.flags = flags;
+    t.sweep = sweep;
     t.smooth = smooth;
     t.trows = trows;
     t.shift_pos = shift_pos;

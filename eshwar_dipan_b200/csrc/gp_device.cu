@@ -335,6 +335,7 @@ struct gp_batch {
   std::vector<gp_derived> derived;
   std::vector<gpd::SimDesc> desc;
   int dev, nsm, grid_b, grid_g, grid_s;   /* grid_s: kf_step (0: bulk and interface kernels apart) */
+  int grid_w;                   /* ks_tiles (FP64 smoothing) */
   std::vector<char> solo;       /* a batch of one: its StepArgs (the step kernels' parameter) */
   bool mul;                     /* every simulation's dx and dy are powers of two (or FP32) */
   bool diag;                    /* off-diagonal D, c_mu, A all zero and no E is -0, in every simulation */
@@ -401,10 +402,11 @@ static int bfail(gp_batch *b, int code, const char *fmt, ...) {
     if (e_ != cudaSuccess) return bfail(b, GP_ECUDA, "%s: %s", #call, cudaGetErrorString(e_));  \
   } while (0)
 
-/* One step: bulk tiles (and the interface list), then the interface tiles.
- * ev: optional events around the two kernels. */
-static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
-  gpd::StatBufs st = {};
+/* What the kernels of the next step (or sweep) from the current buffer are launched with. */
+static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
+  gpd::StepLaunch l;
+  gpd::StatBufs &st = l.st;
+  st = {};
   st.ext = b->ext;
   st.partials = b->partials;
   st.want_sums = want_sums;
@@ -418,15 +420,6 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   st.trows = b->tgrad ? b->trows : nullptr;
   st.bch_div = b->shape.bch_div;
   const int in = b->cur, out = b->cur ^ 1;
-  const void *sin = b->redir_in ? b->redir_in : b->state[in];
-  void *sout = b->redir_in ? b->redir_out : b->state[out];
-  const gpd::TensorMapSlot *tmaps = b->redir_in ? b->redir_map : b->tmaps;
-  const int tbuf = b->redir_in ? 0 : in;
-  if (ev) BK(cudaEventRecord(ev[0], b->stream));
-  if (b->tgrad) BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
-  BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
-                   b->redir_in ? b->redir_have : b->flags[out], b->glist, b->blist, b->counters));
-  gpd::StepLaunch l;
   l.stream = b->stream;
   l.mul = b->mul;
   l.diag = b->diag;
@@ -436,13 +429,24 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   l.consts = b->d_consts;
   l.blist = b->blist;
   l.glist = b->glist;
-  l.tmaps = tmaps;
-  l.buf = tbuf;
-  l.state = sin;
-  l.next = sout;
+  l.tmaps = b->redir_in ? b->redir_map : b->tmaps;
+  l.buf = b->redir_in ? 0 : in;
+  l.state = b->redir_in ? b->redir_in : b->state[in];
+  l.next = b->redir_in ? b->redir_out : b->state[out];
   l.flag_out = b->flags[out];
   l.ctr = b->counters;
-  l.st = st;
+  return l;
+}
+
+/* One step: bulk tiles (and the interface list), then the interface tiles.
+ * ev: optional events around the two kernels. */
+static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
+  gpd::StepLaunch l = batch_launch_args(b, want_sums);
+  const int in = b->cur, out = b->cur ^ 1;
+  if (ev) BK(cudaEventRecord(ev[0], b->stream));
+  if (b->tgrad) BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
+  BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
+                   b->redir_in ? b->redir_have : b->flags[out], b->glist, b->blist, b->counters));
   if (!want_sums && b->grid_s > 0 && b->shape.fused && (!ev || ev[3] == nullptr)) {
     /* one launch for both kinds of tile; ev (with ev[3] null): events after
      * the classification and after the step */
@@ -1154,6 +1158,9 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
     l.tg = b->tgrad;
     l.solo = b->solo.empty() ? nullptr : b->solo.data();
     e = b->L.prepare(l, &bpb, &bpg, &bps);
+    int bpw = 1;
+    if (e == cudaSuccess && b->elem == 8) e = b->L.sweep(l, &bpw);
+    b->grid_w = std::min(nt, b->nsm * std::max(1, bpw));
   }
   if (e != cudaSuccess) {
     rc = bfail(b, GP_ECUDA, "gp_batch_create: %s", cudaGetErrorString(e));
@@ -1268,6 +1275,23 @@ int gp_batch_smooth(gp_batch *b, long nsteps) {
   /* the sweeps run before the first step: the temperature as copied at t = 0 */
   if (b->tgrad && nsteps > 0)
     BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
+  if (b->elem == 8) {
+    /* the step's classification and bulk tiles, the listed rest by ks_tiles */
+    for (long t = 0; t < nsteps; t++) {
+      gpd::StepLaunch l = batch_launch_args(b, 0);
+      l.st.ext = nullptr;   /* the sweeps keep no progress record */
+      l.st.sweep = 1;
+      l.ndone = b->grid_b + b->grid_w;
+      BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[b->cur], b->flags[b->cur ^ 1],
+                       b->glist, b->blist, b->counters));
+      l.grid = b->grid_b;
+      BK(b->L.bulk(l));
+      l.grid = b->grid_w;
+      BK(b->L.sweep(l, nullptr));
+      b->cur ^= 1;
+    }
+    return batch_check_error(b);
+  }
   for (long t = 0; t < nsteps; t++) {
     for (int s = 0; s < b->nsims; s++) {
       const gpd::SimDesc &sd = b->desc[s];

@@ -226,8 +226,9 @@ enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR
 
 /* End of one CTA of the step's bulk or interface kernel (they may run
  * concurrently): the last of the step's ndone CTAs empties the lists and
- * advances the step counter.  Call with all threads. */
-__device__ __forceinline__ void step_finish(int *ctr, int ndone) {
+ * advances the step counter by `steps` (0: a smoothing sweep).  Call with all
+ * threads. */
+__device__ __forceinline__ void step_finish(int *ctr, int ndone, int steps) {
   __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -241,7 +242,7 @@ __device__ __forceinline__ void step_finish(int *ctr, int ndone) {
     ctr[CTR_DONE] = 0;
     ctr[CTR_BULK] = 0;
     ctr[CTR_BHEAD] = 0;
-    ctr[CTR_STEP] = (int)((unsigned)ctr[CTR_STEP] + 1u);
+    ctr[CTR_STEP] = (int)((unsigned)ctr[CTR_STEP] + (unsigned)steps);
     __threadfence();
   }
 }
@@ -1012,7 +1013,7 @@ __global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
-  step_finish(ctr, ndone);
+  step_finish(ctr, ndone, st.sweep ? 0 : 1);
 }
 
 /* an interface tile's shared memory */
@@ -1472,7 +1473,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const R *__restrict__ state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
     const int4 *__restrict__ glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
-  step_finish(ctr, ndone);
+  step_finish(ctr, ndone, 1);
 }
 
 /* One step in one persistent launch: each CTA takes interface tiles while
@@ -1498,7 +1499,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
     }
     __syncthreads();   /* the pass's shared memory becomes the next one's */
   }
-  step_finish(ctr, ndone);
+  step_finish(ctr, ndone, 1);
 }
 
 /* Per simulation, the moving-frame state the temperature rows need: the

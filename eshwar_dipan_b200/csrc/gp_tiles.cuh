@@ -473,6 +473,7 @@ struct StatBufs {
   int mixed;           /* kf_step: odd CTAs take bulk tiles first, then interface tiles */
   const double *trows; /* non-isothermal simulations: per simulation the temperature of each ghosted column y
                           as the phase-field pass reads it, then as the concentration pass reads it */
+  int sweep;           /* kf_bulk: a smoothing sweep's bulk tiles (no step is counted) */
   int diag;            /* every phase's off-diagonal D, c_mu and A are zero and no E is -0 */
   unsigned tma_extra;  /* bytes a box's barrier expects beyond the box: 0, or more to test the give-up path */
   double *dphi_out;    /* NULL, or (a batch of one) the step's delta-phi of every interface tile and its ring in
