@@ -1188,15 +1188,16 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
 #pragma unroll
         for (int a = 0; a < N; a++) {
           p[a] = F[a][i][j + CO];
-          tame = tame && fabs(p[a]) < R(1e18);
-          nu = nu || !(F[a][i + 1][j + CO] == p[a] && F[a][i - 1][j + CO] == p[a] && F[a][i][j + 1 + CO] == p[a] &&
-                       F[a][i][j - 1 + CO] == p[a]);
+          /* bitwise, not short-circuit: branches here cost more than the comparisons */
+          tame = tame & (fabs(p[a]) < R(1e18));
+          nu = nu | (F[a][i + 1][j + CO] != p[a]) | (F[a][i - 1][j + CO] != p[a]) | (F[a][i][j + 1 + CO] != p[a]) |
+               (F[a][i][j - 1 + CO] != p[a]);
         }
 #pragma unroll
-        for (int k = 0; k < K; k++) tame = tame && fabs(F[N + k][i][j + CO]) < R(1e18);
+        for (int k = 0; k < K; k++) tame = tame & (fabs(F[N + k][i][j + CO]) < R(1e18));
         /* (a constant stencil between phases is listed too, for its anti-trapping weights) */
 #pragma unroll
-        for (int a = 0; a < N - 1; a++) nu = nu || !(p[a] == R(0.0) || p[a] == R(1.0));
+        for (int a = 0; a < N - 1; a++) nu = nu | ((p[a] != R(0.0)) & (p[a] != R(1.0)));
       }
       if (in) {
         if (!nu) {
@@ -1273,7 +1274,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
           const R xp = F[a][i + 1][j + CO], xm = F[a][i - 1][j + CO], yp = F[a][i][j + 1 + CO],
                   ym = F[a][i][j - 1 + CO];
           /* a phase that is zero on the stencil is not active */
-          if (N > 2 && p[a] == R(0.0) && xp == R(0.0) && xm == R(0.0) && yp == R(0.0) && ym == R(0.0)) continue;
+          if (N > 2 && ((p[a] == R(0.0)) & (xp == R(0.0)) & (xm == R(0.0)) & (yp == R(0.0)) & (ym == R(0.0)))) continue;
           R dv = divx(divx(xp - p[a], D) - divx(p[a] - xm, D), D);
           dv += divy(divy(yp - p[a], D) - divy(p[a] - ym, D), D);
           if (fabs(dv) > R(0.0)) mask |= 1u << a;
@@ -1458,6 +1459,30 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   __syncthreads();
 }
 
+/* The interface tiles in a kernel: inlined in FP64; in FP32 one copy that every
+ * kernel calls, so that its fused multiply-adds are the same in all of them. */
+template <int N, int K, bool ANISO, bool TG>
+__device__ __noinline__ void general_tiles_f32(const SimDesc *__restrict__ sims, const Consts<float> *__restrict__ consts,
+                                               const TensorMapSlot *__restrict__ tmaps, int buf,
+                                               const float *__restrict__ state, float *__restrict__ next,
+                                               TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                               int *__restrict__ ctr, const StatBufs st) {
+  general_tiles<float, N, K, ANISO, true, TG, false>(StepArgs<float, false>{}, sims, consts, tmaps, buf, state, next,
+                                                     flag_out, glist, ctr, st);
+}
+template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
+__device__ __forceinline__ void step_general(const StepArgs<R, SOLO> &args, const SimDesc *__restrict__ sims,
+                                             const Consts<R> *__restrict__ consts,
+                                             const TensorMapSlot *__restrict__ tmaps, int buf,
+                                             const R *__restrict__ state, R *__restrict__ next,
+                                             TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                             int *__restrict__ ctr, const StatBufs &st) {
+  if constexpr (sizeof(R) == 8)
+    general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+  else
+    general_tiles_f32<N, K, ANISO, TG>(sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+}
+
 /* CTAs of the interface code an SM holds: what its shared memory leaves, at most two (128 registers a thread) */
 template <typename R, int N, int K, bool ANISO>
 constexpr int item_ctas() {
@@ -1472,7 +1497,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const Consts<R> *__restrict__ consts, const TensorMapSlot *__restrict__ tmaps, int buf,
     const R *__restrict__ state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
     const int4 *__restrict__ glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
-  general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+  step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
   step_finish(ctr, ndone, 1);
 }
 
@@ -1494,7 +1519,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
       bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
       bulk_release_warp<R, K>();
     } else {
-      general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr,
+      step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr,
                                                    st);
     }
     __syncthreads();   /* the pass's shared memory becomes the next one's */

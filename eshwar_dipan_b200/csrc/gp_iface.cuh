@@ -190,9 +190,11 @@ __device__ __forceinline__ void item_face(const CT &D, ItemFrame<R, N, K> F, Ite
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const R *S = &F[q ? b : a][0][0] + o;
-          have = have && (S[0] != R(0.0) || S[along] != R(0.0) ||
-                          (!D.rot_identity && (S[cross] != R(0.0) || S[-cross] != R(0.0) ||
-                                               S[along + cross] != R(0.0) || S[along - cross] != R(0.0))));
+          bool any = (S[0] != R(0.0)) | (S[along] != R(0.0));
+          if (!D.rot_identity)
+            any = any | (S[cross] != R(0.0)) | (S[-cross] != R(0.0)) | (S[along + cross] != R(0.0)) |
+                  (S[along - cross] != R(0.0));
+          have = have & any;
         }
       }
       if (have) {
@@ -257,7 +259,7 @@ __device__ __forceinline__ void item_lambda(const CT &D, ItemFrame<R, N, K> F, I
     const R *B = &F[b][0][0] + o;
     const R pb = B[0], bxp = B[BW], bxm = B[-BW], byp = B[1], bym = B[-1];
     /* a phase that is zero on the 5-point stencil has no term here */
-    if (N > 2 && pb == R(0.0) && bxp == R(0.0) && bxm == R(0.0) && byp == R(0.0) && bym == R(0.0)) continue;
+    if (N > 2 && ((pb == R(0.0)) & (bxp == R(0.0)) & (bxm == R(0.0)) & (byp == R(0.0)) & (bym == R(0.0)))) continue;
     const R gxb = R(0.5) * (divx(bxp - pb, D) + divx(pb - bxm, D)), gyb = div2y(byp - bym, D);
     const R gam = D.gamma[a][b];
     /* face means of the other phase: forward and backward x, right and left y */
@@ -684,8 +686,16 @@ __device__ __forceinline__ void item_sums(const CT &D, bool valid, const R *nph,
  * Exact and order-free; NaN is ignored. */
 template <typename R, int N, int K>
 __device__ __forceinline__ void item_extremes(const double *ext, const R *nph, const R *nm, const StatBufs &st, int s) {
-  long long *slot = st.ext + (long long)s * (2 * (N + K));
   /* slot layout: max phi[N], min phi[N], max mu[K], min mu[K] */
+  bool beats = false;
+#pragma unroll
+  for (int f = 0; f < N + K; f++) {
+    const double v = f < N ? (double)nph[f < N ? f : 0] : (double)nm[f < N ? 0 : f - N];
+    const int hi = f < N ? f : 2 * N + (f - N), lo = f < N ? N + f : 2 * N + K + (f - N);
+    beats = beats | (v > ext[hi]) | (v < ext[lo]);
+  }
+  if (!beats) return;
+  long long *slot = st.ext + (long long)s * (2 * (N + K));
 #pragma unroll
   for (int f = 0; f < N + K; f++) {
     const double v = f < N ? (double)nph[f < N ? f : 0] : (double)nm[f < N ? 0 : f - N];
