@@ -473,21 +473,48 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
   }
   __syncwarp();
 
-  R emax[K], emin[K];   /* running mu extremes of the cells this warp stepped */
+  /* Running mu extremes of the cells a lane stepped.  FP64: they start at the
+   * simulation's extremes as they were when the warp moved to it (kept finite, so
+   * that an infinity exceeds them), and a row takes the slow way only where a value
+   * does: two comparisons a value where fmax and fmin took about eight instructions
+   * each, a quarter of the kernel's.  FP32 (three-operand max and min): from
+   * infinities. */
+  constexpr bool F64 = sizeof(R) == 8;
+  R emax[K], emin[K];
 #pragma unroll
   for (int k = 0; k < K; k++) { emax[k] = -INFINITY; emin[k] = INFINITY; }
+  bool beaten = !F64;
   int cur_sim = -1;
+  auto ext_slot = [&](int s) { return st.ext + (long long)s * (2 * (N + K)) + 2 * N; };   /* max mu[K], min mu[K] */
+  auto from_ord = [](long long o) { return __longlong_as_double(o < 0 ? o ^ 0x7fffffffffffffffLL : o); };
   auto flush = [&](int s) {
+    if (__any_sync(0xffffffffu, beaten)) {
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const double a = warp_max(emax[k]), c = warp_min(emin[k]);
-      if (lane == 0 && st.ext) {
-        long long *slot = st.ext + (long long)s * (2 * (N + K));
-        if (a > -INFINITY) atomicMax(slot + 2 * N + k, ord(a));
-        if (c < INFINITY) atomicMin(slot + 2 * N + K + k, ord(c));
+      for (int k = 0; k < K; k++) {
+        const double a = warp_max(emax[k]), c = warp_min(emin[k]);
+        if (lane == 0 && st.ext) {
+          long long *slot = ext_slot(s);
+          /* an extreme that is already there takes no atomic */
+          if (a > from_ord(*(volatile long long *)(slot + k))) atomicMax(slot + k, ord(a));
+          if (c < from_ord(*(volatile long long *)(slot + K + k))) atomicMin(slot + K + k, ord(c));
+        }
       }
-      emax[k] = -INFINITY;
-      emin[k] = INFINITY;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) { emax[k] = -INFINITY; emin[k] = INFINITY; }
+    beaten = !F64;
+  };
+  auto load_ext = [&](int s) {
+    if constexpr (F64) {
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        emax[k] = 1.7976931348623157e308;    /* without a record nothing finite exceeds them */
+        emin[k] = -1.7976931348623157e308;
+        if (st.ext) {
+          emax[k] = fmin(emax[k], from_ord(*(volatile long long *)(ext_slot(s) + k)));
+          emin[k] = fmax(emin[k], from_ord(*(volatile long long *)(ext_slot(s) + K + k)));
+        }
+      }
     }
   };
 
@@ -624,6 +651,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
       cur_sim = s;
       g = sims[s].g;
       off_state = sims[s].off_state;
+      load_ext(s);
     }
     if (cur_key != s * 16 + p) {
       cur_key = s * 16 + p;
@@ -753,6 +781,9 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
          * path) in their order, two cells at a time */
         double2 P[K], FXP[K][K];
         unsigned redo = 0;   /* DIAG: bit 2 rr + e, cell e of row rr to redo with every term */
+        R *mq[K];            /* the row's new mu */
+#pragma unroll
+        for (int k = 0; k < K; k++) mq[k] = mun + k * g.plane + (long long)(x0 + r0) * g.pitch + y;
 #pragma unroll
         for (int l = 0; l < K; l++) {
           const double2 pp = *reinterpret_cast<const double2 *>(&sg.M[l][r0][c]);
@@ -831,31 +862,50 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
             commit_mu(mc, m0, df0, n0, d0);
             commit_mu(mc, m1, df1, n1, d1);
           }
-          /* a left-out term is +-0 only when the values it multiplies are
-           * finite, and they are when every new mu is; otherwise (DIAG) the
-           * cell is redone with every term after the rows (its extremes and
-           * sums are taken then) */
-          bool f0 = true, f1 = v1;
-          if constexpr (DIAG) {
-#pragma unroll
-            for (int k = 0; k < K; k++) { f0 &= fabs(n0[k]) < R(INFINITY); f1 &= fabs(n1[k]) < R(INFINITY); }
-            redo |= (f0 ? 0u : 1u) << (2 * rr);
-            redo |= (v1 && !f1 ? 2u : 0u) << (2 * rr);
-          }
-          const long long o = (long long)x * g.pitch + y;
-          /* the statistics take the cells of their rows */
-          const bool srow = stat_row(g, x);
-          f0 = f0 && srow;
-          f1 = f1 && srow;
+          /* new extremes, or a value that is not finite */
+          bool out = false;
 #pragma unroll
           for (int k = 0; k < K; k++) {
-            if (v1) *reinterpret_cast<double2 *>(mun + k * g.plane + o) = make_double2(n0[k], n1[k]);
-            else mun[k * g.plane + o] = n0[k];
-            /* NaN is ignored by fmax/fmin; a cell to be redone is left out */
-            const R x0 = f0 ? n0[k] : R(NAN), x1 = f1 ? n1[k] : R(NAN);
-            emax[k] = fmax(emax[k], fmax(x0, x1));
-            emin[k] = fmin(emin[k], fmin(x0, x1));
+            out = out | !(n0[k] <= emax[k]) | !(n0[k] >= emin[k]);
+            out = out | (v1 & (!(n1[k] <= emax[k]) | !(n1[k] >= emin[k])));
           }
+          const bool srow = stat_row(g, x);   /* the statistics take the cells of their rows */
+          if (out) {
+            /* a left-out term is +-0 only when the values it multiplies are
+             * finite, and they are when every new mu is; otherwise (DIAG) the
+             * cell is redone with every term after the rows (its extremes are
+             * taken then) */
+            bool f0 = true, f1 = v1;
+            if constexpr (DIAG) {
+#pragma unroll
+              for (int k = 0; k < K; k++) { f0 &= fabs(n0[k]) < R(INFINITY); f1 &= fabs(n1[k]) < R(INFINITY); }
+              redo |= (f0 ? 0u : 1u) << (2 * rr);
+              redo |= (v1 && !f1 ? 2u : 0u) << (2 * rr);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+              if (srow && (e ? f1 : f0)) {
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                  const R v = e ? n1[k] : n0[k];
+                  if (fabs(v) < R(INFINITY)) {
+                    emax[k] = fmax(emax[k], v);
+                    emin[k] = fmin(emin[k], v);
+                    beaten = true;
+                  } else if (v == v && st.ext) {   /* (NaN is ignored) */
+                    if (v > R(0.0)) atomicMax(ext_slot(s) + k, ord(v));
+                    else atomicMin(ext_slot(s) + K + k, ord(v));
+                  }
+                }
+              }
+          }
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            if (v1) *reinterpret_cast<double2 *>(mq[k]) = make_double2(n0[k], n1[k]);
+            else *mq[k] = n0[k];
+            mq[k] += g.pitch;
+          }
+          const long long o = (long long)x * g.pitch + y;
           if (have != p) {
 #pragma unroll
             for (int a = 0; a < N; a++) {
@@ -864,8 +914,10 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
               else phin[a * g.plane + o] = v;
             }
           }
-          if (f0) sum_cell(n0, d0);
-          if (f1) sum_cell(n1, d1);
+          if (SUMS && srow) {
+            sum_cell(n0, d0);
+            if (v1) sum_cell(n1, d1);
+          }
 #pragma unroll
           for (int l = 0; l < K; l++) P[l] = Pn[l];
         }
@@ -884,9 +936,9 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
 #pragma unroll
             for (int k = 0; k < K; k++) {
               mun[k * g.plane + o] = nm[k];
-              if (srow) {
-                emax[k] = fmax(emax[k], nm[k]);
-                emin[k] = fmin(emin[k], nm[k]);
+              if (srow && st.ext && nm[k] == nm[k]) {
+                atomicMax(ext_slot(s) + k, ord((double)nm[k]));
+                atomicMin(ext_slot(s) + K + k, ord((double)nm[k]));
               }
             }
             if (srow) sum_cell(nm, dmu);
