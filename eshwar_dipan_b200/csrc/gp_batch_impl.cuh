@@ -40,7 +40,7 @@ struct BatchLaunch {
   cudaError_t (*prepare)(const StepLaunch &l, int *bulk, int *general, int *step);
   /* the bulk and interface lists of a step; flag_out: the flags of the buffer it
    * writes (copied into the bulk entries) */
-  cudaError_t (*classify)(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
+  cudaError_t (*classify)(int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts, const int *tsim,
                           const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist, int4 *blist, int *ctr);
   cudaError_t (*bulk)(const StepLaunch &l);
   cudaError_t (*general)(const StepLaunch &l);
@@ -68,6 +68,23 @@ struct BatchLaunch {
                        SimDyn *dyn, double *rows);
   size_t elem;
 };
+
+/* A launch that may start while the kernel before it on the stream still runs: the
+ * kernel waits by itself (pdl_begin) before it touches what that one writes. */
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, const A &...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
 
 template <typename R, int N, int K, bool A>
 struct BatchKernels {
@@ -133,25 +150,28 @@ struct BatchKernels {
     else with_bulk_m<true>(l, sums, f);
   }
   static cudaError_t step(const StepLaunch &l) {
+    cudaError_t e = cudaSuccess;
     with_step(l, [&](auto k, const auto &args) {
-      k<<<l.grid, NTI, step_smem, l.stream>>>(args, l.sims, (const Consts<R> *)l.consts, l.blist, l.glist, l.tmaps, l.buf,
-                                              (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
+      e = launch_dependent(k, l.grid, NTI, step_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.blist,
+                           l.glist, l.tmaps, l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
-    return cudaGetLastError();
+    return e;
   }
   static cudaError_t bulk(const StepLaunch &l) {
+    cudaError_t e = cudaSuccess;
     with_bulk(l, l.st.want_sums != 0, [&](auto k) {
-      k<<<l.grid, NTI, bulk_smem, l.stream>>>(l.sims, (const Consts<R> *)l.consts, l.blist, l.tmaps, l.buf,
-                                              (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
+      e = launch_dependent(k, l.grid, NTI, bulk_smem, l.stream, l.sims, (const Consts<R> *)l.consts, l.blist, l.tmaps,
+                           l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
-    return cudaGetLastError();
+    return e;
   }
   static cudaError_t general(const StepLaunch &l) {
+    cudaError_t e = cudaSuccess;
     with_general(l, [&](auto k, const auto &args) {
-      k<<<l.grid, NTI, item_smem, l.stream>>>(args, l.sims, (const Consts<R> *)l.consts, l.tmaps, l.buf,
-                                              (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.ctr, l.ndone, l.st);
+      e = launch_dependent(k, l.grid, NTI, item_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.tmaps,
+                           l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.ctr, l.ndone, l.st);
     });
-    return cudaGetLastError();
+    return e;
   }
   static cudaError_t prepare(const StepLaunch &l, int *bb, int *bg, int *bs) {
     cudaError_t e = cudaSuccess;
@@ -165,12 +185,11 @@ struct BatchKernels {
     with_step(l, [&](auto k, const auto &) { set(k, step_smem, bs); });
     return e;
   }
-  static cudaError_t classify(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts,
+  static cudaError_t classify(int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts,
                               const int *tsim, const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist,
                               int4 *blist, int *ctr) {
-    kf_classify<R><<<(ntiles + NTC - 1) / NTC, NTC, 0, s>>>(sims, (const Consts<R> *)consts, tsim, ntiles, flag_in, flag_out, glist,
-                                                         blist, ctr);
-    return cudaGetLastError();
+    return launch_dependent(kf_classify<R>, (ntiles + NTC - 1) / NTC, NTC, 0, s, solo, sims, (const Consts<R> *)consts,
+                            tsim, ntiles, flag_in, flag_out, glist, blist, ctr);
   }
   static cudaError_t flags(int ntiles, cudaStream_t s, const SimDesc *sims, const int *tsim, const void *state,
                            TileFlags *fl) {
@@ -180,9 +199,8 @@ struct BatchKernels {
   static cudaError_t sweep(const StepLaunch &l, int *blocks) {
     if constexpr (sizeof(R) == 8) {
       if (blocks) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, ks_tiles<R, N, K, A>, NT, 0);
-      ks_tiles<R, N, K, A><<<l.grid, NT, 0, l.stream>>>(l.sims, (const Consts<R> *)l.consts, (const R *)l.state,
-                                                        (R *)l.next, l.flag_out, l.glist, l.st.trows, l.ctr, l.ndone);
-      return cudaGetLastError();
+      return launch_dependent(ks_tiles<R, N, K, A>, l.grid, NT, 0, l.stream, l.sims, (const Consts<R> *)l.consts,
+                              (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.st.trows, l.ctr, l.ndone);
     } else {
       return cudaErrorNotSupported;
     }

@@ -336,6 +336,7 @@ struct gp_batch {
   std::vector<gpd::SimDesc> desc;
   int dev, nsm, grid_b, grid_g, grid_s;   /* grid_s: kf_step (0: bulk and interface kernels apart) */
   int grid_w;                   /* ks_tiles (FP64 smoothing) */
+  gpd::ClassifySim csim;        /* a batch of one: its layout for the classification (else tiles_x 0) */
   std::vector<char> solo;       /* a batch of one: its StepArgs (the step kernels' parameter) */
   bool mul;                     /* every simulation's dx and dy are powers of two (or FP32) */
   bool diag;                    /* off-diagonal D, c_mu, A all zero and no E is -0, in every simulation */
@@ -445,7 +446,7 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   const int in = b->cur, out = b->cur ^ 1;
   if (ev) BK(cudaEventRecord(ev[0], b->stream));
   if (b->tgrad) BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
-  BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
+  BK(b->L.classify(b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
                    b->redir_in ? b->redir_have : b->flags[out], b->glist, b->blist, b->counters));
   if (!want_sums && b->grid_s > 0 && b->shape.fused && (!ev || ev[3] == nullptr)) {
     /* one launch for both kinds of tile; ev (with ev[3] null): events after
@@ -1104,6 +1105,12 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
     }
   }
   b->ntiles = nt;
+  memset(&b->csim, 0, sizeof b->csim);
+  if (nsims == 1) {
+    const gpd::SimDesc &sd = b->desc[0];
+    const gp_derived &d = b->derived[0];
+    b->csim = {sd.g.mx, sd.g.my, sd.tiles_x, {d.bc_x[0][0], d.bc_x[0][1]}, {d.bc_y[0][0], d.bc_y[0][1]}, d.tgrad};
+  }
   if (nsims == 1 && b->L.solo_bytes) {
     b->solo.resize(b->L.solo_bytes);
     b->L.solo_fill(b->solo.data(), consts.data(), &b->desc[0]);
@@ -1282,7 +1289,7 @@ int gp_batch_smooth(gp_batch *b, long nsteps) {
       l.st.ext = nullptr;   /* the sweeps keep no progress record */
       l.st.sweep = 1;
       l.ndone = b->grid_b + b->grid_w;
-      BK(b->L.classify(b->ntiles, b->stream, b->d_desc, b->d_consts, b->d_tsim, b->flags[b->cur], b->flags[b->cur ^ 1],
+      BK(b->L.classify(b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[b->cur], b->flags[b->cur ^ 1],
                        b->glist, b->blist, b->counters));
       l.grid = b->grid_b;
       BK(b->L.bulk(l));

@@ -163,6 +163,12 @@ __device__ __forceinline__ TileFlags uniform_flags(int p) {
   return t;
 }
 
+/* what the classification needs of a simulation (phi's boundary types); tiles_x 0: a
+ * batch of several, read from their descriptors */
+struct ClassifySim {
+  int mx, my, tiles_x, bc_x[2], bc_y[2], tgrad;
+};
+
 /* Bulk test of tile (tile rows by, columns bx) of a simulation, by one
  * thread: every cell of the tile and of its two-cell phi halo holds the exact
  * one-hot phi of one phase.  Returns the phase or -1.  When the halo stays
@@ -170,9 +176,9 @@ __device__ __forceinline__ TileFlags uniform_flags(int p) {
  * neighbour tiles (a corner by either band that contains it); otherwise by the
  * whole-tile flags of the tiles that hold the halo cells after the boundary
  * remap. */
-template <typename R>
-__device__ __forceinline__ int bulk_phase(const Consts<R> &D, const Grid &g, const TileFlags *__restrict__ flags,
-                                          int tile0, int tiles_x, int by, int bx) {
+__device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags *__restrict__ flags, int tile0, int by,
+                                          int bx) {
+  const int tiles_x = g.tiles_x;
   const int x0 = by * TX, y0 = bx * TY;
   const int xl = min(x0 + TX, g.mx) - 1, yl = min(y0 + TY, g.my) - 1;
   if (x0 >= 2 && xl + 2 < g.mx && y0 >= 2 && yl + 2 < g.my) {
@@ -196,8 +202,8 @@ __device__ __forceinline__ int bulk_phase(const Consts<R> &D, const Grid &g, con
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       int x = xs[q], y = ys[q];
-      if (x < 0 || x >= g.mx) x = remap(x, g.mx, D.bc_x[0][0], D.bc_x[0][1]);
-      if (y < 0 || y >= g.my) y = remap(y, g.my, D.bc_y[0][0], D.bc_y[0][1]);
+      if (x < 0 || x >= g.mx) x = remap(x, g.mx, g.bc_x[0], g.bc_x[1]);
+      if (y < 0 || y >= g.my) y = remap(y, g.my, g.bc_y[0], g.bc_y[1]);
       rows[q + 1] = x / TX;
       cols[q + 1] = y / TY;
     }
@@ -215,7 +221,7 @@ __device__ __forceinline__ int bulk_phase(const Consts<R> &D, const Grid &g, con
 /* ------------------------------------------------------------------ */
 
 /* Work-list counters of a batch: [0] interface tiles listed by kf_classify,
- * [1] next interface entry to take, [2] CTAs of kf_bulk and kf_general
+ * [1] interface entries taken beyond the CTAs' first, [2] CTAs of kf_bulk and kf_general
  * finished, [3] step number (keys the FP32 rounding stream), [4] bulk tiles
  * listed, [5] error flag (a TMA box of kf_bulk did not arrive; the host reads
  * and clears it).  The last CTA of the two kernels resets [0..2] and [4] and
@@ -223,6 +229,15 @@ __device__ __forceinline__ int bulk_phase(const Consts<R> &D, const Grid &g, con
  * kf_bulk and kf_general (in either order or side by side). */
 enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR_ERR = 5, CTR_BHEAD = 6,
        CTR_COUNT = 8 };
+
+/* Programmatic dependent launch: the kernels of a step are launched while their
+ * predecessor still runs (every one of its CTAs has started) and wait here, before
+ * they read anything it writes, until it has completed.  A launch gap of a graph
+ * is about 1 us; a step has two. */
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 /* End of one CTA of the step's bulk or interface kernel (they may run
  * concurrently): the last of the step's ndone CTAs empties the lists and
@@ -256,7 +271,7 @@ __device__ __forceinline__ void step_finish(int *ctr, int ndone, int steps) {
  * (NTC threads) spread the flag reads over every SM. */
 constexpr int NTC = 64;
 template <typename R>
-__global__ void __launch_bounds__(NTC) kf_classify(const SimDesc *__restrict__ sims,
+__global__ void __launch_bounds__(NTC) kf_classify(const ClassifySim solo, const SimDesc *__restrict__ sims,
                                                   const Consts<R> *__restrict__ consts, const int *__restrict__ tsim,
                                                   int ntiles, const TileFlags *__restrict__ flag_in,
                                                   const TileFlags *__restrict__ flag_outbuf,
@@ -264,16 +279,28 @@ __global__ void __launch_bounds__(NTC) kf_classify(const SimDesc *__restrict__ s
                                                   int *__restrict__ ctr) {
   const int t = blockIdx.x * NTC + threadIdx.x, lane = threadIdx.x & 31;
   int p = -1, s = 0, by = 0, bx = 0, inside = 0;
+  if (solo.tiles_x) {
+    /* a batch of one: its layout comes with the launch */
+    by = t / solo.tiles_x;
+    bx = t - by * solo.tiles_x;
+  }
+  pdl_begin();
   if (t < ntiles) {
-    s = __ldg(tsim + t);
-    const SimDesc &sd = sims[s];
-    const int lt = t - sd.tile0;
-    by = lt / sd.tiles_x;
-    bx = lt - by * sd.tiles_x;
-    inside = by > 0 && by * TX + TX + 2 <= sd.g.mx && bx > 0 && bx * TY + TY + 2 <= sd.g.my;
+    ClassifySim cs = solo;
+    int tile0 = 0;
+    if (!solo.tiles_x) {
+      s = __ldg(tsim + t);
+      const SimDesc &sd = sims[s];
+      const Consts<R> &D = consts[s];
+      cs = {sd.g.mx, sd.g.my, sd.tiles_x, {D.bc_x[0][0], D.bc_x[0][1]}, {D.bc_y[0][0], D.bc_y[0][1]}, D.tgrad};
+      tile0 = sd.tile0;
+      by = (t - tile0) / cs.tiles_x;
+      bx = t - tile0 - by * cs.tiles_x;
+    }
+    inside = by > 0 && by * TX + TX + 2 <= cs.mx && bx > 0 && bx * TY + TY + 2 <= cs.my;
     /* a non-isothermal simulation steps every tile as an interface tile
      * (whose pure-phase cells take the bulk update at their temperature) */
-    if (!consts[s].tgrad) p = bulk_phase<R>(consts[s], sd.g, flag_in, sd.tile0, sd.tiles_x, by, bx);
+    if (!cs.tgrad) p = bulk_phase(cs, flag_in, tile0, by, bx);
   }
   const unsigned mb = __ballot_sync(0xffffffffu, t < ntiles && p >= 0);
   const unsigned mg = __ballot_sync(0xffffffffu, t < ntiles && p < 0);
@@ -1064,6 +1091,7 @@ __global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk
     const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist,
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  pdl_begin();
   bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
   step_finish(ctr, ndone, st.sweep ? 0 : 1);
 }
@@ -1109,6 +1137,9 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   constexpr unsigned BOX_BYTES = (unsigned)((N + K) * FR * IG::BW * sizeof(R));
   const int nlist = *(volatile int *)(ctr + CTR_LIST);
   if (nlist == 0) return;
+  const bool late = st.mixed && (blockIdx.x & 1);   /* after its bulk tiles */
+  const int first = late ? -1 : (st.mixed ? blockIdx.x >> 1 : blockIdx.x);
+  const int nfirst = st.mixed ? (gridDim.x + 1) >> 1 : gridDim.x;
   using SM = TileSmem<R, N, K, ANISO>;
   SM &sm = *reinterpret_cast<SM *>(step_smem_base);
   __shared__ __align__(16) unsigned char sc_raw[SOLO ? 16 : sizeof(Consts<R>)];
@@ -1132,7 +1163,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     fence_proxy_async_smem();
     if constexpr (sizeof(R) == 8) sm.n_test = sm.n_act = sm.n_task = sm.n_extra = sm.n_j = 0;
     else sm.t.nlist = sm.t.nflist = 0;
-    const int i = atomicAdd(ctr + CTR_HEAD, 1);
+    /* the CTAs that begin with interface tiles own the first entries */
+    const int i = first >= 0 ? first : nfirst + atomicAdd(ctr + CTR_HEAD, 1);
     issue(i < nlist ? __ldg(glist + i) : make_int4(-1, 0, 0, 0), 0);
   }
   int cur_sim = -1;
@@ -1147,7 +1179,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     if (en.x < 0) break;
     const int t = en.x, s = SOLO ? 0 : en.y, x0 = (en.z >> 16) * TX, y0 = (en.z & 0xffff) * TY;
     int nxt = 0;
-    if (tid == 0) nxt = atomicAdd(ctr + CTR_HEAD, 1);   /* used after the next barrier */
+    if (tid == 0) nxt = nfirst + atomicAdd(ctr + CTR_HEAD, 1);   /* used after the next barrier */
     if (s != cur_sim) {
       cur_sim = s;
       if constexpr (!SOLO) {
@@ -1549,6 +1581,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const Consts<R> *__restrict__ consts, const TensorMapSlot *__restrict__ tmaps, int buf,
     const R *__restrict__ state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
     const int4 *__restrict__ glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  pdl_begin();
   step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
   step_finish(ctr, ndone, 1);
 }
@@ -1564,6 +1597,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
     const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist, const int4 *__restrict__ glist,
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+  pdl_begin();
   const int bulk_pass = st.mixed && (blockIdx.x & 1) ? 0 : 1;
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {

@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(NT, N <= 3 ? 2 : 1) ks_tiles(
     const double *__restrict__ trows, int *__restrict__ ctr, int ndone) {
   __shared__ int s_item;
   __shared__ unsigned s_w[TX];
+  pdl_begin();
   const int nlist = *(volatile int *)(ctr + CTR_LIST), wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(ctr + CTR_HEAD, 1);
