@@ -273,7 +273,7 @@ __device__ __forceinline__ T adadq(T qi, const AQPow<T> &p, T dab16) {
 /* ---- phase-field pass ------------------------------------------------- */
 
 /* Anisotropy terms of one face of the 3x3 window S (rows i, columns j): the
- * arithmetic of face_terms (gp_tiles.cuh).  xface: between (i,j) and (i+1,j);
+ * arithmetic of item_face (gp_iface.cuh).  xface: between (i,j) and (i+1,j);
  * else between (i,j) and (i,j+1).  T4[p][0..3] as in the tile face cache. */
 template <typename T, int N>
 __device__ __forceinline__ void aface(const AK<T> &D, const T (&S)[N][3][3], bool xface, int i, int j,
@@ -472,7 +472,7 @@ __device__ __forceinline__ void dphi_cell(const AK<T> &D, const T (&S)[N][3][3],
 
 /* ---- concentration pass ----------------------------------------------- */
 
-/* Quantities of one cell (update_tile's per-cell loop). */
+/* Quantities of one cell of the mu update. */
 template <typename T, int N, int K>
 struct ACell {
   T H[N], CM[N][K], SP[N], DD[K][K];
@@ -495,7 +495,7 @@ __device__ __forceinline__ void acell(const AK<T> &D, const T *p, const T *mm, A
 }
 
 /* Anti-trapping current and diffusion flux products through one face of the
- * window (faces loop of update_tile).  xface: between (i,j) and (i+1,j);
+ * window (the currents of item_current, gp_iface.cuh).  xface: between (i,j) and (i+1,j);
  * else between (i,j) and (i,j+1).  q0/q1: the two cells' quantities; ylo: the
  * interior y of the face's lower cell (y-faces only). */
 template <typename T, int N, int K>

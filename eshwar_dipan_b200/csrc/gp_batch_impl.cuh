@@ -46,6 +46,9 @@ struct BatchLaunch {
   cudaError_t (*general)(const StepLaunch &l);
   /* bulk and interface tiles in one launch (kf_step; not for a sums step) */
   cudaError_t (*step)(const StepLaunch &l);
+  /* FP64: one step of one simulation on the caller's planes (state, next: phi;
+   * solo, mul, st and stream of l) */
+  cudaError_t (*direct)(const StepLaunch &l, const DirectArgs<double, true> &d, int nsm);
   /* the StepArgs of a batch of one (FP32: none, every batch takes the same kernels,
    * since another kernel's fused multiply-adds could round differently) */
   size_t solo_bytes;
@@ -173,6 +176,21 @@ struct BatchKernels {
     });
     return e;
   }
+  template <bool MUL>
+  static cudaError_t direct_m(const StepLaunch &l, const DirectArgs<double, true> &d, int nsm) {
+    auto k = kn_step<double, N, K, A, MUL>;
+    /* on every call: the attribute belongs to the caller's context */
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)item_smem);
+    if (e != cudaSuccess) return e;
+    const int most = nsm * item_ctas<double, N, K, A>();
+    k<<<d.ntiles < most ? d.ntiles : most, NTI, item_smem, l.stream>>>(
+        *reinterpret_cast<const StepArgs<double, true> *>(l.solo), d, (const double *)l.state, (double *)l.next, l.st);
+    return cudaGetLastError();
+  }
+  static cudaError_t direct(const StepLaunch &l, const DirectArgs<double, true> &d, int nsm) {
+    if constexpr (sizeof(R) == 8) return l.mul ? direct_m<true>(l, d, nsm) : direct_m<false>(l, d, nsm);
+    else return cudaErrorNotSupported;
+  }
   static cudaError_t prepare(const StepLaunch &l, int *bb, int *bg, int *bs) {
     cudaError_t e = cudaSuccess;
     auto set = [&](auto k, size_t smem, int *blocks) {
@@ -238,6 +256,7 @@ struct BatchKernels {
     t.classify = classify;
     t.bulk = bulk;
     t.step = step;
+    t.direct = direct;
     t.solo_bytes = SOLO ? sizeof(StepArgs<R, true>) : 0;
     t.solo_fill = solo_fill;
     t.general = general;

@@ -1,8 +1,8 @@
 /*
  * gp_device.cu -- libgp: the C ABI (include/gp.h) over the sm_100a kernels.
  * Host orchestration only; the kernels are in gp_fused.cuh (the stepping
- * engine), gp_tiles.cuh (shared tile code and the two-pass kernels of
- * gp_step_noalloc) and gp_smooth.cuh (the smoothing sweeps).
+ * engine), gp_iface.cuh (its interface tiles), gp_tiles.cuh (what they share) and
+ * gp_smooth.cuh (the smoothing sweeps).
  *
  *  - gp_batch: simulations of different sizes and parameters stepped together
  *    by two kernels per step (bulk tiles, then interface tiles from a device
@@ -10,13 +10,14 @@
  *    storage form (both in gp_kernels.cu); steps are replayed as CUDA graphs of
  *    GP_GRAPH_STEPS steps.
  *  - gp_ctx: one simulation, a batch of one.
- *  - gp_step_noalloc: one FP64 step on caller-owned buffers, two-pass kernels
- *    with constants in __constant__ memory and a fixed scratch array.
+ *  - gp_step_noalloc: one FP64 step on caller-owned buffers, one launch of the
+ *    interface tiles' code over every tile.
  */
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <climits>
 #include <cstdarg>
@@ -35,8 +36,6 @@
 
 #include "gp_adjoint_launch.h"
 #include "gp_batch_impl.cuh"
-
-static __constant__ gpd::Consts<double> cD;
 
 extern "C" const char *gp_host_thread_error(void);
 
@@ -124,6 +123,18 @@ gpd::Consts<R> make_consts(const gp_derived &d) {
   return c;
 }
 
+/* every phase's off-diagonal D, c_mu and A are zero and no E is -0: the step may
+ * leave the off-diagonal terms out */
+bool diagonal(const gp_derived &d) {
+  for (int a = 0; a < d.N; a++)
+    for (int k = 0; k < d.K; k++) {
+      if (d.E[a][k] == 0.0 && std::signbit(d.E[a][k])) return false;
+      for (int l = 0; l < d.K; l++)
+        if (k != l && (d.Dbulk[a][k][l] != 0.0 || d.cmu[a][k][l] != 0.0 || d.A[a][k][l] != 0.0)) return false;
+    }
+  return true;
+}
+
 gpd::Grid make_grid(const gp_derived &d, int pitch_multiple) {
   gpd::Grid g;
   g.mx = (int)d.mx;
@@ -189,64 +200,6 @@ void stats_from(gp_stats *r, const long long *mm, const double *sums, int N, int
   }
   r->nonfinite = (long long)llround(sums[2 * N + 2 * K]);
   r->steps_done = steps;
-}
-
-}  // namespace
-
-/* ======================================================================= */
-/* two-pass FP64 kernels of gp_step_noalloc: one CTA per tile, constants   */
-/* in __constant__ memory                                                  */
-/* ======================================================================= */
-
-namespace gpd {
-
-template <int N, int K, bool A>
-__global__ void __launch_bounds__(NT) k_dphi(const double *__restrict__ phi, const double *__restrict__ mu,
-                                             double *__restrict__ dphi, Grid g) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  dphi_tile<double, N, K, A>(cD, g, phi, mu, dphi, blockIdx.y * TX - 1, blockIdx.x * TY - 1,
-                             *reinterpret_cast<DphiSmem<double, N> *>(smraw));
-}
-
-template <int N, int K>
-__global__ void __launch_bounds__(NT) k_update(const double *__restrict__ phi, const double *__restrict__ mu,
-                                               const double *__restrict__ dphi, double *__restrict__ phin,
-                                               double *__restrict__ mun, Grid g, StatBufs st) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  update_tile<double, N, K>(cD, g, phi, mu, dphi, phin, mun, blockIdx.y * TX, blockIdx.x * TY, st,
-                            (long long)blockIdx.y * gridDim.x + blockIdx.x,
-                            *reinterpret_cast<UpdSmem<double, N, K> *>(smraw));
-}
-
-}  // namespace gpd
-
-namespace {
-
-struct Kern {
-  void (*dphi)(const double *, const double *, double *, gpd::Grid);
-  void (*upd)(const double *, const double *, const double *, double *, double *, gpd::Grid, gpd::StatBufs);
-  size_t smem_dphi, smem_upd;
-};
-
-template <int N, int K, bool A>
-Kern make() {
-  Kern k;
-  k.dphi = gpd::k_dphi<N, K, A>;
-  k.upd = gpd::k_update<N, K>;
-  k.smem_dphi = sizeof(gpd::DphiSmem<double, N>);
-  k.smem_upd = sizeof(gpd::UpdSmem<double, N, K>);
-  return k;
-}
-
-bool pick(int N, int K, bool A, Kern *out) {
-#define CASE(n, k)                                       \
-  if (N == n && K == k) {                                \
-    *out = A ? make<n, k, true>() : make<n, k, false>(); \
-    return true;                                         \
-  }
-  CASE(2, 1) CASE(3, 1) CASE(4, 1) CASE(2, 2) CASE(3, 2) CASE(4, 2)
-#undef CASE
-  return false;
 }
 
 }  // namespace
@@ -1134,15 +1087,7 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
   for (int s = 0; s < nsims; s++)
     if (b->elem == 8 && !(pow2(b->derived[s].dx) && pow2(b->derived[s].dy))) b->mul = false;
   b->diag = true;
-  for (int s = 0; s < nsims; s++) {
-    const gp_derived &d = b->derived[s];
-    for (int a = 0; a < N; a++)
-      for (int k = 0; k < K; k++) {
-        if (d.E[a][k] == 0.0 && std::signbit(d.E[a][k])) b->diag = false;   /* E = -0 */
-        for (int l = 0; l < K; l++)
-          if (k != l && (d.Dbulk[a][k][l] != 0.0 || d.cmu[a][k][l] != 0.0 || d.A[a][k][l] != 0.0)) b->diag = false;
-      }
-  }
+  for (int s = 0; s < nsims; s++) b->diag = b->diag && diagonal(b->derived[s]);
   /* the give-up path of kf_bulk's barrier waits, exercised by a test: the
    * barriers expect more bytes than a box brings, and the polls are few */
   b->mbar_tries = gpd::MBAR_TRIES;
@@ -2131,20 +2076,17 @@ int gp_adjoint_replay(gp_ctx *c, long nsteps, double *max_abs_diff, long long *n
 /* device buffers from its own pool or arena allocator and forbids any     */
 /* other allocation (memory budgets fixed up front, allocator locks it     */
 /* must not contend on, or code paths where a failing allocation cannot be */
-/* handled).  For them the step's only scratch buffer, delta-phi over the  */
-/* interior plus a one-cell ring, lives in this fixed array instead of      */
-/* per-context cudaMalloc'd memory.  Every GPU that loads the library holds */
-/* these 32 MiB until the process exits.                                    */
+/* handled).  For them every tile of the grid is stepped as an interface    */
+/* tile, which keeps delta-phi in shared memory; constants and layout are   */
+/* the kernel's parameters.  (200x152 binary: 18.1 us a call; two passes     */
+/* over a delta-phi array after a copy of the constants took 20.5.)         */
 
-
-#define GP_NOALLOC_SCRATCH_DOUBLES (4u * 1024u * 1024u)   /* 32 MiB */
-static __device__ __align__(256) double g_noalloc_scratch[GP_NOALLOC_SCRATCH_DOUBLES];
+/* grids whose delta-phi planes (with the ring) hold more doubles are refused */
+#define GP_NOALLOC_MAX_DOUBLES (4u * 1024u * 1024u)
 
 #define GP_NOALLOC_MAX_DEVICES 64
-/* Device address of g_noalloc_scratch per device, looked up on the first call
- * on that device.  In host code the array's name only stands in for the
- * symbol; kernels must be given the address cudaGetSymbolAddress returns. */
-static double *g_noalloc_ptr[GP_NOALLOC_MAX_DEVICES];
+/* SM count per device: looked up once, a repeated lookup writes the same value */
+static std::atomic<int> g_noalloc_nsm[GP_NOALLOC_MAX_DEVICES];
 
 extern "C" int gp_step_noalloc(const gp_params *p, const double *phi_in, const double *mu_in, double *phi_out,
                                double *mu_out, void *stream) {
@@ -2156,19 +2098,16 @@ extern "C" int gp_step_noalloc(const gp_params *p, const double *phi_in, const d
   if (gp_host_derive(p, &d, err, sizeof err) != GP_OK) return fail(nullptr, GP_EINVAL, "gp_step_noalloc: %s", err);
   if (d.tgrad || d.shift)
     return fail(nullptr, GP_EUNSUPPORTED, "gp_step_noalloc: isothermal runs without a moving frame only");
-  Kern k;
-  if (!pick(d.N, d.K, d.aniso != 0, &k)) return fail(nullptr, GP_EINVAL, "gp_step_noalloc: no kernel for N=%d K=%d", d.N, d.K);
+  gpd::BatchLaunch L;
+  if (!batch_launch(GP_FP64, d.N, d.K, d.aniso != 0, &L))
+    return fail(nullptr, GP_EINVAL, "gp_step_noalloc: no kernel for N=%d K=%d", d.N, d.K);
   gpd::Grid g = make_grid(d, 1); /* caller's planes are contiguous [field][MESH_X][MESH_Y] */
-  gpd::Consts<double> cs = make_consts<double>(d);
-  /* the scratch holds the delta-phi planes (N of them, interior plus a
-   * one-cell ring); k_dphi rewrites all of it before k_update reads it, so
-   * what an earlier call left there needs no clearing */
   const size_t need = (size_t)d.N * (size_t)g.dplane;
-  if (need > GP_NOALLOC_SCRATCH_DOUBLES)
+  if (need > GP_NOALLOC_MAX_DOUBLES)
     return fail(nullptr, GP_EINVAL,
-                "gp_step_noalloc: grid %ldx%ld with %d phases needs %zu doubles of scratch, the fixed maximum is %u "
-                "(about 1.3 million cells for 3 phases); use gp_init/gp_step for larger grids",
-                d.mx, d.my, d.N, need, GP_NOALLOC_SCRATCH_DOUBLES);
+                "gp_step_noalloc: the delta-phi of a grid of %ldx%ld with %d phases is %zu doubles, the fixed maximum is "
+                "%u (about 1.3 million cells for 3 phases); use gp_init/gp_step for larger grids",
+                d.mx, d.my, d.N, need, GP_NOALLOC_MAX_DOUBLES);
   /* the step reads every input cell's neighbours after other cells' outputs
    * are written: an output range may share no byte with an input range or
    * with the other output range */
@@ -2192,27 +2131,31 @@ extern "C" int gp_step_noalloc(const gp_params *p, const double *phi_in, const d
   int dev = 0;
   CK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= GP_NOALLOC_MAX_DEVICES) return fail(nullptr, GP_EINVAL, "gp_step_noalloc: device %d", dev);
-  if (!g_noalloc_ptr[dev]) {
-    void *ptr = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
-    if (e != cudaSuccess || !ptr)
-      return fail(nullptr, GP_ECUDA, "gp_step_noalloc: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
-    g_noalloc_ptr[dev] = (double *)ptr;
+  if (!g_noalloc_nsm[dev]) {
+    int nsm = 0;
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    g_noalloc_nsm[dev] = nsm;
   }
-  double *scratch = g_noalloc_ptr[dev];
-  cudaStream_t s = (cudaStream_t)stream;
-  CK(cudaFuncSetAttribute(k.dphi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem_dphi));
-  CK(cudaFuncSetAttribute(k.upd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem_upd));
-  CK(cudaMemcpyToSymbolAsync(cD, &cs, sizeof(cs), 0, cudaMemcpyHostToDevice, s));
-  gpd::StatBufs st = {};
-  st.ext = nullptr;      /* no progress record on this path: no extremes */
-  st.partials = nullptr; /* and no sums */
-  st.want_sums = 0;
-  double *dphi = scratch;
-  dim3 gd((g.my + 2 + gpd::TY - 1) / gpd::TY, (g.mx + 2 + gpd::TX - 1) / gpd::TX);
-  dim3 gu((g.my + gpd::TY - 1) / gpd::TY, (g.mx + gpd::TX - 1) / gpd::TX);
-  k.dphi<<<gd, gpd::NT, k.smem_dphi, s>>>(phi_in, mu_in, dphi, g);
-  k.upd<<<gu, gpd::NT, k.smem_upd, s>>>(phi_in, mu_in, dphi, phi_out, mu_out, g, st);
-  CK(cudaGetLastError());
+  gpd::SimDesc sd;
+  memset(&sd, 0, sizeof sd);
+  sd.g = g;
+  sd.tiles_x = (g.my + gpd::TY - 1) / gpd::TY;
+  const gpd::Consts<double> cs = make_consts<double>(d);
+  gpd::StepArgs<double, true> args;
+  L.solo_fill(&args, &cs, &sd);
+  gpd::StepLaunch l;
+  l.stream = (cudaStream_t)stream;
+  l.mul = pow2(d.dx) && pow2(d.dy);
+  l.solo = &args;
+  l.state = phi_in;
+  l.next = phi_out;
+  l.st = {};   /* no progress record on this path */
+  l.st.diag = diagonal(d) ? 1 : 0;
+  gpd::DirectArgs<double, true> da;
+  da.mu = mu_in;
+  da.mu_next = mu_out;
+  da.tiles_x = sd.tiles_x;
+  da.ntiles = sd.tiles_x * ((g.mx + gpd::TX - 1) / gpd::TX);
+  CK(L.direct(l, da, g_noalloc_nsm[dev]));
   return GP_OK;
 }

@@ -804,8 +804,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
     };
     if (v0 && nr > 0) {
       if constexpr (sizeof(R) == 8) {
-        /* ---- FP64: the reference's bulk expressions (update_tile's uniform
-         * path) in their order, two cells at a time */
+        /* ---- FP64: the reference's bulk expressions in their order, two cells at a time */
         double2 P[K], FXP[K][K];
         unsigned redo = 0;   /* DIAG: bit 2 rr + e, cell e of row rr to redo with every term */
         R *mq[K];            /* the row's new mu */
@@ -1120,12 +1119,25 @@ __device__ __forceinline__ const Consts<R> &pick_consts(const StepArgs<R, SOLO> 
   else return *sc;
 }
 
+/* DIRECT: every tile of one simulation on the caller's planes (phi and mu apart,
+ * any pitch), without lists, flags, boxes or a progress record: gp_step_noalloc.
+ * CTA b takes tiles b, b + grid, ... */
+template <typename R, bool DIRECT>
+struct DirectArgs {};
+template <typename R>
+struct DirectArgs<R, true> {
+  const R *mu;
+  R *mu_next;
+  int ntiles, tiles_x;
+};
+
 /* Interface tiles of one step: the CTA takes tiles from the interface list
  * until it is empty, the next one's box in flight while one is stepped.  TG: some
  * simulation is non-isothermal.  A box whose bytes do not arrive within the poll
  * limit sets ctr[CTR_ERR]; the CTA then stops taking tiles. */
-template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
-__device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, const SimDesc *__restrict__ sims,
+template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO, bool DIRECT>
+__device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, const DirectArgs<R, DIRECT> &direct,
+                                              const SimDesc *__restrict__ sims,
                                               const Consts<R> *__restrict__ consts,
                                               const TensorMapSlot *__restrict__ tmaps, int buf,
                                               const R *__restrict__ state, R *__restrict__ next,
@@ -1135,7 +1147,9 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   using IG = ItemGeom<R>;
   constexpr int CO = IG::CO, NWI = NTI / 32;
   constexpr unsigned BOX_BYTES = (unsigned)((N + K) * FR * IG::BW * sizeof(R));
-  const int nlist = *(volatile int *)(ctr + CTR_LIST);
+  int nlist = 0;
+  if constexpr (DIRECT) nlist = direct.ntiles;
+  else nlist = *(volatile int *)(ctr + CTR_LIST);
   if (nlist == 0) return;
   const bool late = st.mixed && (blockIdx.x & 1);   /* after its bulk tiles */
   const int first = late ? -1 : (st.mixed ? blockIdx.x >> 1 : blockIdx.x);
@@ -1146,6 +1160,11 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   Consts<R> *const scp = reinterpret_cast<Consts<R> *>(sc_raw);
   const CT &D = static_cast<const CT &>(pick_consts<R, SOLO>(args, scp));
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  auto entry = [&](int i) {
+    /* (fits: the size limit on padded planes leaves at most 8192 rows of tiles) */
+    if constexpr (DIRECT) return make_int4(i, 0, ((i / direct.tiles_x) << 16) | (i % direct.tiles_x), 0);
+    else return __ldg(glist + i);
+  };
   /* thread 0: note an entry in slot c and start its box */
   auto issue = [&](const int4 &en, int c) {
     sm.ent[c] = en;
@@ -1164,8 +1183,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     if constexpr (sizeof(R) == 8) sm.n_test = sm.n_act = sm.n_task = sm.n_extra = sm.n_j = 0;
     else sm.t.nlist = sm.t.nflist = 0;
     /* the CTAs that begin with interface tiles own the first entries */
-    const int i = first >= 0 ? first : nfirst + atomicAdd(ctr + CTR_HEAD, 1);
-    issue(i < nlist ? __ldg(glist + i) : make_int4(-1, 0, 0, 0), 0);
+    const int i = DIRECT || first >= 0 ? first : nfirst + atomicAdd(ctr + CTR_HEAD, 1);
+    issue(i < nlist ? entry(i) : make_int4(-1, 0, 0, 0), 0);
   }
   int cur_sim = -1;
   unsigned parity = 0;   /* bit c: the phase of slot c's barrier its next box completes */
@@ -1179,7 +1198,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     if (en.x < 0) break;
     const int t = en.x, s = SOLO ? 0 : en.y, x0 = (en.z >> 16) * TX, y0 = (en.z & 0xffff) * TY;
     int nxt = 0;
-    if (tid == 0) nxt = nfirst + atomicAdd(ctr + CTR_HEAD, 1);   /* used after the next barrier */
+    if (DIRECT) nxt = t + (int)gridDim.x;
+    else if (tid == 0) nxt = nfirst + atomicAdd(ctr + CTR_HEAD, 1);   /* used after the next barrier */
     if (s != cur_sim) {
       cur_sim = s;
       if constexpr (!SOLO) {
@@ -1224,7 +1244,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         }
       }
       __syncthreads();
-      const R *src = state + off_state;
+      const R *src = state + off_state, *srcm = src + N * g.plane;
+      if constexpr (DIRECT) srcm = direct.mu;
       for (int q = tid; q < FR * FC; q += NTI) {
         const int i = q / FC, j = q - i * FC;
         const int r = sm.row[0][i], c = sm.col[0][j], rm = sm.row[1][i], cm = sm.col[1][j];
@@ -1232,7 +1253,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         for (int a = 0; a < N; a++) F[a][i][j + CO] = (r >= 0 && c >= 0) ? __ldg(src + a * g.plane + (r + c)) : R(0.0);
 #pragma unroll
         for (int k = 0; k < K; k++)
-          F[N + k][i][j + CO] = (rm >= 0 && cm >= 0) ? __ldg(src + (N + k) * g.plane + (rm + cm)) : R(0.0);
+          F[N + k][i][j + CO] = (rm >= 0 && cm >= 0) ? __ldg(srcm + k * g.plane + (rm + cm)) : R(0.0);
       }
       fence_proxy_async_smem();   /* before a later box overwrites this slot */
       __syncthreads();
@@ -1249,7 +1270,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         break;   /* no other box is in flight */
       }
       int4 nent = make_int4(-1, 0, 0, 0);
-      if (tid == 0 && nxt < nlist) nent = __ldg(glist + nxt);
+      if (tid == 0 && nxt < nlist) nent = entry(nxt);
       tile32<R, N, K, ANISO>(D, g, F, x0, y0, st, sm.t, tpf, tcc, dp, nph, nm, dmu, [&]() {
         if (tid == 0) issue(nent, cur ^ 1);   /* the other slot was last read a tile ago */
       });
@@ -1340,7 +1361,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     }
     const bool dg = st.diag && tame;
     int4 nent = make_int4(-1, 0, 0, 0);
-    if (tid == 0 && nxt < nlist) nent = __ldg(glist + nxt);
+    if (tid == 0 && nxt < nlist) nent = entry(nxt);
 
     /* ---- listed cells: active phases */
     const int ntest = sm.n_test;
@@ -1519,11 +1540,12 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     }
     int oh = -1;
     if (valid) {
-      R *out = next + off_state + (long long)x * g.pitch + y;
+      R *out = next + off_state + (long long)x * g.pitch + y, *outm = out + N * g.plane;
+      if constexpr (DIRECT) outm = direct.mu_next + (long long)x * g.pitch + y;
 #pragma unroll
       for (int a = 0; a < N; a++) out[a * g.plane] = nph[a];
 #pragma unroll
-      for (int k = 0; k < K; k++) out[(N + k) * g.plane] = nm[k];
+      for (int k = 0; k < K; k++) outm[k * g.plane] = nm[k];
       oh = one_hot<R, N>(nph);
       if (st.ext && stat_row(g, x)) item_extremes<R, N, K>(sm.ext, nph, nm, st, s);
     }
@@ -1533,7 +1555,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     }
     if (st.want_sums) item_sums<R, N, K, TG>(D, valid && stat_row(g, x), nph, nm, dp, dmu, st, t, Tc);
     __syncthreads();   /* the tile's shared memory is free, its rows' flag bits are written */
-    if (tid == 32) flag_out[t] = flags_of_rows(sm.fm[cur]);
+    if (!DIRECT && tid == 32) flag_out[t] = flags_of_rows(sm.fm[cur]);
   }
   __syncthreads();
   if (tid == 0) {
@@ -1551,7 +1573,7 @@ __device__ __noinline__ void general_tiles_f32(const SimDesc *__restrict__ sims,
                                                const float *__restrict__ state, float *__restrict__ next,
                                                TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
                                                int *__restrict__ ctr, const StatBufs st) {
-  general_tiles<float, N, K, ANISO, true, TG, false>(StepArgs<float, false>{}, sims, consts, tmaps, buf, state, next,
+  general_tiles<float, N, K, ANISO, true, TG, false, false>(StepArgs<float, false>{}, DirectArgs<float, false>{}, sims, consts, tmaps, buf, state, next,
                                                      flag_out, glist, ctr, st);
 }
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
@@ -1562,7 +1584,8 @@ __device__ __forceinline__ void step_general(const StepArgs<R, SOLO> &args, cons
                                              TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
                                              int *__restrict__ ctr, const StatBufs &st) {
   if constexpr (sizeof(R) == 8)
-    general_tiles<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+    general_tiles<R, N, K, ANISO, MUL, TG, SOLO, false>(args, DirectArgs<R, false>{}, sims, consts, tmaps, buf, state,
+                                                        next, flag_out, glist, ctr, st);
   else
     general_tiles_f32<N, K, ANISO, TG>(sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
 }
@@ -1584,6 +1607,15 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
   pdl_begin();
   step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
   step_finish(ctr, ndone, 1);
+}
+
+/* One step of one simulation on the caller's planes (gp_step_noalloc). */
+template <typename R, int N, int K, bool ANISO, bool MUL>
+__global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kn_step(
+    const __grid_constant__ StepArgs<R, true> args, const __grid_constant__ DirectArgs<R, true> direct,
+    const R *__restrict__ phi, R *__restrict__ phi_next, const __grid_constant__ StatBufs st) {
+  general_tiles<R, N, K, ANISO, MUL, false, true, true>(args, direct, nullptr, nullptr, nullptr, 0, phi, phi_next,
+                                                        nullptr, nullptr, nullptr, st);
 }
 
 /* One step in one persistent launch: each CTA takes interface tiles while

@@ -38,7 +38,7 @@ struct ItemSmem32 {
 #define FB(i, j) F[b][i][(j) + CO]
 
 /* Anisotropy terms of one face of the ring region for all pairs: the same
- * arithmetic as face_terms (function_A_01.h:163-215 through functionQ.h and
+ * order of operations as the reference (function_A_01.h:163-215 through functionQ.h and
  * anisotropy_01.h) on the two-cell-halo layout.  xface: face between P rows
  * i and i+1 at column j; else between columns j and j+1 of row i. */
 template <typename R, int N, int K, typename CT>
@@ -95,7 +95,7 @@ __device__ __forceinline__ void ring_face_terms(const CT &D, ItemFrame<R, N, K> 
 
 /* delta-phi of one ring cell (ring coordinates ri, rj; its phi at P row ri+1,
  * column rj+1) from the staged tile: calculate_divergence_phasefield_2D
- * (calculate_divergence_phasefield.h:4-62) in the same arithmetic as dphi_tile.
+ * (calculate_divergence_phasefield.h:4-62).
  * Not inlined: as a call of its own it gets its own register allocation, and
  * the interface tiles spill far less under the 128-register cap of two CTAs
  * per SM (FP64 ternary 3-phase: 732 bytes of spill stores inlined, about 200

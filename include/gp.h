@@ -269,16 +269,10 @@ void gp_batch_destroy(gp_batch *b);
  * [N][MESH_X][MESH_Y] and [K][MESH_X][MESH_Y] on the current device; neither
  * output may share a byte with an input or with the other output (GP_EINVAL
  * otherwise); stream is a cudaStream_t (NULL = default stream).
- * The step's scratch (delta-phi over the interior plus a one-cell ring) lives
- * in a fixed 32 MiB array inside the library that every GPU which loads the
- * library keeps until exit; grids needing more (about 1.3 million cells with
- * 3 phases) are rejected with GP_EINVAL and a message.  The first call on a
- * device looks up that array's device address (cudaGetSymbolAddress).  No
- * call may be recorded by stream capture: each one copies the step's constant
- * block from host (pageable) memory into the library's __constant__ block,
- * which a captured graph could not replay.  All calls share the array, so
- * calls that overlap on the GPU (other streams, other host threads) race; the
- * same holds for the constant block its kernels read.  The call is
+ * Grids whose delta-phi (N planes with a one-cell ring) is more than 4 Mi
+ * doubles (about 1.3 million cells with 3 phases) are rejected with GP_EINVAL
+ * and a message.  Calls share no device memory beyond the caller's buffers.
+ * Recording a call by stream capture is not supported.  The call is
  * asynchronous on `stream`; no progress record is produced.  Results are those
  * of gp_step. */
 int gp_step_noalloc(const gp_params *p, const double *phi_in, const double *mu_in,
