@@ -258,8 +258,17 @@ class Simulation:
         out = AdjOut()
         out.phi0_bar = g_phi.data_ptr()
         out.mu0_bar = g_mu.data_ptr()
+        # the call's device memory from torch's allocator, which keeps and gives
+        # it back by torch's rules (allocated on the stream waited for below)
+        ws, n = None, lib().gp_adjoint_ws_bytes(self._h, ctypes.byref(req))
+        if n:
+            try:
+                ws = torch.empty(n, dtype=torch.uint8, device=dev)
+            except torch.OutOfMemoryError:
+                n = 0
         torch.cuda.current_stream(dev).synchronize()   # the inputs are written
-        check(lib().gp_adjoint(self._h, ctypes.byref(req), ctypes.byref(out)), self._h)
+        check(lib().gp_adjoint_ws(self._h, ctypes.byref(req), ctypes.byref(out),
+                                  ws.data_ptr() if n else None, n), self._h)
         return _adj_result(out, g_phi, g_mu)
 
     def adjoint_replay(self, nsteps):

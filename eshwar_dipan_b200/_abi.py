@@ -155,6 +155,8 @@ SIGNATURES = {
     "gp_batch_last_error": (ctypes.c_char_p, [c_void_p]),
     "gp_batch_destroy": (None, [c_void_p]),
     "gp_adjoint": (c_int, [c_void_p, POINTER(AdjReq), POINTER(AdjOut)]),
+    "gp_adjoint_ws_bytes": (c_size_t, [c_void_p, POINTER(AdjReq)]),
+    "gp_adjoint_ws": (c_int, [c_void_p, POINTER(AdjReq), POINTER(AdjOut), c_void_p, c_size_t]),
     "gp_adjoint_replay": (c_int, [c_void_p, c_long, POINTER(c_double), POINTER(c_longlong)]),
     "gp_stream": (c_void_p, [c_void_p]),
     "gp_destroy": (None, [c_void_p]),

@@ -289,6 +289,7 @@ struct gp_batch {
   std::vector<gpd::SimDesc> desc;
   int dev, nsm, grid_b, grid_g, grid_s;   /* grid_s: kf_step (0: bulk and interface kernels apart) */
   int grid_w;                   /* ks_tiles (FP64 smoothing) */
+  void *block;                  /* the device memory that the pointers here lie in */
   gpd::ClassifySim csim;        /* a batch of one: its layout for the classification (else tiles_x 0) */
   std::vector<char> solo;       /* a batch of one: its StepArgs (the step kernels' parameter) */
   bool mul;                     /* every simulation's dx and dy are powers of two (or FP32) */
@@ -956,25 +957,9 @@ void gp_batch_destroy(gp_batch *b) {
   if (!b) return;
   if (b->stream) cudaStreamSynchronize(b->stream);
   batch_drop_graphs(b);
-  for (int p = 0; p < 2; p++) cudaFree(b->state[p]);
   for (int i = 0; i < 4; i++)
     if (b->ev[i]) cudaEventDestroy(b->ev[i]);
-  cudaFree(b->flags[0]);   /* flags[1] is part of the same allocation */
-  cudaFree(b->glist);
-  cudaFree(b->blist);
-  cudaFree(b->d_desc);
-  cudaFree(b->d_consts);
-  cudaFree(b->d_tsim);
-  cudaFree(b->d_seg0);
-  cudaFree(b->d_segn);
-  cudaFree(b->ext);
-  cudaFree(b->partials);
-  cudaFree(b->sums_sim);
-  cudaFree(b->counters);
-  cudaFree(b->tmaps);
-  cudaFree(b->trows);
-  cudaFree(b->dyn);
-  cudaFree(b->spos);
+  cudaFree(b->block);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -1148,35 +1133,43 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
       else if (b->ncand > 1) b->tune_next = 0;
     }
   }
-#define BALLOC(ptr, bytes)                                                                        \
-  do {                                                                                            \
-    if (cudaMalloc((void **)&(ptr), (bytes)) != cudaSuccess) {                                     \
-      rc = bfail(b, GP_ENOMEM, "gp_batch_create: cudaMalloc of %zu bytes failed", (size_t)(bytes)); \
-      gp_batch_destroy(b);                                                                        \
-      return rc;                                                                                  \
-    }                                                                                             \
-  } while (0)
-  BALLOC(b->state[0], (size_t)off * b->elem);
-  BALLOC(b->state[1], (size_t)off * b->elem);
-  BALLOC(b->flags[0], 2 * sizeof(gpd::TileFlags) * (size_t)nt);
+  /* one block for all of a batch's buffers: an allocation or a release is a
+   * driver call of 0.1 to 0.7 ms, and a rollout creates two contexts a pass */
+  {
+    std::vector<std::pair<void **, size_t>> parts;
+    size_t bytes = 0;
+    auto part = [&](void *p, size_t n) {
+      parts.push_back({(void **)p, bytes});
+      bytes += (n + 511) / 512 * 512;
+    };
+    part(&b->state[0], (size_t)off * b->elem);
+    part(&b->state[1], (size_t)off * b->elem);
+    part(&b->flags[0], 2 * sizeof(gpd::TileFlags) * (size_t)nt);
+    part(&b->glist, sizeof(int4) * (size_t)nt);
+    part(&b->blist, sizeof(int4) * (size_t)nt);
+    part(&b->d_desc, sizeof(gpd::SimDesc) * nsims);
+    part(&b->d_consts, csz * nsims);
+    part(&b->d_tsim, sizeof(int) * (size_t)nt);
+    part(&b->d_seg0, sizeof(int) * nsims);
+    part(&b->d_segn, sizeof(int) * nsims);
+    part(&b->ext, sizeof(long long) * (size_t)ne * nsims);
+    part(&b->partials, sizeof(double) * (size_t)ns * nt);
+    part(&b->sums_sim, sizeof(double) * (size_t)ns * nsims);
+    part(&b->counters, gpd::CTR_COUNT * sizeof(int));
+    part(&b->tmaps, sizeof(gpd::TensorMapSlot) * 2 * gpd::MAP_KINDS * (size_t)nsims);
+    part(&b->spos, sizeof(int) * (size_t)nsims);
+    part(&b->trows, sizeof(double) * (size_t)std::max(offT, 1));
+    part(&b->dyn, sizeof(gpd::SimDyn) * (size_t)nsims);
+    if (cudaMalloc(&b->block, bytes) != cudaSuccess) {
+      b->block = nullptr;
+      rc = bfail(b, GP_ENOMEM, "gp_batch_create: cudaMalloc of %zu bytes failed", bytes);
+      gp_batch_destroy(b);
+      return rc;
+    }
+    for (const auto &p : parts) *p.first = (char *)b->block + p.second;
+  }
   b->flags[1] = b->flags[0] + nt;
-  BALLOC(b->glist, sizeof(int4) * (size_t)nt);
-  BALLOC(b->blist, sizeof(int4) * (size_t)nt);
-  BALLOC(b->d_desc, sizeof(gpd::SimDesc) * nsims);
-  BALLOC(b->d_consts, csz * nsims);
-  BALLOC(b->d_tsim, sizeof(int) * (size_t)nt);
-  BALLOC(b->d_seg0, sizeof(int) * nsims);
-  BALLOC(b->d_segn, sizeof(int) * nsims);
-  BALLOC(b->ext, sizeof(long long) * (size_t)ne * nsims);
-  BALLOC(b->partials, sizeof(double) * (size_t)ns * nt);
-  BALLOC(b->sums_sim, sizeof(double) * (size_t)ns * nsims);
-  BALLOC(b->counters, gpd::CTR_COUNT * sizeof(int));
-  BALLOC(b->tmaps, sizeof(gpd::TensorMapSlot) * 2 * gpd::MAP_KINDS * (size_t)nsims);
-  BALLOC(b->spos, sizeof(int) * (size_t)nsims);
   if (b->shift) b->tune_next = b->ncand;   /* the first chunks end at the frame checks: no tuning */
-  BALLOC(b->trows, sizeof(double) * (size_t)std::max(offT, 1));
-  BALLOC(b->dyn, sizeof(gpd::SimDyn) * (size_t)nsims);
-#undef BALLOC
   std::vector<gpd::TensorMapSlot> tm(2 * gpd::MAP_KINDS * (size_t)nsims);
   if (encode_all_maps(b, tm.data()) != GP_OK) {
     rc = GP_ECUDA;
@@ -1632,13 +1625,64 @@ struct AdjBufs {
   int *ncells = nullptr;
   gpd::TileFlags *unknown = nullptr;   /* whole-tape mode: "unknown" flags of every tile (redir_have) */
   cudaGraphExec_t first[2] = {nullptr, nullptr};   /* whole-tape mode: the first graph of each sweep */
-  ~AdjBufs() {   /* ybar, xbar and dphibar point into rblk */
+  void *own = nullptr;      /* the block all of these lie in, when it is not the caller's */
+  cudaStream_t stream = nullptr;
+  ~AdjBufs() {
     for (cudaGraphExec_t ge : first)
       if (ge) cudaGraphExecDestroy(ge);
-    cudaFree(snap); cudaFree(seg); cudaFree(dphi); cudaFree(pbar); cudaFree(final_state); cudaFree(rblk);
-    cudaFree(dtape); cudaFree(smaps); cudaFree(cells); cudaFree(ncells); cudaFree(unknown);
+    /* on an early return too, nothing may still run on the caller's block */
+    if (own) cudaFree(own);
+    else cudaStreamSynchronize(stream);
   }
 };
+
+/* What a call keeps, and where it lies in one block of device memory. */
+struct AdjPlan {
+  long nsnap;
+  bool dtape;
+  size_t RB;   /* doubles of a reverse block */
+  size_t snap, seg, rblk, dphi, pbar, final_state, dtape_at, smaps, unknown, cells, ncells, bytes;
+};
+
+/* snapshots of the state besides the start state: the caller's number, or
+ * one state every checkpoint_every steps, or as many as half the free
+ * device memory (fre) holds (every state, when they fit: no step is
+ * recomputed).  With every state kept, the forward pass also keeps each step's
+ * delta-phi when that fits as well, and the reverse sweep does not recompute it. */
+AdjPlan adj_plan(const gp_batch *b, const gp_adj_req *req, size_t fre) {
+  const gpd::Grid &g = b->desc[0].g;
+  const int N = b->derived[0].N, K = b->derived[0].K;
+  const size_t S = (size_t)(N + K) * g.plane, Sd = (size_t)N * g.dplane;
+  const long T = req->nsteps;
+  AdjPlan p;
+  if (req->snapshots > 0) p.nsnap = req->snapshots;
+  else if (req->checkpoint_every > 0) p.nsnap = (T + req->checkpoint_every - 1) / req->checkpoint_every;
+  else p.nsnap = (long)std::min<size_t>((size_t)T, fre / 2 / (S * 8));
+  p.nsnap = std::max(0L, std::min(p.nsnap, T - 1));
+  p.dtape = p.nsnap == T - 1 && (size_t)T * (S + Sd) * 8 <= fre / 2;
+  /* a reverse block: the adjoint of a state (S), of its delta-phi (Sd) and
+   * the two list counters of the reverse passes; a reverse step reads one
+   * block and clears and fills the other with one memset */
+  p.RB = S + Sd + 8;
+  p.bytes = 0;
+  auto take = [&](size_t n) {
+    const size_t at = p.bytes;
+    p.bytes += (n + 511) / 512 * 512;
+    return at;
+  };
+  p.snap = take(S * (size_t)(p.nsnap + 1) * 8);   /* slot 0: the start state */
+  p.seg = take(S * 8);                            /* the state before the last step */
+  p.rblk = take(2 * p.RB * 8);
+  p.dphi = take(Sd * 8);
+  p.pbar = take(gpd::ADJ_NPARAM * 8);
+  p.final_state = take(S * 8);
+  p.cells = take((size_t)(g.mx + 2) * (g.my + 2) * sizeof(int2));
+  p.ncells = take(sizeof(int));
+  p.dtape_at = take(p.dtape ? Sd * (size_t)T * 8 : 0);
+  p.smaps = take(p.dtape ? sizeof(gpd::TensorMapSlot) * gpd::MAP_KINDS * (size_t)T : 0);
+  p.unknown = take(p.dtape ? sizeof(gpd::TileFlags) * (size_t)b->ntiles : 0);
+  return p;
+}
 
 int adj_check(gp_ctx *c, gpd::AdjLaunch *L) {
   if (!c || !c->b) return fail(c, GP_EINVAL, "gp_adjoint: NULL context");
@@ -1684,7 +1728,22 @@ gpd::AdjParams adj_params(const gp_params &p) {
 
 extern "C" {
 
-int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) {
+int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) { return gp_adjoint_ws(c, req, out, nullptr, 0); }
+
+/* A block of 1 GB costs 3 to 4 ms to allocate and 3 to 9 ms to free, in a
+ * call that works for 9 ms on the GPU (512^2, 100 steps); a caller with an
+ * allocator of its own passes it in.  The bound keeps what such an allocator
+ * may hold on to small beside the memory that later contexts need. */
+size_t gp_adjoint_ws_bytes(gp_ctx *c, const gp_adj_req *req) {
+  gpd::AdjLaunch L;
+  if (adj_check(c, &L) != GP_OK || !req || req->nsteps < 1) return 0;
+  size_t fre = 0, tot = 0;
+  if (cudaSetDevice(c->b->dev) != cudaSuccess || cudaMemGetInfo(&fre, &tot) != cudaSuccess) return 0;
+  const size_t n = adj_plan(c->b, req, fre).bytes;
+  return n <= std::min<size_t>((size_t)2 << 30, fre / 16) ? n : 0;
+}
+
+int gp_adjoint_ws(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out, void *ws, size_t ws_bytes) {
   gpd::AdjLaunch L;
   int rc = adj_check(c, &L);
   if (rc) return rc;
@@ -1703,47 +1762,42 @@ int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) {
   const cudaMemcpyKind d2h = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   CK(cudaSetDevice(b->dev));
 
-  /* snapshots of the state besides the start state: the caller's number, or
-   * one state every checkpoint_every steps, or as many as half the free
-   * device memory holds (every state, when they fit: no step is recomputed).
-   * With every state kept, the forward pass also keeps each step's delta-phi
-   * when that fits as well, and the reverse sweep does not recompute it. */
-  long nsnap;
   size_t fre = 0, tot = 0;
   CK(cudaMemGetInfo(&fre, &tot));
-  if (req->snapshots > 0) nsnap = req->snapshots;
-  else if (req->checkpoint_every > 0) nsnap = (T + req->checkpoint_every - 1) / req->checkpoint_every;
-  else nsnap = (long)std::min<size_t>((size_t)T, fre / 2 / (S * 8));
-  nsnap = std::max(0L, std::min(nsnap, T - 1));
-  const bool dtape = nsnap == T - 1 && (size_t)T * (S + Sd) * 8 <= fre / 2;
+  const AdjPlan plan = adj_plan(b, req, fre + ws_bytes);   /* the caller's block would be free without it */
+  const long nsnap = plan.nsnap;
+  const bool dtape = plan.dtape;
   const gpd::AdjParams prm = adj_params(b->params[0]);
   const void *consts = b->d_consts;
   AdjBufs m;
-#define AALLOC(ptr, n)                                                                                  \
-  do {                                                                                                  \
-    if (cudaMalloc((void **)&(ptr), (n) * sizeof(double)) != cudaSuccess)                               \
-      return fail(c, GP_ENOMEM, "gp_adjoint: cudaMalloc of %zu bytes failed", (size_t)(n) * sizeof(double)); \
-  } while (0)
-  /* a reverse block: the adjoint of a state (S), of its delta-phi (Sd) and
-   * the two list counters of the reverse passes; a reverse step reads one
-   * block and clears and fills the other with one memset */
-  const size_t RB = S + Sd + 8;
-  AALLOC(m.snap, S * (size_t)(nsnap + 1));   /* slot 0: the start state */
-  AALLOC(m.seg, S);                          /* the state before the last step */
-  AALLOC(m.rblk, 2 * RB);
-  AALLOC(m.dphi, Sd);
-  AALLOC(m.pbar, gpd::ADJ_NPARAM);
-  AALLOC(m.final_state, S);
-  if (dtape) AALLOC(m.dtape, Sd * (size_t)T);
-#undef AALLOC
+  m.stream = b->stream;
+  char *blk = (char *)ws;
+  if (!blk || ws_bytes < plan.bytes || ((size_t)blk & 255)) {
+    if (cudaMalloc(&m.own, plan.bytes) != cudaSuccess) {
+      m.own = nullptr;
+      return fail(c, GP_ENOMEM, "gp_adjoint: cudaMalloc of %zu bytes failed", plan.bytes);
+    }
+    blk = (char *)m.own;
+  }
+  const size_t RB = plan.RB;
+  m.snap = (double *)(blk + plan.snap);
+  m.seg = (double *)(blk + plan.seg);
+  m.rblk = (double *)(blk + plan.rblk);
+  m.dphi = (double *)(blk + plan.dphi);
+  m.pbar = (double *)(blk + plan.pbar);
+  m.final_state = (double *)(blk + plan.final_state);
+  m.cells = (int2 *)(blk + plan.cells);
+  m.ncells = (int *)(blk + plan.ncells);
+  if (dtape) {
+    m.dtape = (double *)(blk + plan.dtape_at);
+    m.smaps = (gpd::TensorMapSlot *)(blk + plan.smaps);
+    m.unknown = (gpd::TileFlags *)(blk + plan.unknown);
+  }
   if (dtape) {
     std::vector<gpd::TensorMapSlot> hm(gpd::MAP_KINDS * (size_t)T);
     for (long t = 0; t < T; t++)
       if ((rc = encode_maps(b, 0, m.snap + S * (size_t)t, &hm[gpd::MAP_KINDS * (size_t)t])) != GP_OK)
         return fail(c, rc, "%s", b->err);
-    if (cudaMalloc((void **)&m.smaps, sizeof(gpd::TensorMapSlot) * hm.size()) != cudaSuccess ||
-        cudaMalloc((void **)&m.unknown, sizeof(gpd::TileFlags) * (size_t)b->ntiles) != cudaSuccess)
-      return fail(c, GP_ENOMEM, "gp_adjoint: cudaMalloc of the slot maps failed");
     CK(cudaMemcpyAsync(m.smaps, hm.data(), sizeof(gpd::TensorMapSlot) * hm.size(), cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemsetAsync(m.unknown, 0xfe, sizeof(gpd::TileFlags) * (size_t)b->ntiles, b->stream));
     /* the interface tiles write the delta-phi of their cells and rings; every
@@ -1755,12 +1809,6 @@ int gp_adjoint(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out) {
   auto rbar = [&](int k) { return m.rblk + RB * (size_t)k; };
   m.ybar = rbar(0);
   std::vector<char> have_dphi((size_t)T, 0);
-  {
-    const size_t ncell = (size_t)(g.mx + 2) * (g.my + 2);
-    if (cudaMalloc((void **)&m.cells, ncell * sizeof(int2)) != cudaSuccess ||
-        cudaMalloc((void **)&m.ncells, sizeof(int)) != cudaSuccess)
-      return fail(c, GP_ENOMEM, "gp_adjoint: cudaMalloc of the cell list failed");
-  }
   const long long steps0 = b->steps;
   /* the three timing events, destroyed on every return */
   struct Events {

@@ -327,6 +327,16 @@ typedef struct gp_adj_out {
 
 int gp_adjoint(gp_ctx *ctx, const gp_adj_req *req, gp_adj_out *out);
 
+/* gp_adjoint in device memory of the caller's (ws, 256-byte aligned, ws_bytes
+ * long, on the context's device).  Work that used it before has to be complete;
+ * it is free again on return, also after an error.  gp_adjoint_ws_bytes: the
+ * bytes that the request takes, or 0 when the library should allocate them
+ * (over 2 GiB or a sixteenth of the free memory, or a request that gp_adjoint
+ * refuses).  With a NULL, unaligned or smaller ws the call allocates and frees
+ * its memory like gp_adjoint. */
+size_t gp_adjoint_ws_bytes(gp_ctx *ctx, const gp_adj_req *req);
+int gp_adjoint_ws(gp_ctx *ctx, const gp_adj_req *req, gp_adj_out *out, void *ws, size_t ws_bytes);
+
 /* Verification of the adjoint's cell functions: nsteps steps evaluated with
  * them (one thread per cell, no tiles) against gp_step's kernels from the same
  * start state; *max_abs_diff receives the largest difference of any field
