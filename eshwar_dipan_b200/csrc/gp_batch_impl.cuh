@@ -225,14 +225,10 @@ struct BatchKernels {
   }
   static cudaError_t smooth(cudaStream_t s, const void *consts, const void *phi, const void *mu, void *phin,
                             void *mun, Grid g, const double *tcc) {
-    if constexpr (sizeof(R) == 4) {
-      dim3 grid((g.my + 127) / 128, g.mx);
-      k_smooth<R, N, K, A><<<grid, 128, 0, s>>>((const Consts<R> *)consts, (const R *)phi, (const R *)mu, (R *)phin,
-                                                (R *)mun, g, tcc);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
+    dim3 grid((g.my + 127) / 128, g.mx);
+    k_smooth<R, N, K, A><<<grid, 128, 0, s>>>((const Consts<R> *)consts, (const R *)phi, (const R *)mu, (R *)phin,
+                                              (R *)mun, g, tcc);
+    return cudaGetLastError();
   }
   static cudaError_t shift_pos(int ntiles, cudaStream_t s, const SimDesc *sims, const void *consts, const int *tsim,
                                const void *state, int *pos) {

@@ -1220,7 +1220,19 @@ int gp_batch_smooth(gp_batch *b, long nsteps) {
   /* the sweeps run before the first step: the temperature as copied at t = 0 */
   if (b->tgrad && nsteps > 0)
     BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
-  if (b->elem == 8) {
+  /* FP64: three dependent launches by tile kind take about 20 us before the size
+   * counts; one launch over every cell takes 11 us and grows with the cells and
+   * their fields.  Measured us a sweep, every cell / by tile kind: two phases, 1024
+   * tiles 17.5 / 28.9, 1920 tiles 25 / 30, 3072 tiles 36 / 33; four phases and two
+   * solutes, 532 tiles 23 / 36, 1024 tiles 34 / 38, 1920 tiles 57 / 40.  Both cross
+   * where tiles * fields is about 8000.  Over every cell each simulation is a launch
+   * of its own, which moves the line: three of 300^2 with three fields 27.8 / 31.0,
+   * four 36 / 31; two of 300^2 with five fields 29 / 36, three 41 / 37; two of 200x256
+   * with six fields 35.3 / 36.8, of 300^2 40 / 37. */
+  const long fields = b->N + b->K, launch = fields == 3 ? 2100 : fields < 6 ? 3000 : 5000;
+  const bool by_kind = b->elem == 8 && (b->nsims > (fields == 3 ? 3 : 2) ||
+                                        (long)b->ntiles * fields + launch * (b->nsims - 1) >= 8000);
+  if (by_kind) {
     /* the step's classification and bulk tiles, the listed rest by ks_tiles */
     for (long t = 0; t < nsteps; t++) {
       gpd::StepLaunch l = batch_launch_args(b, 0);

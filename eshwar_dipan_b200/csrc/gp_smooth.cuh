@@ -10,8 +10,9 @@
  * there is a zero), so the step's classification and kf_bulk take those tiles and
  * ks_tiles the listed rest, over all simulations of a batch at once.  The nine
  * sweeps of a 2048^2 ternary grid with 64 seeds: every cell by the general path
- * 2.9 ms; bulk tiles apart 0.5 ms.  The FP32 form rounds a bulk cell of a sweep to
- * nearest and of a step stochastically, and keeps one kernel over every cell.
+ * 2.9 ms; bulk tiles apart 0.5 ms.  Small grids (gp_batch_smooth has the line) take
+ * k_smooth, one launch over every cell.  So does the FP32 form: it rounds a bulk cell
+ * of a sweep to nearest and of a step stochastically.
  */
 #pragma once
 #include "gp_fused.cuh"
@@ -198,7 +199,7 @@ __device__ __forceinline__ void smooth_cell(const Consts<R> &D, const R *__restr
   supd_cell<R, N, K>(D, phi, mu, d, nph, phin, mun, g, tcc, np, nq, x, y);
 }
 
-/* One FP32 sweep, one thread per interior cell. */
+/* One sweep, one thread per interior cell. */
 template <typename R, int N, int K, bool ANISO>
 __global__ void __launch_bounds__(128, N <= 3 ? 4 : 3) k_smooth(const Consts<R> *__restrict__ Dp, const R *__restrict__ phi, const R *__restrict__ mu,
                          R *__restrict__ phin, R *__restrict__ mun, Grid g, const double *__restrict__ tcc) {

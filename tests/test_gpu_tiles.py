@@ -77,3 +77,38 @@ def test_noalloc(tmp_path, name):
             assert np.isfinite(b).all()
             assert bits_equal(a.cpu().numpy(), b), "call %d: %s" % (n, mismatch_report(a.cpu().numpy(), b))
         src, dst = dst, src
+
+
+@pytest.mark.parametrize("name", ["above", "below", "iso", "whole"])
+def test_smooth_by_tile_kinds_in_a_batch(tmp_path, name):
+    """Four simulations take the sweep by tile kinds at any size (one of these
+    grids alone takes one launch over every cell)."""
+    p, phi, mu, o = _start(tmp_path, name)
+    b = gp.Batch([p] * 4, [(phi, mu)] * 4, precision=gp.GP_FP64)
+    o.smooth(9)
+    o.step(1)
+    b.smooth(9)
+    b.step(1, stats=False)
+    for s in range(4):
+        for x, y in zip(b.get(s), o.get()):
+            assert bits_equal(x, y), mismatch_report(x, y)
+    b.close()
+
+
+@pytest.mark.parametrize("tiles", [2666, 2667])
+def test_smooth_on_both_sides_of_the_line(tmp_path, tiles):
+    """tiles * (phases + solutes) just below and above 8000."""
+    mesh = (8, 32 * tiles)
+    ip, fp = write_case(str(tmp_path), "line", dict(N=2, K=1, mesh=mesh, dab=0.03, d_solid=0.0),
+                        seeds=[(0, 3, 40 + 9000 * i, 6.0) for i in range(8)])
+    p = gp.load_params(ip)
+    phi, mu = gp.fill(p, fp)
+    o = Oracle(p, recip_div=1)
+    o.set(phi, mu)
+    with gp.Simulation(p, phi, mu) as sim:
+        sim.smooth(3)
+        sim.step(1, stats=False)
+        o.smooth(3)
+        o.step(1)
+        for a, b in zip(sim.get(), o.get()):
+            assert bits_equal(a, b), mismatch_report(a, b)
