@@ -2138,8 +2138,8 @@ int gp_adjoint_replay(gp_ctx *c, long nsteps, double *max_abs_diff, long long *n
 /* must not contend on, or code paths where a failing allocation cannot be */
 /* handled).  For them every tile of the grid is stepped as an interface    */
 /* tile, which keeps delta-phi in shared memory; constants and layout are   */
-/* the kernel's parameters.  (200x152 binary: 18.1 us a call; two passes     */
-/* over a delta-phi array after a copy of the constants took 20.5.)         */
+/* the kernel's parameters.  (200x152 binary: 18 to 20 us a call; two passes */
+/* over a delta-phi array after a copy of the constants took 20.5 to 22.)   */
 
 /* grids whose delta-phi planes (with the ring) hold more doubles are refused */
 #define GP_NOALLOC_MAX_DOUBLES (4u * 1024u * 1024u)

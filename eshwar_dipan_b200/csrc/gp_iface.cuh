@@ -25,9 +25,9 @@
  * instruction fetches as the two whole ones), and in a batch of one the constants
  * in the kernel's parameters, where they are operands and not shared-memory loads.
  * Measured, all interface tiles of a step before and after (B200, FP64): 5034
- * tiles of a 4096^2 ternary three-phase grid 394 to 233 us; 1260 anisotropic ones
- * of a 2048^2 grid 155 to 105 us; 440 with a rotated pair and 1.5-spaced cells 150
- * to 81 us; 268 four-phase ones 58 to 47 us.
+ * tiles of a 4096^2 ternary three-phase grid 394 to 226 us; 1260 anisotropic ones
+ * of a 2048^2 grid 155 to 100 us; 440 with a rotated pair and 1.5-spaced cells 150
+ * to 77 us; 268 four-phase ones 58 to 41 us.
  * The arithmetic of each cell is the reference's, in its order (FP64; the FP32
  * form's tiles are in gp_iface32.cuh).  Terms of a
  * phase that is exactly zero over a stencil are left out: each is +-0 added to a
