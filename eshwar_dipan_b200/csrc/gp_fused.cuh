@@ -156,6 +156,15 @@ __device__ __forceinline__ TileFlags flags_of_rows(const unsigned *w) {
   return t;
 }
 
+__device__ __forceinline__ TileFlags ld_step(const TileFlags *p) {
+  union {
+    unsigned long long w;
+    TileFlags t;
+  } v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v.w) : "l"(p));
+  return v.t;
+}
+
 __device__ __forceinline__ TileFlags uniform_flags(int p) {
   TileFlags t;
   t.whole = t.top = t.bot = t.left = t.right = (signed char)p;
@@ -176,16 +185,16 @@ struct ClassifySim {
  * neighbour tiles (a corner by either band that contains it); otherwise by the
  * whole-tile flags of the tiles that hold the halo cells after the boundary
  * remap. */
-__device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags *__restrict__ flags, int tile0, int by,
+__device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags *flags, int tile0, int by,
                                           int bx) {
   const int tiles_x = g.tiles_x;
   const int x0 = by * TX, y0 = bx * TY;
   const int xl = min(x0 + TX, g.mx) - 1, yl = min(y0 + TY, g.my) - 1;
   if (x0 >= 2 && xl + 2 < g.mx && y0 >= 2 && yl + 2 < g.my) {
     const TileFlags *f = flags + tile0 + by * tiles_x + bx;
-    const TileFlags ul = f[-tiles_x - 1], u = f[-tiles_x], ur = f[-tiles_x + 1];
-    const TileFlags l = f[-1], c = f[0], r = f[1];
-    const TileFlags dl = f[tiles_x - 1], d = f[tiles_x], dr = f[tiles_x + 1];
+    const TileFlags ul = ld_step(f - tiles_x - 1), u = ld_step(f - tiles_x), ur = ld_step(f - tiles_x + 1);
+    const TileFlags l = ld_step(f - 1), c = ld_step(f), r = ld_step(f + 1);
+    const TileFlags dl = ld_step(f + tiles_x - 1), d = ld_step(f + tiles_x), dr = ld_step(f + tiles_x + 1);
     const int p = c.whole;
     const bool ok = p >= 0 && u.bot == p && d.top == p && l.right == p && r.left == p &&
                     (ul.bot == p || ul.right == p) && (ur.bot == p || ur.left == p) &&
@@ -208,10 +217,10 @@ __device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags 
       cols[q + 1] = y / TY;
     }
   }
-  const int p = flags[tile0 + by * tiles_x + bx].whole;
+  const int p = ld_step(flags + tile0 + by * tiles_x + bx).whole;
   bool ok = p >= 0;
 #pragma unroll
-  for (int q = 0; q < 25; q++) ok = ok && flags[tile0 + rows[q / 5] * tiles_x + cols[q % 5]].whole == p;
+  for (int q = 0; q < 25; q++) ok = ok && ld_step(flags + tile0 + rows[q / 5] * tiles_x + cols[q % 5]).whole == p;
   return ok ? p : -1;
 }
 
@@ -232,7 +241,7 @@ enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR
 
 /* Programmatic dependent launch: the kernels of a step are launched while their
  * predecessor still runs (every one of its CTAs has started) and wait here, before
- * they read anything it writes, until it has completed.  A launch gap of a graph
+ * they read anything it writes (with ld_step only), until it has completed.  A launch gap of a graph
  * is about 1 us; a step has two.  Graph time of a step, before and after: 256^2 20.7
  * to 18.4 us, 1024^2 34.0 to 30.7; large grids within 2 % (2048^2 119.7 to 121.6). */
 __device__ __forceinline__ void pdl_begin() {
@@ -274,8 +283,8 @@ constexpr int NTC = 64;
 template <typename R>
 __global__ void __launch_bounds__(NTC) kf_classify(const ClassifySim solo, const SimDesc *__restrict__ sims,
                                                   const Consts<R> *__restrict__ consts, const int *__restrict__ tsim,
-                                                  int ntiles, const TileFlags *__restrict__ flag_in,
-                                                  const TileFlags *__restrict__ flag_outbuf,
+                                                  int ntiles, const TileFlags *flag_in,
+                                                  const TileFlags *flag_outbuf,
                                                   int4 *__restrict__ glist, int4 *__restrict__ blist,
                                                   int *__restrict__ ctr) {
   const int t = blockIdx.x * NTC + threadIdx.x, lane = threadIdx.x & 31;
@@ -316,7 +325,7 @@ __global__ void __launch_bounds__(NTC) kf_classify(const ClassifySim solo, const
   if (t < ntiles) {
     if (p >= 0)
       blist[bb + __popc(mb & below)] =
-          make_int4(t | (p << 28), s | (((int)flag_outbuf[t].whole & 0xff) << 24), (by << 16) | bx, 0);
+          make_int4(t | (p << 28), s | (((int)ld_step(flag_outbuf + t).whole & 0xff) << 24), (by << 16) | bx, 0);
     else
       glist[bg + __popc(mg & below)] = make_int4(t, s, (by << 16) | bx, inside);
   }
@@ -482,9 +491,8 @@ __device__ __forceinline__ void bulk_cell_full_f64(const double *__restrict__ st
  * beside the interface code it made both spill. */
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
 __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
-                                           const int4 *__restrict__ blist,
-                                           const TensorMapSlot *__restrict__ tmaps, int buf,
-                                           const R *__restrict__ state, R *__restrict__ next,
+                                           const int4 *blist, const TensorMapSlot *__restrict__ tmaps, int buf,
+                                           const R *state, R *__restrict__ next,
                                            TileFlags *__restrict__ flag_out, int *__restrict__ ctr,
                                            const StatBufs st) {
   using G = BulkGeom<R, K>;
@@ -568,7 +576,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
     n = max(0, min(c, nbulk - start));
     const int r = lane - 16 * half;
     if (r >= 0 && r < n) {
-      const int4 e = __ldg(blist + start + r);
+      const int4 e = ld_step(blist + start + r);
       q_item = e.x;
       q_s = e.y;
       q_xy = e.z;
@@ -639,7 +647,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
   /* FP32: flux-divergence coefficients of the bulk update (x and y) */
   f2 CX2[K][K], CY2[K][K];
   /* FP32: the step's part of the rounding key */
-  const unsigned skey = sizeof(R) == 4 ? mix32(__ldg(st.round_step) * 0x9e3779b9u + 0x632be5abu) : 0u;
+  const unsigned skey = sizeof(R) == 4 ? mix32(ld_step(st.round_step) * 0x9e3779b9u + 0x632be5abu) : 0u;
 
   /* the qi-th box a warp issues goes to stage qi % NST and completes phase
    * (qi / NST) & 1 of that stage's barrier; NST-1 boxes are in flight while a
@@ -740,7 +748,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
           if (y < 0 || y >= g.my) y = remap(y, g.my, by0, by1);
           const R *src = mu + (long long)x * g.pitch + y;
 #pragma unroll
-          for (int k = 0; k < K; k++) sg.M[k][i][j + CO] = __ldg(src + (long long)k * g.plane);
+          for (int k = 0; k < K; k++) sg.M[k][i][j + CO] = ld_step(src + (long long)k * g.plane);
         }
       }
       fence_proxy_async_smem();   /* before a later box overwrites this stage */
@@ -1088,8 +1096,8 @@ __device__ __forceinline__ void bulk_release_warp() {
 
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
 __global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk(
-    const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist,
-    const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
+    const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *blist,
+    const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
   bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
@@ -1141,8 +1149,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
                                               const SimDesc *__restrict__ sims,
                                               const Consts<R> *__restrict__ consts,
                                               const TensorMapSlot *__restrict__ tmaps, int buf,
-                                              const R *__restrict__ state, R *__restrict__ next,
-                                              TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                              const R *state, R *__restrict__ next,
+                                              TileFlags *__restrict__ flag_out, const int4 *glist,
                                               int *__restrict__ ctr, const StatBufs &st) {
   using CT = typename std::conditional<MUL, ConstsMul<R>, Consts<R>>::type;
   using IG = ItemGeom<R>;
@@ -1164,7 +1172,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   auto entry = [&](int i) {
     /* (fits: the size limit on padded planes leaves at most 8192 rows of tiles) */
     if constexpr (DIRECT) return make_int4(i, 0, ((i / direct.tiles_x) << 16) | (i % direct.tiles_x), 0);
-    else return __ldg(glist + i);
+    else return ld_step(glist + i);
   };
   /* thread 0: note an entry in slot c and start its box */
   auto issue = [&](const int4 &en, int c) {
@@ -1250,11 +1258,19 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
       for (int q = tid; q < FR * FC; q += NTI) {
         const int i = q / FC, j = q - i * FC;
         const int r = sm.row[0][i], c = sm.col[0][j], rm = sm.row[1][i], cm = sm.col[1][j];
+        R v[N + K];
 #pragma unroll
-        for (int a = 0; a < N; a++) F[a][i][j + CO] = (r >= 0 && c >= 0) ? __ldg(src + a * g.plane + (r + c)) : R(0.0);
+        for (int f = 0; f < N + K; f++) v[f] = R(0.0);
+        if (r >= 0 && c >= 0) {
 #pragma unroll
-        for (int k = 0; k < K; k++)
-          F[N + k][i][j + CO] = (rm >= 0 && cm >= 0) ? __ldg(srcm + k * g.plane + (rm + cm)) : R(0.0);
+          for (int a = 0; a < N; a++) v[a] = ld_step(src + a * g.plane + (r + c));
+        }
+        if (rm >= 0 && cm >= 0) {
+#pragma unroll
+          for (int k = 0; k < K; k++) v[N + k] = ld_step(srcm + k * g.plane + (rm + cm));
+        }
+#pragma unroll
+        for (int f = 0; f < N + K; f++) F[f][i][j + CO] = v[f];
       }
       fence_proxy_async_smem();   /* before a later box overwrites this slot */
       __syncthreads();
@@ -1264,7 +1280,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     const bool valid = x < g.mx && y < g.my;
     R dp[N], nph[N], nm[K];
     double dmu[K];
-    const double Tc = (TG && D.tgrad && valid) ? tcc[y + 3] : 0.0;
+    const double Tc = (TG && D.tgrad && valid) ? ld_step(tcc + y + 3) : 0.0;
     if constexpr (sizeof(R) == 4) {
       if (!__syncthreads_and(ok)) {
         if (tid == 0) atomicExch(ctr + CTR_ERR, 1);
@@ -1491,7 +1507,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         if (q < ntask) {
           const int v = sm.TASK[q], e = v & 1023;
           item_lambda<R, N, K, ANISO, TG>(D, F, sm, e, v >> 10, tame, dg,
-                                          TG && D.tgrad ? tpf[y0 - 1 + e % RC + 3] : 0.0);
+                                          TG && D.tgrad ? ld_step(tpf + y0 - 1 + e % RC + 3) : 0.0);
         } else if (q >= t32) {
           const int e = sm.LIST[q - t32], ri = e / RC, rj = e - ri * RC;
           const unsigned act = sm.ACT[e];
@@ -1571,8 +1587,8 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
 template <int N, int K, bool ANISO, bool TG>
 __device__ __noinline__ void general_tiles_f32(const SimDesc *__restrict__ sims, const Consts<float> *__restrict__ consts,
                                                const TensorMapSlot *__restrict__ tmaps, int buf,
-                                               const float *__restrict__ state, float *__restrict__ next,
-                                               TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                               const float *state, float *__restrict__ next,
+                                               TileFlags *__restrict__ flag_out, const int4 *glist,
                                                int *__restrict__ ctr, const StatBufs st) {
   general_tiles<float, N, K, ANISO, true, TG, false, false>(StepArgs<float, false>{}, DirectArgs<float, false>{}, sims, consts, tmaps, buf, state, next,
                                                      flag_out, glist, ctr, st);
@@ -1581,8 +1597,8 @@ template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
 __device__ __forceinline__ void step_general(const StepArgs<R, SOLO> &args, const SimDesc *__restrict__ sims,
                                              const Consts<R> *__restrict__ consts,
                                              const TensorMapSlot *__restrict__ tmaps, int buf,
-                                             const R *__restrict__ state, R *__restrict__ next,
-                                             TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
+                                             const R *state, R *__restrict__ next,
+                                             TileFlags *__restrict__ flag_out, const int4 *glist,
                                              int *__restrict__ ctr, const StatBufs &st) {
   if constexpr (sizeof(R) == 8)
     general_tiles<R, N, K, ANISO, MUL, TG, SOLO, false>(args, DirectArgs<R, false>{}, sims, consts, tmaps, buf, state,
@@ -1603,8 +1619,8 @@ template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
     const Consts<R> *__restrict__ consts, const TensorMapSlot *__restrict__ tmaps, int buf,
-    const R *__restrict__ state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
-    const int4 *__restrict__ glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+    const R *state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
+    const int4 *glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
   step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
   step_finish(ctr, ndone, 1);
@@ -1627,8 +1643,8 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kn_step(
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO, bool DIAG>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
     const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
-    const Consts<R> *__restrict__ consts, const int4 *__restrict__ blist, const int4 *__restrict__ glist,
-    const TensorMapSlot *__restrict__ tmaps, int buf, const R *__restrict__ state, R *__restrict__ next,
+    const Consts<R> *__restrict__ consts, const int4 *blist, const int4 *glist,
+    const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
   const int bulk_pass = st.mixed && (blockIdx.x & 1) ? 0 : 1;

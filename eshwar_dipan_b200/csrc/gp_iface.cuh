@@ -408,7 +408,7 @@ __device__ __forceinline__ R item_sphi(ItemFrame<R, N, K> F, int i, int j, int a
 /* Anti-trapping current through face f of the tile (calculate_fluxes_concentration.h:4-145) */
 template <typename R, int N, int K, bool ANISO, bool TG, typename CT>
 __device__ __forceinline__ void item_current(const CT &D, ItemFrame<R, N, K> F, ItemSmem<R, N, K, ANISO> &sm, int f,
-                                             int y0, int my, bool dg, const double *__restrict__ tcc) {
+                                             int y0, int my, bool dg, const double *tcc) {
   constexpr int L = N - 1, CO = ItemGeom<R>::CO, BW = ItemGeom<R>::BW;
   const bool xface = f < JXF;
   const int f0 = f - JXF;
@@ -429,8 +429,8 @@ __device__ __forceinline__ void item_current(const CT &D, ItemFrame<R, N, K> F, 
     at_T = D.tgrad;
     if (at_T) {
       /* the ghosted columns of the two cells (cells past my+1 are not needed: clamped) */
-      e_at<R, N, K>(D, tcc[min(y0 - 1 + fj + 3, my + 5)], E0);
-      e_at<R, N, K>(D, tcc[min(y0 - 1 + (xface ? fj : fj + 1) + 3, my + 5)], E1);
+      e_at<R, N, K>(D, ld_step(tcc + min(y0 - 1 + fj + 3, my + 5)), E0);
+      e_at<R, N, K>(D, ld_step(tcc + min(y0 - 1 + (xface ? fj : fj + 1) + 3, my + 5)), E1);
     }
   }
   /* the gradient across the face and the mean tangential one */

@@ -268,8 +268,8 @@ __device__ __noinline__ void ring_dphi(const CT &D, ItemFrame<R, N, K> F, const 
  * dmu.  hook: called once by every thread after the first pass. */
 template <typename R, int N, int K, bool ANISO, typename CT, typename HOOK>
 __device__ __forceinline__ void tile32(const CT &D, const Grid &g, ItemFrame<R, N, K> F, int x0, int y0,
-                                       const StatBufs &st, ItemSmem32<R, N, K> &sm, const double *__restrict__ tpf,
-                                       const double *__restrict__ tcc, R (&dp)[N], R (&nph)[N], R (&nm)[K],
+                                       const StatBufs &st, ItemSmem32<R, N, K> &sm, const double *tpf,
+                                       const double *tcc, R (&dp)[N], R (&nph)[N], R (&nm)[K],
                                        double (&dmu)[K], HOOK &&hook) {
   constexpr int L = N - 1, CO = ItemGeom<R>::CO;
 
@@ -344,7 +344,7 @@ __device__ __forceinline__ void tile32(const CT &D, const Grid &g, ItemFrame<R, 
     const int e = sm.LIST[q];
     const int ri = e / SW, rj = e - ri * SW;
     R d[N];
-    ring_dphi<R, N, K, ANISO>(D, F, sm, ri, rj, sm.ACT[e], d, D.tgrad ? tpf[y0 - 1 + rj + 3] : 0.0);
+    ring_dphi<R, N, K, ANISO>(D, F, sm, ri, rj, sm.ACT[e], d, D.tgrad ? ld_step(tpf + y0 - 1 + rj + 3) : 0.0);
 #pragma unroll
     for (int a = 0; a < N; a++) sm.DP[a][e] = d[a];
   }
@@ -365,7 +365,7 @@ __device__ __forceinline__ void tile32(const CT &D, const Grid &g, ItemFrame<R, 
     for (int k = 0; k < K; k++) mm[k] = MR(k, e);
     R Ec[N][K];
     /* the ghosted column of ring cell e (cells past my+1 are not needed: clamped) */
-    if (D.tgrad) e_at<R, N, K>(D, tcc[min(y0 - 1 + e % SW + 3, g.my + 5)], Ec);
+    if (D.tgrad) e_at<R, N, K>(D, ld_step(tcc + min(y0 - 1 + e % SW + 3, g.my + 5)), Ec);
 #pragma unroll
     for (int a = 0; a < N; a++) {
       R hv = h<R, N>(p, a);
@@ -459,7 +459,7 @@ __device__ __forceinline__ void tile32(const CT &D, const Grid &g, ItemFrame<R, 
 #pragma unroll
     for (int k = 0; k < K; k++) m[k] = MR(k, c);
     commit_cell<R, N, K>(D, sm.w.u.FX, sm.w.u.FY, sm.w.u.JX, sm.w.u.JY, sm.w.u.CM, sm.w.u.H, i, j, x, y, ph, dp, m,
-                         nph, nm, dmu, st, D.tgrad ? tcc[y + 3] : 0.0);
+                         nph, nm, dmu, st, D.tgrad ? ld_step(tcc + y + 3) : 0.0);
   }
 #undef PRIJ
 #undef PR

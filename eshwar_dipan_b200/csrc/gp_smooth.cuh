@@ -39,10 +39,18 @@ __device__ __forceinline__ Nbr3 nbr3(const Consts<R> &D, const Grid &g, int fiel
   return n;
 }
 
+/* A sweep's loads: STEP for ks_tiles, which is launched while its predecessor runs
+ * (ld_step); k_smooth is an ordinary launch and takes the read-only path. */
+template <bool STEP, typename T>
+__device__ __forceinline__ T ld_sweep(const T *p) {
+  if constexpr (STEP) return ld_step(p);
+  else return __ldg(p);
+}
+
 /* calculate_divergence_phasefield_smooth_2D (calculate_divergence_phasefield.h:63-158)
  * at interior cell (x, y): its delta-phi into d. */
-template <typename R, int N, bool ANISO>
-__device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *__restrict__ phi, const Grid &g,
+template <typename R, int N, bool ANISO, bool STEP>
+__device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *phi, const Grid &g,
                                            const Nbr3 &np, R (&d)[N]) {
   R S[N][3][3];
 #pragma unroll
@@ -50,7 +58,7 @@ __device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *__restri
 #pragma unroll
     for (int u = 0; u < 3; u++)
 #pragma unroll
-      for (int v = 0; v < 3; v++) S[a][u][v] = __ldg(phi + a * g.plane + np.o(u, v));
+      for (int v = 0; v < 3; v++) S[a][u][v] = ld_sweep<STEP>(phi + a * g.plane + np.o(u, v));
   R ph[N], dv[N], gcx[N], gcy[N], lam[N];
   bool act[N];
 #pragma unroll
@@ -108,10 +116,10 @@ __device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *__restri
 /* calculate_divergence_concentration_smooth_2D (calculate_divergence_concentration.h:154-253)
  * at interior cell (x, y), given the cell's delta-phi of the sweep (the pass
  * reads no other cell's) */
-template <typename R, int N, int K>
-__device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *__restrict__ phi, const R *__restrict__ mu,
+template <typename R, int N, int K, bool STEP>
+__device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *phi, const R *mu,
                                           const R (&dph)[N], R (&nph)[N], R *__restrict__ phin, R *__restrict__ mun,
-                                          const Grid &g, const double *__restrict__ tcc, const Nbr3 &np,
+                                          const Grid &g, const double *tcc, const Nbr3 &np,
                                           const Nbr3 &nq, int x, int y) {
   /* cells: 0 centre, 1 front (x+1), 2 back (x-1), 3 right (y+1), 4 left (y-1) */
   const int cu[5] = {1, 2, 0, 1, 1}, cv[5] = {1, 1, 1, 2, 0};
@@ -119,9 +127,9 @@ __device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *__restric
 #pragma unroll
   for (int q = 0; q < 5; q++) {
 #pragma unroll
-    for (int a = 0; a < N; a++) P[q][a] = __ldg(phi + a * g.plane + np.o(cu[q], cv[q]));
+    for (int a = 0; a < N; a++) P[q][a] = ld_sweep<STEP>(phi + a * g.plane + np.o(cu[q], cv[q]));
 #pragma unroll
-    for (int k = 0; k < K; k++) M[q][k] = __ldg(mu + k * g.plane + nq.o(cu[q], cv[q]));
+    for (int k = 0; k < K; k++) M[q][k] = ld_sweep<STEP>(mu + k * g.plane + nq.o(cu[q], cv[q]));
 #pragma unroll
     for (int k = 0; k < K; k++)
 #pragma unroll
@@ -151,7 +159,7 @@ __device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *__restric
     R cn[K], E[N][K];
     /* the cell's temperature in a non-isothermal run
      * (calculate_divergence_concentration.h:167-170) */
-    if (D.tgrad) e_at<R, N, K>(D, tcc[y + 3], E);
+    if (D.tgrad) e_at<R, N, K>(D, ld_sweep<STEP>(tcc + y + 3), E);
 #pragma unroll
     for (int k = 0; k < K; k++)
       cn[k] = (D.tgrad ? c_muE<R, K>(D, E[bulk], m, bulk, k) : c_mu<R, K>(D, m, bulk, k)) + D.dt * (divflux[k]);
@@ -189,14 +197,14 @@ __device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *__restric
  * cell, then the concentration pass's update, which reads the delta-phi of no
  * other cell (the two passes in one, without a delta-phi buffer between them).
  * nph: the cell's new phi. */
-template <typename R, int N, int K, bool ANISO>
-__device__ __forceinline__ void smooth_cell(const Consts<R> &D, const R *__restrict__ phi, const R *__restrict__ mu,
+template <typename R, int N, int K, bool ANISO, bool STEP>
+__device__ __forceinline__ void smooth_cell(const Consts<R> &D, const R *phi, const R *mu,
                                             R (&nph)[N], R *__restrict__ phin, R *__restrict__ mun, const Grid &g,
-                                            const double *__restrict__ tcc, int x, int y) {
+                                            const double *tcc, int x, int y) {
   const Nbr3 np = nbr3(D, g, 0, x, y), nq = nbr3(D, g, 1, x, y);
   R d[N];
-  sdphi_cell<R, N, ANISO>(D, phi, g, np, d);
-  supd_cell<R, N, K>(D, phi, mu, d, nph, phin, mun, g, tcc, np, nq, x, y);
+  sdphi_cell<R, N, ANISO, STEP>(D, phi, g, np, d);
+  supd_cell<R, N, K, STEP>(D, phi, mu, d, nph, phin, mun, g, tcc, np, nq, x, y);
 }
 
 /* One sweep, one thread per interior cell. */
@@ -206,7 +214,7 @@ __global__ void __launch_bounds__(128, N <= 3 ? 4 : 3) k_smooth(const Consts<R> 
   const int y = blockIdx.x * blockDim.x + threadIdx.x, x = blockIdx.y;
   if (y >= g.my) return;
   R nph[N];
-  smooth_cell<R, N, K, ANISO>(*Dp, phi, mu, nph, phin, mun, g, tcc, x, y);
+  smooth_cell<R, N, K, ANISO, false>(*Dp, phi, mu, nph, phin, mun, g, tcc, x, y);
 }
 
 /* The listed tiles of a sweep over a batch: persistent CTAs over the interface
@@ -214,9 +222,9 @@ __global__ void __launch_bounds__(128, N <= 3 ? 4 : 3) k_smooth(const Consts<R> 
  * the ndone CTAs of this kernel and kf_bulk empties the lists; a sweep is no step. */
 template <typename R, int N, int K, bool ANISO>
 __global__ void __launch_bounds__(NT, N <= 3 ? 2 : 1) ks_tiles(
-    const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const R *__restrict__ state,
-    R *__restrict__ next, TileFlags *__restrict__ flag_out, const int4 *__restrict__ glist,
-    const double *__restrict__ trows, int *__restrict__ ctr, int ndone) {
+    const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const R *state,
+    R *__restrict__ next, TileFlags *__restrict__ flag_out, const int4 *glist,
+    const double *trows, int *__restrict__ ctr, int ndone) {
   __shared__ int s_item;
   __shared__ unsigned s_w[TX];
   pdl_begin();
@@ -226,7 +234,7 @@ __global__ void __launch_bounds__(NT, N <= 3 ? 2 : 1) ks_tiles(
     __syncthreads();
     const int item = s_item;
     if (item >= nlist) break;
-    const int4 en = __ldg(glist + item);
+    const int4 en = ld_step(glist + item);
     const SimDesc &sd = sims[en.y];
     const Grid g = sd.g;
     const int x = (en.z >> 16) * TX + wid, y = (en.z & 0xffff) * TY + lane;
@@ -237,7 +245,7 @@ __global__ void __launch_bounds__(NT, N <= 3 ? 2 : 1) ks_tiles(
       R *phin = next + sd.off_state;
       const long long om = (long long)N * g.plane;
       R nph[N];
-      smooth_cell<R, N, K, ANISO>(consts[en.y], phi, phi + om, nph, phin, phin + om, g,
+      smooth_cell<R, N, K, ANISO, true>(consts[en.y], phi, phi + om, nph, phin, phin + om, g,
                                   trows ? trows + sd.off_T + (g.my + 6) : nullptr, x, y);
       oh = one_hot<R, N>(nph);
     }

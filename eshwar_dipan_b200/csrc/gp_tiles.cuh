@@ -139,6 +139,32 @@ __device__ __forceinline__ long long ord(double v) {
   return i < 0 ? i ^ 0x7fffffffffffffffLL : i;
 }
 
+/* Loads of what a step's kernels write: states, flags, lists, counters, temperature
+ * rows.  The kernels of a step are launched while the one that writes these still
+ * runs (pdl_begin, gp_fused.cuh), so they are not read-only for a kernel's lifetime:
+ * no __ldg, no const __restrict__ pointer to them, and no load that the compiler
+ * may move to before the wait (volatile, as the wait is). */
+__device__ __forceinline__ double ld_step(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_step(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_step(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int4 ld_step(const int4 *p) {
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 struct StatBufs {
   long long *ext;      /* running extremes [simulations][2*(N+K)] (ordered ints, atomic max/min), or NULL */
   double *partials;    /* [tiles][2N+2K+1] sums when want_sums */
@@ -305,7 +331,7 @@ __device__ __forceinline__ void commit_cell(const CT &D, const R (&FX)[K][K][NXF
     R cn[K];
 #pragma unroll
     for (int k = 0; k < K; k++) cn[k] = D.dt * (divflux[k]) - divjat[k];
-    bulk_commit_f32<R, N, K>(D, bulk, cn, ph, dp, m, nph, nm, dmu, round_key(__ldg(st.round_step), x, y));
+    bulk_commit_f32<R, N, K>(D, bulk, cn, ph, dp, m, nph, nm, dmu, round_key(ld_step(st.round_step), x, y));
   } else if (bulk >= 0) {
     R cn[K];
 #pragma unroll
@@ -371,7 +397,7 @@ __device__ __forceinline__ void commit_cell(const CT &D, const R (&FX)[K][K][NXF
 #pragma unroll
       for (int a = 0; a < N; a++) nph[a] = ph[a] + dp[a];
     } else {
-      const unsigned key = round_key(__ldg(st.round_step), x, y);
+      const unsigned key = round_key(ld_step(st.round_step), x, y);
 #pragma unroll
       for (int k = 0; k < K; k++) nm[k] = round_stochastic(m64[k], key, N + k);
 #pragma unroll
