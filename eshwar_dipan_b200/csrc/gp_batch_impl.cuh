@@ -24,7 +24,8 @@ struct StepLaunch {
   const SimDesc *sims;
   const void *consts;
   const int4 *blist, *glist;
-  const TensorMapSlot *tmaps;   /* per simulation and state buffer the maps MAP_MU and MAP_ALL */
+  BoxMaps maps;                 /* a batch of one: the maps of `state` */
+  const TensorMapSlot *tmaps;   /* else, per simulation and state buffer, the maps MAP_MU and MAP_ALL (device) */
   int buf;                      /* the buffer `state` is */
   const void *state;
   void *next;
@@ -156,14 +157,14 @@ struct BatchKernels {
     cudaError_t e = cudaSuccess;
     with_step(l, [&](auto k, const auto &args) {
       e = launch_dependent(k, l.grid, NTI, step_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.blist,
-                           l.glist, l.tmaps, l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
+                           l.glist, l.maps, l.tmaps, l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
     return e;
   }
   static cudaError_t bulk(const StepLaunch &l) {
     cudaError_t e = cudaSuccess;
     with_bulk(l, l.st.want_sums != 0, [&](auto k) {
-      e = launch_dependent(k, l.grid, NTI, bulk_smem, l.stream, l.sims, (const Consts<R> *)l.consts, l.blist, l.tmaps,
+      e = launch_dependent(k, l.grid, NTI, bulk_smem, l.stream, l.sims, (const Consts<R> *)l.consts, l.blist, l.maps, l.tmaps,
                            l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
     return e;
@@ -171,7 +172,7 @@ struct BatchKernels {
   static cudaError_t general(const StepLaunch &l) {
     cudaError_t e = cudaSuccess;
     with_general(l, [&](auto k, const auto &args) {
-      e = launch_dependent(k, l.grid, NTI, item_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.tmaps,
+      e = launch_dependent(k, l.grid, NTI, item_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.maps, l.tmaps,
                            l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.ctr, l.ndone, l.st);
     });
     return e;

@@ -313,6 +313,7 @@ struct gp_batch {
   int4 *blist;                  /* bulk tiles of the current step (entries written by kf_classify) */
   int *counters;                /* gpd::CTR_* */
   gpd::TensorMapSlot *tmaps;    /* [nsims][2][MAP_KINDS]: TMA maps of each simulation's planes in state[0], state[1] */
+  std::vector<gpd::TensorMapSlot> hmaps;   /* a batch of one: the same on the host (a parameter of its launches) */
   int cur;
   long long *ext;               /* running extremes per simulation [nsims][2(N+K)] */
   bool tgrad;                   /* some simulation is non-isothermal: temperature rows each step */
@@ -384,8 +385,11 @@ static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   l.consts = b->d_consts;
   l.blist = b->blist;
   l.glist = b->glist;
-  l.tmaps = b->redir_in ? b->redir_map : b->tmaps;
-  l.buf = b->redir_in ? 0 : in;
+  l.maps.one = b->nsims == 1;
+  if (l.maps.one)
+    memcpy(l.maps.m, b->redir_in ? b->redir_map : b->hmaps.data() + in * gpd::MAP_KINDS, sizeof l.maps.m);
+  l.tmaps = b->tmaps;
+  l.buf = in;
   l.state = b->redir_in ? b->redir_in : b->state[in];
   l.next = b->redir_in ? b->redir_out : b->state[out];
   l.flag_out = b->flags[out];
@@ -1193,6 +1197,7 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
   BUP(b->d_segn, segn.data(), sizeof(int) * nsims);
   BUP(b->ext, ext.data(), sizeof(long long) * ext.size());
   BUP(b->tmaps, tm.data(), sizeof(gpd::TensorMapSlot) * tm.size());
+  if (nsims == 1) b->hmaps = tm;
 #undef BUP
   if (cudaMemsetAsync(b->dyn, 0, sizeof(gpd::SimDyn) * (size_t)nsims, b->stream) != cudaSuccess ||
       cudaMemsetAsync(b->counters, 0, gpd::CTR_COUNT * sizeof(int), b->stream) != cudaSuccess) {
@@ -1632,7 +1637,6 @@ struct AdjBufs {
          *pbar = nullptr, *final_state = nullptr;
   double *rblk = nullptr;   /* two reverse blocks: adjoint of a state, adjoint of its delta-phi, list counters */
   double *dtape = nullptr;  /* delta-phi of every step, written by the forward pass (whole-tape mode) */
-  gpd::TensorMapSlot *smaps = nullptr;   /* whole-tape mode: the tensor maps of each slot's planes */
   int2 *cells = nullptr;    /* cells of a reverse pass that take the dual passes */
   int *ncells = nullptr;
   gpd::TileFlags *unknown = nullptr;   /* whole-tape mode: "unknown" flags of every tile (redir_have) */
@@ -1653,7 +1657,7 @@ struct AdjPlan {
   long nsnap;
   bool dtape;
   size_t RB;   /* doubles of a reverse block */
-  size_t snap, seg, rblk, dphi, pbar, final_state, dtape_at, smaps, unknown, cells, ncells, bytes;
+  size_t snap, seg, rblk, dphi, pbar, final_state, dtape_at, unknown, cells, ncells, bytes;
 };
 
 /* snapshots of the state besides the start state: the caller's number, or
@@ -1691,7 +1695,6 @@ AdjPlan adj_plan(const gp_batch *b, const gp_adj_req *req, size_t fre) {
   p.cells = take((size_t)(g.mx + 2) * (g.my + 2) * sizeof(int2));
   p.ncells = take(sizeof(int));
   p.dtape_at = take(p.dtape ? Sd * (size_t)T * 8 : 0);
-  p.smaps = take(p.dtape ? sizeof(gpd::TensorMapSlot) * gpd::MAP_KINDS * (size_t)T : 0);
   p.unknown = take(p.dtape ? sizeof(gpd::TileFlags) * (size_t)b->ntiles : 0);
   return p;
 }
@@ -1802,15 +1805,9 @@ int gp_adjoint_ws(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out, void *ws, s
   m.ncells = (int *)(blk + plan.ncells);
   if (dtape) {
     m.dtape = (double *)(blk + plan.dtape_at);
-    m.smaps = (gpd::TensorMapSlot *)(blk + plan.smaps);
     m.unknown = (gpd::TileFlags *)(blk + plan.unknown);
   }
   if (dtape) {
-    std::vector<gpd::TensorMapSlot> hm(gpd::MAP_KINDS * (size_t)T);
-    for (long t = 0; t < T; t++)
-      if ((rc = encode_maps(b, 0, m.snap + S * (size_t)t, &hm[gpd::MAP_KINDS * (size_t)t])) != GP_OK)
-        return fail(c, rc, "%s", b->err);
-    CK(cudaMemcpyAsync(m.smaps, hm.data(), sizeof(gpd::TensorMapSlot) * hm.size(), cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemsetAsync(m.unknown, 0xfe, sizeof(gpd::TileFlags) * (size_t)b->ntiles, b->stream));
     /* the interface tiles write the delta-phi of their cells and rings; every
      * other cell of every step keeps this +0.0 */
@@ -1942,18 +1939,21 @@ int gp_adjoint_ws(gp_ctx *c, const gp_adj_req *req, gp_adj_out *out, void *ws, s
    * from graph to graph): the host captures a graph while the GPU runs the
    * one before it, and the first graph of each sweep before the timed
    * region, as a plain run's graphs are captured before it runs. */
+  gpd::TensorMapSlot slot_map[gpd::MAP_KINDS];   /* of the slot a step reads; a launch takes a copy */
   auto capture_forward = [&](long t0, cudaGraphExec_t *ge) -> int {
     const long t1 = std::min<long>(T, t0 + GP_GRAPH_STEPS);
     return capture_graph(
         b,
         [&]() -> int {
           for (long t = t0; t < t1; t++) {
+            int r = encode_maps(b, 0, slot_ptr((int)t), slot_map);
+            if (r != GP_OK) return r;
             b->redir_in = slot_ptr((int)t);
             b->redir_out = t + 1 < T ? slot_ptr((int)t + 1) : m.final_state;
-            b->redir_map = m.smaps + gpd::MAP_KINDS * t;
+            b->redir_map = slot_map;
             b->redir_have = m.unknown;
             b->dphi_out = m.dtape + Sd * (size_t)t;
-            const int r = batch_step_once(b, 0, nullptr);
+            r = batch_step_once(b, 0, nullptr);
             b->redir_in = nullptr;
             b->redir_out = nullptr;
             b->redir_map = nullptr;

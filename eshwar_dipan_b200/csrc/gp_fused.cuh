@@ -389,6 +389,29 @@ struct alignas(64) TensorMapSlot {
   unsigned long long w[16];
 };
 
+/* The maps of a batch of one (one != 0), for the buffer a launch reads: they come as
+ * a kernel parameter, where the launch itself makes them current.  A batch of
+ * several reads them from global memory. */
+struct BoxMaps {
+  TensorMapSlot m[MAP_KINDS];
+  int one;
+};
+
+/* The map of a box of simulation s, to be used by the calling thread.  The copy unit
+ * keeps descriptors it has read; one in global memory may be an older one's from the
+ * same address until a fence on it, once per block and map (ready: the last map the
+ * thread fenced). */
+__device__ __forceinline__ const TensorMapSlot *box_map(const BoxMaps &maps, const TensorMapSlot *tmaps, int s, int buf,
+                                                        int kind, const TensorMapSlot *&ready) {
+  if (maps.one) return &maps.m[kind];
+  const TensorMapSlot *const m = tmaps + (2 * s + buf) * MAP_KINDS + kind;
+  if (m != ready) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
+    ready = m;
+  }
+  return m;
+}
+
 /* Shared memory of one warp of kf_bulk: NST stages of mu with a one-cell halo,
  * each filled by one TMA box.  A box starts CO columns left of the halo
  * column so that its first column is 16-byte aligned (y0 - 1 - CO is a
@@ -491,7 +514,8 @@ __device__ __forceinline__ void bulk_cell_full_f64(const double *__restrict__ st
  * beside the interface code it made both spill. */
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
 __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts,
-                                           const int4 *blist, const TensorMapSlot *__restrict__ tmaps, int buf,
+                                           const int4 *blist, const BoxMaps &maps,
+                                           const TensorMapSlot *__restrict__ tmaps, int buf,
                                            const R *state, R *__restrict__ next,
                                            TileFlags *__restrict__ flag_out, int *__restrict__ ctr,
                                            const StatBufs st) {
@@ -608,13 +632,14 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
     pa++;
     return true;
   };
+  const TensorMapSlot *ready = nullptr;
   /* lane 0: start the TMA box of a tile into stage b and note its entry */
   auto issue = [&](const BulkEntry &en, int b) {
     if (lane == 0) {
       ws.meta[b] = en;
       const unsigned bar = smem_addr(&ws.bar[b]);
       mbar_expect_tx(bar, G::BOX_BYTES + st.tma_extra);
-      tma_load_3d(smem_addr(&ws.st[b]), tmaps + (2 * en.s + buf) * MAP_KINDS + MAP_MU, en.y0 - 1 - CO, en.x0 - 1, 0, bar);
+      tma_load_3d(smem_addr(&ws.st[b]), box_map(maps, tmaps, en.s, buf, MAP_MU, ready), en.y0 - 1 - CO, en.x0 - 1, 0, bar);
     }
   };
 
@@ -1097,10 +1122,10 @@ __device__ __forceinline__ void bulk_release_warp() {
 template <typename R, int N, int K, bool SUMS, bool MUL, bool DIAG>
 __global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk(
     const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *blist,
-    const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
+    const __grid_constant__ BoxMaps maps, const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
-  bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
+  bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, maps, tmaps, buf, state, next, flag_out, ctr, st);
   step_finish(ctr, ndone, st.sweep ? 0 : 1);
 }
 
@@ -1147,7 +1172,7 @@ struct DirectArgs<R, true> {
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO, bool DIRECT>
 __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, const DirectArgs<R, DIRECT> &direct,
                                               const SimDesc *__restrict__ sims,
-                                              const Consts<R> *__restrict__ consts,
+                                              const Consts<R> *__restrict__ consts, const BoxMaps &maps,
                                               const TensorMapSlot *__restrict__ tmaps, int buf,
                                               const R *state, R *__restrict__ next,
                                               TileFlags *__restrict__ flag_out, const int4 *glist,
@@ -1174,14 +1199,15 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     if constexpr (DIRECT) return make_int4(i, 0, ((i / direct.tiles_x) << 16) | (i % direct.tiles_x), 0);
     else return ld_step(glist + i);
   };
+  const TensorMapSlot *ready = nullptr;
   /* thread 0: note an entry in slot c and start its box */
   auto issue = [&](const int4 &en, int c) {
     sm.ent[c] = en;
-    if (en.x >= 0 && en.w) {
+    if (!DIRECT && en.x >= 0 && en.w) {
       const unsigned bar = smem_addr(&sm.bar[c]);
       mbar_expect_tx(bar, BOX_BYTES + st.tma_extra);
-      tma_load_3d(smem_addr(&sm.F[c]), tmaps + (2 * en.y + buf) * MAP_KINDS + MAP_ALL, (en.z & 0xffff) * TY - 2 - CO,
-                  (en.z >> 16) * TX - 2, 0, bar);
+      tma_load_3d(smem_addr(&sm.F[c]), box_map(maps, tmaps, en.y, buf, MAP_ALL, ready),
+                  (en.z & 0xffff) * TY - 2 - CO, (en.z >> 16) * TX - 2, 0, bar);
     }
   };
   if (tid == 0) {
@@ -1586,25 +1612,25 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
  * kernel calls, so that its fused multiply-adds are the same in all of them. */
 template <int N, int K, bool ANISO, bool TG>
 __device__ __noinline__ void general_tiles_f32(const SimDesc *__restrict__ sims, const Consts<float> *__restrict__ consts,
-                                               const TensorMapSlot *__restrict__ tmaps, int buf,
+                                               const BoxMaps &maps, const TensorMapSlot *__restrict__ tmaps, int buf,
                                                const float *state, float *__restrict__ next,
                                                TileFlags *__restrict__ flag_out, const int4 *glist,
                                                int *__restrict__ ctr, const StatBufs st) {
-  general_tiles<float, N, K, ANISO, true, TG, false, false>(StepArgs<float, false>{}, DirectArgs<float, false>{}, sims, consts, tmaps, buf, state, next,
-                                                     flag_out, glist, ctr, st);
+  general_tiles<float, N, K, ANISO, true, TG, false, false>(StepArgs<float, false>{}, DirectArgs<float, false>{}, sims, consts, maps, tmaps, buf,
+                                                     state, next, flag_out, glist, ctr, st);
 }
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
 __device__ __forceinline__ void step_general(const StepArgs<R, SOLO> &args, const SimDesc *__restrict__ sims,
-                                             const Consts<R> *__restrict__ consts,
+                                             const Consts<R> *__restrict__ consts, const BoxMaps &maps,
                                              const TensorMapSlot *__restrict__ tmaps, int buf,
                                              const R *state, R *__restrict__ next,
                                              TileFlags *__restrict__ flag_out, const int4 *glist,
                                              int *__restrict__ ctr, const StatBufs &st) {
   if constexpr (sizeof(R) == 8)
-    general_tiles<R, N, K, ANISO, MUL, TG, SOLO, false>(args, DirectArgs<R, false>{}, sims, consts, tmaps, buf, state,
-                                                        next, flag_out, glist, ctr, st);
+    general_tiles<R, N, K, ANISO, MUL, TG, SOLO, false>(args, DirectArgs<R, false>{}, sims, consts, maps, tmaps, buf,
+                                                        state, next, flag_out, glist, ctr, st);
   else
-    general_tiles_f32<N, K, ANISO, TG>(sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+    general_tiles_f32<N, K, ANISO, TG>(sims, consts, maps, tmaps, buf, state, next, flag_out, glist, ctr, st);
 }
 
 /* CTAs of the interface code an SM holds: what its shared memory leaves, at most two (128 registers a thread) */
@@ -1618,11 +1644,12 @@ constexpr int item_ctas() {
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
-    const Consts<R> *__restrict__ consts, const TensorMapSlot *__restrict__ tmaps, int buf,
-    const R *state, R *__restrict__ next, TileFlags *__restrict__ flag_out,
-    const int4 *glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
+    const Consts<R> *__restrict__ consts, const __grid_constant__ BoxMaps maps,
+    const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
+    TileFlags *__restrict__ flag_out, const int4 *glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
-  step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr, st);
+  step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, maps, tmaps, buf, state, next, flag_out, glist, ctr,
+                                                 st);
   step_finish(ctr, ndone, 1);
 }
 
@@ -1631,8 +1658,8 @@ template <typename R, int N, int K, bool ANISO, bool MUL>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kn_step(
     const __grid_constant__ StepArgs<R, true> args, const __grid_constant__ DirectArgs<R, true> direct,
     const R *__restrict__ phi, R *__restrict__ phi_next, const __grid_constant__ StatBufs st) {
-  general_tiles<R, N, K, ANISO, MUL, false, true, true>(args, direct, nullptr, nullptr, nullptr, 0, phi, phi_next,
-                                                        nullptr, nullptr, nullptr, st);
+  general_tiles<R, N, K, ANISO, MUL, false, true, true>(args, direct, nullptr, nullptr, BoxMaps{}, nullptr, 0, phi,
+                                                        phi_next, nullptr, nullptr, nullptr, st);
 }
 
 /* One step in one persistent launch: each CTA takes interface tiles while
@@ -1643,7 +1670,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kn_step(
 template <typename R, int N, int K, bool ANISO, bool MUL, bool TG, bool SOLO, bool DIAG>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
     const __grid_constant__ StepArgs<R, SOLO> args, const SimDesc *__restrict__ sims,
-    const Consts<R> *__restrict__ consts, const int4 *blist, const int4 *glist,
+    const Consts<R> *__restrict__ consts, const int4 *blist, const int4 *glist, const __grid_constant__ BoxMaps maps,
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
   pdl_begin();
@@ -1651,11 +1678,11 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {
     if (pass == bulk_pass) {
-      bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, blist, tmaps, buf, state, next, flag_out, ctr, st);
+      bulk_tiles<R, N, K, false, MUL, DIAG>(sims, consts, blist, maps, tmaps, buf, state, next, flag_out, ctr, st);
       bulk_release_warp<R, K>();
     } else {
-      step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, tmaps, buf, state, next, flag_out, glist, ctr,
-                                                   st);
+      step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, maps, tmaps, buf, state, next, flag_out, glist,
+                                                   ctr, st);
     }
     __syncthreads();   /* the pass's shared memory becomes the next one's */
   }
