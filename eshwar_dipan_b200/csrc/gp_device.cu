@@ -385,8 +385,8 @@ static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   l.consts = b->d_consts;
   l.blist = b->blist;
   l.glist = b->glist;
-  l.maps.one = b->nsims == 1;
-  if (l.maps.one)
+  l.maps.nsims = b->nsims;
+  if (b->nsims == 1)
     memcpy(l.maps.m, b->redir_in ? b->redir_map : b->hmaps.data() + in * gpd::MAP_KINDS, sizeof l.maps.m);
   l.tmaps = b->tmaps;
   l.buf = in;

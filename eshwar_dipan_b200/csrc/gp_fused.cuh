@@ -217,10 +217,13 @@ __device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags 
       cols[q + 1] = y / TY;
     }
   }
-  const int p = ld_step(flags + tile0 + by * tiles_x + bx).whole;
+  int w[25];   /* all loads first: one after the other they would be a chain */
+#pragma unroll
+  for (int q = 0; q < 25; q++) w[q] = ld_step(flags + tile0 + rows[q / 5] * tiles_x + cols[q % 5]).whole;
+  const int p = w[0];   /* the tile itself */
   bool ok = p >= 0;
 #pragma unroll
-  for (int q = 0; q < 25; q++) ok = ok && ld_step(flags + tile0 + rows[q / 5] * tiles_x + cols[q % 5]).whole == p;
+  for (int q = 1; q < 25; q++) ok = ok & (w[q] == p);
   return ok ? p : -1;
 }
 
@@ -244,9 +247,11 @@ enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR
  * they read anything it writes (with ld_step only), until it has completed.  A launch gap of a graph
  * is about 1 us; a step has two.  Graph time of a step, before and after: 256^2 20.7
  * to 18.4 us, 1024^2 34.0 to 30.7; large grids within 2 % (2048^2 119.7 to 121.6). */
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_launch();
+  pdl_wait();
 }
 
 /* End of one CTA of the step's bulk or interface kernel (they may run
@@ -389,24 +394,51 @@ struct alignas(64) TensorMapSlot {
   unsigned long long w[16];
 };
 
-/* The maps of a batch of one (one != 0), for the buffer a launch reads: they come as
+/* The maps of a batch of one (nsims 1), for the buffer a launch reads: they come as
  * a kernel parameter, where the launch itself makes them current.  A batch of
  * several reads them from global memory. */
 struct BoxMaps {
   TensorMapSlot m[MAP_KINDS];
-  int one;
+  int nsims;
 };
 
-/* The map of a box of simulation s, to be used by the calling thread.  The copy unit
- * keeps descriptors it has read; one in global memory may be an older one's from the
- * same address until a fence on it, once per block and map (ready: the last map the
- * thread fenced). */
+/* The copy unit keeps descriptors it has read; one in global memory may be an older
+ * one's from the same address until a block has fenced it.  The host writes the maps
+ * once, before any step, so in a batch of at most BOX_FENCE_AHEAD simulations every
+ * block fences all of them ahead of its wait, while the kernel before finishes; in a
+ * larger one a thread fences a map when it moves to its simulation.  Step times,
+ * ahead / at each move: 24 simulations of 128^2 to 1024^2 82 / 89 us, 64 of 256^2 50
+ * / 54 us, 256 of 256^2 148 / 148 us, 256 of 128^2 110 / 103 us, 1024 of 64^2 443 /
+ * 380 us (FP32; FP64 alike). */
+constexpr int BOX_FENCE_AHEAD = 128;
+__device__ __forceinline__ void box_fence(const TensorMapSlot *m) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
+}
+/* Start of a kernel that issues boxes of the kinds in KINDS (bit k: kind k).  SOLO: a
+ * batch of one. */
+template <unsigned KINDS, bool SOLO>
+__device__ __forceinline__ void box_begin(const BoxMaps &maps, const TensorMapSlot *tmaps, int buf) {
+  pdl_launch();
+  if (!SOLO && maps.nsims > 1 && maps.nsims <= BOX_FENCE_AHEAD) {
+    static_assert(BOX_FENCE_AHEAD <= NTI, "a thread per simulation");
+    const int s = threadIdx.x;
+    if (s < maps.nsims) {
+#pragma unroll
+      for (int k = 0; k < MAP_KINDS; k++)
+        if ((KINDS >> k) & 1u) box_fence(tmaps + (2 * s + buf) * MAP_KINDS + k);
+    }
+    __syncthreads();
+  }
+  pdl_wait();
+}
+/* the map of a box of simulation s, after box_begin, to be used by the calling thread
+ * (ready: the map that it fenced last) */
 __device__ __forceinline__ const TensorMapSlot *box_map(const BoxMaps &maps, const TensorMapSlot *tmaps, int s, int buf,
                                                         int kind, const TensorMapSlot *&ready) {
-  if (maps.one) return &maps.m[kind];
+  if (maps.nsims == 1) return &maps.m[kind];
   const TensorMapSlot *const m = tmaps + (2 * s + buf) * MAP_KINDS + kind;
-  if (m != ready) {
-    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
+  if (maps.nsims > BOX_FENCE_AHEAD && m != ready) {
+    box_fence(m);
     ready = m;
   }
   return m;
@@ -1124,7 +1156,7 @@ __global__ void __launch_bounds__(NTI, sizeof(R) == 4 && K == 1 ? 3 : 2) kf_bulk
     const SimDesc *__restrict__ sims, const Consts<R> *__restrict__ consts, const int4 *blist,
     const __grid_constant__ BoxMaps maps, const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
-  pdl_begin();
+  box_begin<1u << MAP_MU, false>(maps, tmaps, buf);
   bulk_tiles<R, N, K, SUMS, MUL, DIAG>(sims, consts, blist, maps, tmaps, buf, state, next, flag_out, ctr, st);
   step_finish(ctr, ndone, st.sweep ? 0 : 1);
 }
@@ -1647,7 +1679,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
     const Consts<R> *__restrict__ consts, const __grid_constant__ BoxMaps maps,
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, const int4 *glist, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
-  pdl_begin();
+  box_begin<1u << MAP_ALL, SOLO>(maps, tmaps, buf);
   step_general<R, N, K, ANISO, MUL, TG, SOLO>(args, sims, consts, maps, tmaps, buf, state, next, flag_out, glist, ctr,
                                                  st);
   step_finish(ctr, ndone, 1);
@@ -1673,7 +1705,7 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_step(
     const Consts<R> *__restrict__ consts, const int4 *blist, const int4 *glist, const __grid_constant__ BoxMaps maps,
     const TensorMapSlot *__restrict__ tmaps, int buf, const R *state, R *__restrict__ next,
     TileFlags *__restrict__ flag_out, int *__restrict__ ctr, int ndone, const __grid_constant__ StatBufs st) {
-  pdl_begin();
+  box_begin<1u << MAP_MU | 1u << MAP_ALL, SOLO>(maps, tmaps, buf);
   const int bulk_pass = st.mixed && (blockIdx.x & 1) ? 0 : 1;
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {

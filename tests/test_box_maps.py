@@ -1,6 +1,8 @@
 """Tensor maps of the step kernels' boxes: a map in global memory needs an
 acquire fence before a block's first use of it (the copy unit may hold what lay
-at its address before); a batch of one gets its maps as a kernel parameter.
+at its address before); a batch of one gets its maps as a kernel parameter, one of
+up to 128 fences them all at the start of a block, a larger one where a thread
+moves to a simulation.
 
 The GPU tests put different maps at the same addresses one after the other.
 States are compared bit for bit.  Gradients: as in test_gpu_adjoint_ws.py.
@@ -26,11 +28,21 @@ def test_boxes_take_their_map_from_box_map():
         src = re.sub(r"/\*.*?\*/|//[^\n]*", "", f.read(), flags=re.S)
     calls = re.findall(r"(?<!void )tma_load_3d\(smem_addr\([^()]*\),\s*(\w+)", src)
     assert calls == ["box_map", "box_map"]
-    body = src[src.index("*box_map("):]
-    body = body[:body.index("\n}\n")]
-    fence = body.index("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;")
-    # only the kernel parameter's map is returned before the fence
-    assert re.findall(r"return ([^;]*);", body[:fence]) == ["&maps.m[kind]"]
+    def body(name):
+        t = src[src.index(name):]
+        return t[:t.index("\n}\n")]
+
+    assert "fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" in body("void box_fence(")
+    # the kernel parameter's map, else a fence ahead of the wait or here
+    assert re.findall(r"return ([^;]*);", body("*box_map(")) == ["&maps.m[kind]", "m"]
+    assert re.search(r"if \(maps.nsims > BOX_FENCE_AHEAD && m != ready\) \{\s*box_fence\(m\);", body("*box_map("))
+    ahead = body("void box_begin(")
+    assert "maps.nsims > 1 && maps.nsims <= BOX_FENCE_AHEAD" in ahead
+    assert ahead.index("box_fence(") < ahead.index("__syncthreads();") < ahead.index("pdl_wait();")
+    for kernel, kinds in (("kf_bulk", "1u << MAP_MU"), ("kf_general", "1u << MAP_ALL"),
+                          ("kf_step", "1u << MAP_MU | 1u << MAP_ALL")):
+        k = src[src.index(" %s(\n" % kernel):]
+        assert re.search(r"\{\s*box_begin<([^,]*),", k).group(1) == kinds
     params = re.findall(r"([\w ]*)BoxMaps maps,", src)
     assert len(params) == 3 and all(q.strip() == "const __grid_constant__" for q in params)
 
@@ -87,9 +99,9 @@ def test_adjoint_in_one_block_on_several_grids(tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("prec", ["FP64", "FP32"])
-def test_batches_one_after_the_other(tmp_path, prec):
-    """Batches of two grids, each in the memory that the one before gave back, and
+@pytest.mark.parametrize("prec,times", [("FP64", 1), ("FP32", 1), ("FP64", 64), ("FP32", 64), ("FP64", 65)])
+def test_batches_one_after_the_other(tmp_path, prec, times):
+    """Batches of two grids (`times` of each), each in the memory that the one before gave back, and
     alone: a batch's simulations step as they do alone (maps from global memory
     and from the parameter), in FP64 as the oracle does."""
     precision = getattr(gp, "GP_" + prec)
@@ -106,7 +118,7 @@ def test_batches_one_after_the_other(tmp_path, prec):
             for a, b in zip(ref[mesh][3:], o.get()):
                 assert bits_equal(a, b), mismatch_report(a, b)
     for pair in [(0, 1), (1, 2), (2, 0), (1, 0)]:
-        ms = [ref[MESHES[i]] for i in pair]
+        ms = [ref[MESHES[i]] for i in pair] * times
         b = gp.Batch([m[0] for m in ms], [(m[1], m[2]) for m in ms], precision=precision)
         b.step(7, stats=False)
         for i, m in enumerate(ms):

@@ -52,7 +52,7 @@ def _all():
 
 def _dependent(funcs):
     """the kernels launched by launch_dependent and every device function they reach"""
-    kernels = {n for n, defs in funcs.items() if any("pdl_begin()" in b for _, b in defs)}
+    kernels = {n for n, defs in funcs.items() if any("pdl_begin()" in b or "box_begin<" in b for _, b in defs)}
     seen, todo = set(), set(kernels)
     while todo:
         n = todo.pop()
