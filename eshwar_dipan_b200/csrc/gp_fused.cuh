@@ -1304,7 +1304,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         const int f = tid / (FR + FC), u = tid - f * (FR + FC), reach = 2 - f;
         if (u < FR) {
           const int x = x0 - 2 + u;
-          sm.row[f][u] = (x >= -reach && x < g.mx + reach) ? remap(x, g.mx, D.bc_x[f][0], D.bc_x[f][1]) * g.pitch : -1;
+          sm.row[f][u] = (x >= -reach && x < g.mx + reach) ? remap(x, g.mx, D.bc_x[f][0], D.bc_x[f][1]) : -1;
         } else {
           const int y = y0 - 2 + (u - FR);
           sm.col[f][u - FR] = (y >= -reach && y < g.my + reach) ? remap(y, g.my, D.bc_y[f][0], D.bc_y[f][1]) : -1;
@@ -1320,12 +1320,14 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
 #pragma unroll
         for (int f = 0; f < N + K; f++) v[f] = R(0.0);
         if (r >= 0 && c >= 0) {
+          const R *cell = src + plane_offset(g, r, c);
 #pragma unroll
-          for (int a = 0; a < N; a++) v[a] = ld_step(src + a * g.plane + (r + c));
+          for (int a = 0; a < N; a++) v[a] = ld_step(cell + a * g.plane);
         }
         if (rm >= 0 && cm >= 0) {
+          const R *cell = srcm + plane_offset(g, rm, cm);
 #pragma unroll
-          for (int k = 0; k < K; k++) v[N + k] = ld_step(srcm + k * g.plane + (rm + cm));
+          for (int k = 0; k < K; k++) v[N + k] = ld_step(cell + k * g.plane);
         }
 #pragma unroll
         for (int f = 0; f < N + K; f++) F[f][i][j + CO] = v[f];

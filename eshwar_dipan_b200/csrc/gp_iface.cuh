@@ -60,7 +60,7 @@ struct alignas(128) ItemCommon {
   unsigned long long bar[2];
   int4 ent[2];
   unsigned fm[2][TX];                   /* per tile row: flag bits of the new phi (row_flag_bits) */
-  int row[2][FR], col[2][FC];
+  int row[2][FR], col[2][FC];           /* of phi and mu: the rows and columns that a frame's are copies of, or -1 */
 };
 
 template <typename R, int N, int K, bool ANISO>

@@ -21,19 +21,23 @@ namespace gpd {
 
 /* Offsets of the cells (x-1..x+1, y-1..y+1) of interior cell (x, y) in a
  * field's planes, ghosts through the boundary remap of that field (0 phi,
- * 1 mu): o(u, v) = row[u] + col[v].  Computed once per cell; 32 bits hold
- * any offset inside a plane (a plane of 2^32 FP64 cells is 32 GB). */
+ * 1 mu): o(u, v) = row[u] + col[v].  Computed once per cell.  FP64: 32 bits hold
+ * any offset (two buffers of three planes of 2^32 cells are 206 GB); FP32 planes
+ * may be larger. */
+template <typename R>
 struct Nbr3 {
-  unsigned row[3], col[3];
-  __device__ __forceinline__ unsigned o(int u, int v) const { return row[u] + col[v]; }
+  using off = typename std::conditional<sizeof(R) == 8, unsigned, long long>::type;
+  off row[3];
+  unsigned col[3];
+  __host__ __device__ __forceinline__ off o(int u, int v) const { return row[u] + col[v]; }
 };
 template <typename R>
-__device__ __forceinline__ Nbr3 nbr3(const Consts<R> &D, const Grid &g, int field, int x, int y) {
-  Nbr3 n;
+__host__ __device__ __forceinline__ Nbr3<R> nbr3(const Consts<R> &D, const Grid &g, int field, int x, int y) {
+  Nbr3<R> n;
   const int bx0 = D.bc_x[field][0], bx1 = D.bc_x[field][1], by0 = D.bc_y[field][0], by1 = D.bc_y[field][1];
 #pragma unroll
   for (int u = 0; u < 3; u++) {
-    n.row[u] = (unsigned)remap(x - 1 + u, g.mx, bx0, bx1) * (unsigned)g.pitch;
+    n.row[u] = (typename Nbr3<R>::off)plane_offset(g, remap(x - 1 + u, g.mx, bx0, bx1), 0);
     n.col[u] = (unsigned)remap(y - 1 + u, g.my, by0, by1);
   }
   return n;
@@ -51,7 +55,7 @@ __device__ __forceinline__ T ld_sweep(const T *p) {
  * at interior cell (x, y): its delta-phi into d. */
 template <typename R, int N, bool ANISO, bool STEP>
 __device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *phi, const Grid &g,
-                                           const Nbr3 &np, R (&d)[N]) {
+                                           const Nbr3<R> &np, R (&d)[N]) {
   R S[N][3][3];
 #pragma unroll
   for (int a = 0; a < N; a++)
@@ -119,8 +123,8 @@ __device__ __forceinline__ void sdphi_cell(const Consts<R> &D, const R *phi, con
 template <typename R, int N, int K, bool STEP>
 __device__ __forceinline__ void supd_cell(const Consts<R> &D, const R *phi, const R *mu,
                                           const R (&dph)[N], R (&nph)[N], R *__restrict__ phin, R *__restrict__ mun,
-                                          const Grid &g, const double *tcc, const Nbr3 &np,
-                                          const Nbr3 &nq, int x, int y) {
+                                          const Grid &g, const double *tcc, const Nbr3<R> &np,
+                                          const Nbr3<R> &nq, int x, int y) {
   /* cells: 0 centre, 1 front (x+1), 2 back (x-1), 3 right (y+1), 4 left (y-1) */
   const int cu[5] = {1, 2, 0, 1, 1}, cv[5] = {1, 1, 1, 2, 0};
   R P[5][N], M[5][K], Dv[5][K][K];
@@ -201,7 +205,7 @@ template <typename R, int N, int K, bool ANISO, bool STEP>
 __device__ __forceinline__ void smooth_cell(const Consts<R> &D, const R *phi, const R *mu,
                                             R (&nph)[N], R *__restrict__ phin, R *__restrict__ mun, const Grid &g,
                                             const double *tcc, int x, int y) {
-  const Nbr3 np = nbr3(D, g, 0, x, y), nq = nbr3(D, g, 1, x, y);
+  const Nbr3<R> np = nbr3(D, g, 0, x, y), nq = nbr3(D, g, 1, x, y);
   R d[N];
   sdphi_cell<R, N, ANISO, STEP>(D, phi, g, np, d);
   supd_cell<R, N, K, STEP>(D, phi, mu, d, nph, phin, mun, g, tcc, np, nq, x, y);

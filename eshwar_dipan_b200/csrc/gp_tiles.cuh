@@ -30,6 +30,11 @@ struct Grid {
   int sx0, sx1;          /* rows the progress statistics cover (a slab's own rows; all by default) */
 };
 
+/* offset of a cell in its plane (a plane may hold more than 2^31 cells) */
+__host__ __device__ __forceinline__ long long plane_offset(const Grid &g, int x, int y) {
+  return (long long)x * g.pitch + y;
+}
+
 /* rows moved by one gp_rows_pack / gp_rows_unpack call: item i is row
  * row[i] of state field field[i] */
 constexpr int ROW_ITEMS_MAX = 64;
@@ -45,7 +50,7 @@ __device__ __forceinline__ bool stat_row(const Grid &g, int x) { return x >= g.s
  * (assign_buffer_points_conditions / assign_boundary_points_values,
  * utility_functions.h:471-654): Neumann mirrors about the boundary cell,
  * periodic wraps with period m-1. */
-__device__ __forceinline__ int remap(int v, int m, int tlo, int thi) {
+__host__ __device__ __forceinline__ int remap(int v, int m, int tlo, int thi) {
   int g = v + 3, r = m + 6, src = g;
   if (g < 3) {
     int j = 2 - g;
