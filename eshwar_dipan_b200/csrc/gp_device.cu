@@ -2097,8 +2097,13 @@ int gp_adjoint_replay(gp_ctx *c, long nsteps, double *max_abs_diff, long long *n
   const size_t S = (size_t)(N + K) * g.plane, Sd = (size_t)N * g.dplane;
   const gpd::AdjParams prm = adj_params(b->params[0]);
   AdjBufs m;
-  if (cudaMalloc((void **)&m.seg, 2 * S * 8) != cudaSuccess || cudaMalloc((void **)&m.dphi, Sd * 8) != cudaSuccess)
-    return fail(c, GP_ENOMEM, "gp_adjoint_replay: cudaMalloc failed");
+  m.stream = b->stream;
+  if (cudaMalloc(&m.own, (2 * S + Sd) * 8) != cudaSuccess) {
+    m.own = nullptr;
+    return fail(c, GP_ENOMEM, "gp_adjoint_replay: cudaMalloc of %zu bytes failed", (2 * S + Sd) * 8);
+  }
+  m.seg = (double *)m.own;
+  m.dphi = m.seg + 2 * S;
   double *a = m.seg, *a2 = m.seg + S;
   CK(cudaMemcpyAsync(a, b->state[b->cur], S * 8, cudaMemcpyDeviceToDevice, b->stream));
   for (long s = 0; s < nsteps; s++) {
