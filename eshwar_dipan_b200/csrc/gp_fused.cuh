@@ -1356,7 +1356,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
      * 5-point stencil has no active phase (delta-phi is 0, or the projection's clamp
      * of a negative phi), the others are listed; D; whether the fields are of
      * ordinary size (left-out terms are then +-0) */
-    bool tame = true;
+    bool tame = D.quick_span != 0;
     for (int rt = wid; rt < RR + 1; rt += NWI) {
       const int ri = rt < RR ? rt : lane >> 1, rj = rt < RR ? lane : 32 + (lane & 1);
       const bool in = rt < RR || lane < 2 * RR;
@@ -1371,12 +1371,12 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         for (int a = 0; a < N; a++) {
           p[a] = F[a][i][j + CO];
           /* bitwise, not short-circuit: branches here cost more than the comparisons */
-          tame = tame & (fabs(p[a]) < R(1e18));
+          tame = tame & (fabs(p[a]) < R(PHI_TAME));
           nu = nu | (F[a][i + 1][j + CO] != p[a]) | (F[a][i - 1][j + CO] != p[a]) | (F[a][i][j + 1 + CO] != p[a]) |
                (F[a][i][j - 1 + CO] != p[a]);
         }
 #pragma unroll
-        for (int k = 0; k < K; k++) tame = tame & (fabs(F[N + k][i][j + CO]) < R(1e18));
+        for (int k = 0; k < K; k++) tame = tame & (fabs(F[N + k][i][j + CO]) < R(MU_TAME));
         /* (a constant stencil between phases is listed too, for its anti-trapping weights) */
 #pragma unroll
         for (int a = 0; a < N - 1; a++) nu = nu | ((p[a] != R(0.0)) & (p[a] != R(1.0)));
@@ -1415,6 +1415,17 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         if (lane == 0) b = atomicAdd(&sm.n_test, __popc(m));
         b = __shfl_sync(0xffffffffu, b, 0);
         if (nu) sm.TEST[b + __popc(m & ((1u << lane) - 1u))] = (short)e;
+      }
+    }
+    {
+      /* the phi of the frame around the ring, by warps that had one row above */
+      const int q = tid - (RR + 1 - NWI) * 32;
+      constexpr int TOP = 2 * FC, ALL = TOP + 2 * (FR - 2);
+      if (q >= 0 && q < ALL) {
+        const int i = q < TOP ? (q < FC ? 0 : FR - 1) : 1 + ((q - TOP) >> 1);
+        const int j = q < TOP ? (q < FC ? q : q - FC) : ((q - TOP) & 1) * (FC - 1);
+#pragma unroll
+        for (int a = 0; a < N; a++) tame = tame & (fabs(F[a][i][j + CO]) < R(PHI_TAME));
       }
     }
     tame = __syncthreads_and(ok && tame);
@@ -1556,7 +1567,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
       }
       __syncthreads();
       const int nf = 2 * nact + sm.n_extra;
-      for (int q = tid; q < nf; q += NTI) item_face<R, N, K, ANISO>(D, F, sm, sm.FLIST[q]);
+      for (int q = tid; q < nf; q += NTI) item_face<R, N, K, ANISO>(D, F, sm, sm.FLIST[q], tame);
       __syncthreads();
     }
     {

@@ -30,14 +30,19 @@
  * to 77 us; 268 four-phase ones 58 to 41 us.
  * The arithmetic of each cell is the reference's, in its order (FP64; the FP32
  * form's tiles are in gp_iface32.cuh).  Terms of a
- * phase that is exactly zero over a stencil are left out: each is +-0 added to a
- * sum that starts at +0.
+ * phase that is exactly zero over a stencil, and off-diagonal terms whose constants
+ * are zero, are left out: each is +-0 added to a sum that starts at +0, as long as
+ * its other factors are finite.  That is checked for a whole tile (tame): every phi
+ * of its frame below PHI_TAME and every mu of its ring below MU_TAME, between
+ * spacings of 2^-60 to 2^60, which keeps the eighth powers of the anisotropy and the
+ * products of the free energies finite; a tile that fails takes every term.
  */
 #pragma once
 #include "gp_tiles.cuh"
 
 namespace gpd {
 
+constexpr double PHI_TAME = 16.0, MU_TAME = 1e18;
 constexpr int NTI = NT;                                      /* threads of the step kernels' CTAs */
 constexpr int FR = TX + 4, FC = TY + 4;                      /* staged frame: two-cell halo */
 constexpr int RR = TX + 2, RC = TY + 2, RS = RR * RC;        /* ring region: one-cell halo */
@@ -171,7 +176,8 @@ __device__ __forceinline__ R dwdphi_rt(const CT &D, const R (&ph)[N], R pa, unsi
  * (b,a).  x-faces lie between frame rows i and i+1 at column j, y-faces between
  * columns j and j+1 of row i. */
 template <typename R, int N, int K, bool ANISO, typename CT>
-__device__ __forceinline__ void item_face(const CT &D, ItemFrame<R, N, K> F, ItemSmem<R, N, K, ANISO> &sm, int fidx) {
+__device__ __forceinline__ void item_face(const CT &D, ItemFrame<R, N, K> F, ItemSmem<R, N, K, ANISO> &sm, int fidx,
+                                          bool tame) {
   constexpr int CO = ItemGeom<R>::CO, BW = ItemGeom<R>::BW;
   const bool xface = fidx < IXF;
   const int f = fidx - IXF;
@@ -196,6 +202,7 @@ __device__ __forceinline__ void item_face(const CT &D, ItemFrame<R, N, K> F, Ite
                   (S[along - cross] != R(0.0));
           have = have & any;
         }
+        have = have | !tame;
       }
       if (have) {
 #pragma unroll
@@ -259,7 +266,7 @@ __device__ __forceinline__ void item_lambda(const CT &D, ItemFrame<R, N, K> F, I
     const R *B = &F[b][0][0] + o;
     const R pb = B[0], bxp = B[BW], bxm = B[-BW], byp = B[1], bym = B[-1];
     /* a phase that is zero on the 5-point stencil has no term here */
-    if (N > 2 && ((pb == R(0.0)) & (bxp == R(0.0)) & (bxm == R(0.0)) & (byp == R(0.0)) & (bym == R(0.0)))) continue;
+    if (N > 2 && tame && ((pb == R(0.0)) & (bxp == R(0.0)) & (bxm == R(0.0)) & (byp == R(0.0)) & (bym == R(0.0)))) continue;
     const R gxb = R(0.5) * (divx(bxp - pb, D) + divx(pb - bxm, D)), gyb = div2y(byp - bym, D);
     const R gam = D.gamma[a][b];
     /* face means of the other phase: forward and backward x, right and left y */
@@ -554,6 +561,7 @@ __device__ __forceinline__ void item_commit(const CT &D, ItemFrame<R, N, K> F, c
   if (bulk >= 0) {
     {
       R cn[K];
+      bool ordinary = true;   /* (a current may not be, where a lambda was not) */
 #pragma unroll
       for (int k = 0; k < K; k++) {
         R cm = R(0.0);
@@ -565,6 +573,7 @@ __device__ __forceinline__ void item_commit(const CT &D, ItemFrame<R, N, K> F, c
           cm = c_mu_d<R, K>(D, m, bulk, k, dg);
         }
         cn[k] = cm + D.dt * (divflux[k]) - divjat[k];
+        if (K > 1) ordinary = ordinary & (fabs(cn[k]) < R(MU_TAME));
       }
 #pragma unroll
       for (int k = 0; k < K; k++) {
@@ -573,7 +582,7 @@ __device__ __forceinline__ void item_commit(const CT &D, ItemFrame<R, N, K> F, c
           for (int a = 0; a < N; a++)
             if (a == bulk) nm[k] = MuE<R, K>(D, E[TG ? a : 0], cn, a, k);
         } else {
-          nm[k] = mu_d<R, K>(D, cn, bulk, k, dg);
+          nm[k] = mu_d<R, K>(D, cn, bulk, k, dg && ordinary);
         }
         dmu[k] = (double)nm[k] - (double)m[k];
       }
@@ -595,10 +604,14 @@ __device__ __forceinline__ void item_commit(const CT &D, ItemFrame<R, N, K> F, c
      * allocated but never filled by the reference (taken as 0) and the struct
      * member GRADIENT is never set, so the term is a signed zero */
     R sdc = R(0.0);
+    bool ordinary = tame;
+#pragma unroll
+    for (int a = 0; a < N; a++)
+      if (N > 2) ordinary = ordinary & (fabs(dp[a]) < R(MU_TAME));
 #pragma unroll
     for (int a = 0; a < N; a++) {
       /* a phase the cell neither holds nor gains: h and its terms are +-0 */
-      if (N > 2 && tame && ph[a] == R(0.0) && dp[a] == R(0.0)) continue;
+      if (N > 2 && ordinary && ph[a] == R(0.0) && dp[a] == R(0.0)) continue;
       R sdh = R(0.0);
 #pragma unroll
       for (int b = 0; b < N; b++) sdh += dh<R, N>(ph, a, b) * dp[b];
