@@ -1274,9 +1274,9 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         int *dst = reinterpret_cast<int *>(scp);
         for (int w = tid; w < (int)(sizeof(Consts<R>) / sizeof(int)); w += NTI) dst[w] = __ldg(src + w);
       }
-      if (tid < 2 * (N + K)) {
-        const long long o = st.ext ? *(volatile long long *)(st.ext + (long long)s * (2 * (N + K)) + tid) : 0;
-        sm.ext[tid] = __longlong_as_double(o < 0 ? o ^ 0x7fffffffffffffffLL : o);
+      if (lane < 2 * (N + K)) {
+        const long long o = st.ext ? *(volatile long long *)(st.ext + (long long)s * (2 * (N + K)) + lane) : 0;
+        sm.ext[wid][lane] = __longlong_as_double(o < 0 ? o ^ 0x7fffffffffffffffLL : o);
       }
       if constexpr (SOLO) {
         g = args.sd.g;
@@ -1635,8 +1635,13 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
 #pragma unroll
       for (int k = 0; k < K; k++) outm[k * g.plane] = nm[k];
       oh = one_hot<R, N>(nph);
-      if (st.ext && stat_row(g, x)) item_extremes<R, N, K>(sm.ext, nph, nm, st, s);
+    } else {
+#pragma unroll
+      for (int a = 0; a < N; a++) nph[a] = R(0.0);
+#pragma unroll
+      for (int k = 0; k < K; k++) nm[k] = R(0.0);
     }
+    if (st.ext && stat_row(g, x)) item_extremes<R, N, K>(sm.ext[wid], valid, nph, nm, st, s);
     {
       const unsigned b = row_flag_bits<N>(valid, oh);
       if (lane == 0) sm.fm[cur][wid] = b;
