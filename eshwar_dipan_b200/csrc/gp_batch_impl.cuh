@@ -183,8 +183,8 @@ struct BatchKernels {
     /* on every call: the attribute belongs to the caller's context */
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)item_smem);
     if (e != cudaSuccess) return e;
-    const int most = nsm * item_ctas<double, N, K, A>();
-    k<<<d.ntiles < most ? d.ntiles : most, NTI, item_smem, l.stream>>>(
+    const int most = nsm * item_ctas<double, N, K, A>(), few = (d.ntiles + NOALLOC_TILES - 1) / NOALLOC_TILES;
+    k<<<d.ntiles < most ? d.ntiles : (few > most ? few : most), NTI, item_smem, l.stream>>>(
         *reinterpret_cast<const StepArgs<double, true> *>(l.solo), d, (const double *)l.state, (double *)l.next, l.st);
     return cudaGetLastError();
   }

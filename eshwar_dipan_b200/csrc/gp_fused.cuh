@@ -377,6 +377,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int tri
   return false;
 }
 
+/* eight bytes of global memory into shared memory, asynchronously (n = 0: zeros) */
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, unsigned n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 /* x/dx and y/dy of the bulk kernel: a multiplication by the reciprocal when
  * the spacing is a power of two (MUL, chosen at launch), else the division */
 template <bool MUL, typename R>
@@ -1187,7 +1193,8 @@ __device__ __forceinline__ const Consts<R> &pick_consts(const StepArgs<R, SOLO> 
 
 /* DIRECT: every tile of one simulation on the caller's planes (phi and mu apart,
  * any pitch), without lists, flags, boxes or a progress record: gp_step_noalloc.
- * CTA b takes tiles b, b + grid, ... */
+ * CTA b takes tiles b, b + grid, ..., the next one's frame on its way by cp.async
+ * while one is stepped (planes of any pitch have no tensor map). */
 template <typename R, bool DIRECT>
 struct DirectArgs {};
 template <typename R>
@@ -1258,6 +1265,37 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
   Grid g = {};
   long long off_state = 0;
   const double *tpf = nullptr, *tcc = nullptr;
+  /* DIRECT: the frame of tile t into slot c, every thread its cells */
+  auto fetch = [&](int t, int c) {
+    if constexpr (DIRECT) {
+      const Grid &gd = args.sd.g;
+      const int x0 = t / direct.tiles_x * TX, y0 = (t - t / direct.tiles_x * direct.tiles_x) * TY;
+      const bool inside = x0 >= 2 && x0 + TX + 2 <= gd.mx && y0 >= 2 && y0 + TY + 2 <= gd.my;
+      for (int q = tid; q < FR * FC; q += NTI) {
+        const int i = q / FC, j = q - i * FC;
+        int x = x0 - 2 + i, y = y0 - 2 + j, xm = x, ym = y;
+        unsigned np = 8, nm = 8;
+        if (!inside) {
+          /* the cells after the boundary remap of phi and mu; zeros where no needed
+           * cell lies (phi: [-2, m+1], mu: [-1, m]) */
+          const bool need = x < gd.mx + 2 && y < gd.my + 2;
+          const bool needm = x >= -1 && x < gd.mx + 1 && y >= -1 && y < gd.my + 1;
+          np = need ? 8 : 0;
+          nm = needm ? 8 : 0;
+          xm = needm ? remap(x, gd.mx, D.bc_x[1][0], D.bc_x[1][1]) : 0;
+          ym = needm ? remap(y, gd.my, D.bc_y[1][0], D.bc_y[1][1]) : 0;
+          x = need ? remap(x, gd.mx, D.bc_x[0][0], D.bc_x[0][1]) : 0;
+          y = need ? remap(y, gd.my, D.bc_y[0][0], D.bc_y[0][1]) : 0;
+        }
+        const R *cell = state + plane_offset(gd, x, y), *cellm = direct.mu + plane_offset(gd, xm, ym);
+#pragma unroll
+        for (int a = 0; a < N; a++) cp_async8(&sm.F[c][a][i][j + CO], cell + a * gd.plane, np);
+#pragma unroll
+        for (int k = 0; k < K; k++) cp_async8(&sm.F[c][N + k][i][j + CO], cellm + k * gd.plane, nm);
+      }
+    }
+  };
+  if (DIRECT) fetch(first, 0);
   __syncthreads();
 #pragma unroll 1
   for (int cur = 0;; cur ^= 1) {
@@ -1294,7 +1332,11 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     }
     R(&F)[N + K][FR][IG::BW] = sm.F[cur];
     bool ok = true;
-    if (en.w) {
+    if constexpr (DIRECT) {
+      cp_async_wait();
+      __syncthreads();   /* everyone's cells of this frame; the other slot was last read a tile ago */
+      if (nxt < nlist) fetch(nxt, cur ^ 1);
+    } else if (en.w) {
       ok = mbar_wait(smem_addr(&sm.bar[cur]), (parity >> cur) & 1u, st.mbar_tries);
       parity ^= 1u << cur;
     } else {
@@ -1312,7 +1354,6 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
       }
       __syncthreads();
       const R *src = state + off_state, *srcm = src + N * g.plane;
-      if constexpr (DIRECT) srcm = direct.mu;
       for (int q = tid; q < FR * FC; q += NTI) {
         const int i = q / FC, j = q - i * FC;
         const int r = sm.row[0][i], c = sm.col[0][j], rm = sm.row[1][i], cm = sm.col[1][j];
@@ -1451,6 +1492,11 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     int4 nent = make_int4(-1, 0, 0, 0);
     if (tid == 0 && nxt < nlist) nent = entry(nxt);
 
+    /* a tile without a listed cell has no active phase and no current */
+    const bool listed = sm.n_test != 0;
+    if (!listed) {
+      if (tid == 0) issue(nent, cur ^ 1);   /* the other slot was last read a tile ago */
+    } else {
     /* ---- listed cells: active phases */
     const int ntest = sm.n_test;
     for (int q0 = 32 * wid; q0 < ntest; q0 += NTI) {
@@ -1595,6 +1641,12 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     for (int q = tid; q < nact; q += NTI) item_dphi<R, N, K, ANISO>(D, F, sm, sm.LIST[q]);
     __syncthreads();
     if (tid == 0) sm.n_test = sm.n_act = sm.n_task = sm.n_extra = sm.n_j = 0;   /* for the next tile */
+    if (nj > 0) {
+      for (int q = tid; q < nj; q += NTI)
+        item_current<R, N, K, ANISO, TG>(D, F, sm, sm.JLIST[q], y0, g.my, dg, tcc);
+      __syncthreads();
+    }
+    }
     if (st.dphi_out) {
       /* the adjoint's tape: the delta-phi of the tile and of its ring cells
        * (the domain's ring included), as the reverse sweep reads it */
@@ -1607,11 +1659,6 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
         }
       }
     }
-    if (nj > 0) {
-      for (int q = tid; q < nj; q += NTI)
-        item_current<R, N, K, ANISO, TG>(D, F, sm, sm.JLIST[q], y0, g.my, dg, tcc);
-      __syncthreads();
-    }
 
     /* ---- per cell: mu update, phi commit */
     if (valid) {
@@ -1623,7 +1670,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
       }
 #pragma unroll
       for (int k = 0; k < K; k++) m[k] = F[N + k][tx + 2][ty + 2 + CO];
-      item_commit<R, N, K, ANISO, TG>(D, F, sm, tx, ty, x, y, tame, dg, ph, dp, m, nph, nm, dmu, Tc);
+      item_commit<R, N, K, ANISO, TG>(D, F, sm, tx, ty, x, y, tame, dg, listed, ph, dp, m, nph, nm, dmu, Tc);
     }
     }
     int oh = -1;
@@ -1703,7 +1750,17 @@ __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kf_general(
   step_finish(ctr, ndone, 1);
 }
 
-/* One step of one simulation on the caller's planes (gp_step_noalloc). */
+/* One step of one simulation on the caller's planes (gp_step_noalloc).  On a grid of
+ * many tiles, most of them without an interface, the latency of a tile bounds it:
+ * hence the next frame on its way and the short path of a tile without a listed cell.
+ * A CTA takes two tiles where there are more tiles than resident CTAs, so that a free
+ * SM takes the next two: with all tiles dealt out at the start the CTA with the most
+ * interface tiles ended late (1000x300: 45 us; two tiles 29, one tile 31), and one
+ * tile per CTA has no next frame (1440x1400, one seed: 88 us, two tiles 78).  Binary
+ * anisotropic 1440x1400 with 20 seeds: two passes of small CTAs over a delta-phi array
+ * 111 us, one launch without all this 160 us, with it 93 us; three-phase ternary
+ * 1160x1130: 161, 125 and 85 us. */
+constexpr int NOALLOC_TILES = 2;
 template <typename R, int N, int K, bool ANISO, bool MUL>
 __global__ void __launch_bounds__(NTI, item_ctas<R, N, K, ANISO>()) kn_step(
     const __grid_constant__ StepArgs<R, true> args, const __grid_constant__ DirectArgs<R, true> direct,

@@ -512,16 +512,17 @@ __device__ __forceinline__ void item_current(const CT &D, ItemFrame<R, N, K> F, 
  * (calculate_divergence_concentration.h:24-140): divergences of the diffusion
  * flux and the current, then the bulk branch (mu = Mu_a(c_a(mu) + dc)) or the
  * interface branch (dmu = (dc/dmu)^-1 dc, inverted in FP64), then phi +=
- * delta-phi.  x, y: the cell's interior coordinates. */
+ * delta-phi.  x, y: the cell's interior coordinates; currents: some face of the tile
+ * may carry one. */
 template <typename R, int N, int K, bool ANISO, bool TG, typename CT>
 __device__ __forceinline__ void item_commit(const CT &D, ItemFrame<R, N, K> F, const ItemSmem<R, N, K, ANISO> &sm,
-                                            int tx, int ty, int x, int y, bool tame, bool dg, const R *ph, const R *dp,
-                                            const R *m, R *nph, R *nm, double *dmu, double Tc) {
+                                            int tx, int ty, int x, int y, bool tame, bool dg, bool currents,
+                                            const R *ph, const R *dp, const R *m, R *nph, R *nm, double *dmu, double Tc) {
   constexpr int CO = ItemGeom<R>::CO;
   const R cst = D.obstacle ? D.jat_obst : D.jat_well;
   const int c = RI(tx + 1, ty + 1);
-  const bool hxf = (sm.JW[tx + 1] >> ty) & 1u, hxb = (sm.JW[tx] >> ty) & 1u;
-  const bool hyr = (sm.JW[TX + 1 + tx] >> (ty + 1)) & 1u, hyl = (sm.JW[TX + 1 + tx] >> ty) & 1u;
+  const bool hxf = currents && ((sm.JW[tx + 1] >> ty) & 1u), hxb = currents && ((sm.JW[tx] >> ty) & 1u);
+  const bool hyr = currents && ((sm.JW[TX + 1 + tx] >> (ty + 1)) & 1u), hyl = currents && ((sm.JW[TX + 1 + tx] >> ty) & 1u);
   const int xf = (tx + 1) * TY + ty, xb = tx * TY + ty, yr = JXF + tx * (TY + 1) + ty + 1, yl = yr - 1;
   R divflux[K], divjat[K];
 #pragma unroll
