@@ -294,13 +294,12 @@ struct gp_batch {
   std::vector<char> solo;       /* a batch of one: its StepArgs (the step kernels' parameter) */
   bool mul;                     /* every simulation's dx and dy are powers of two (or FP32) */
   bool diag;                    /* off-diagonal D, c_mu, A all zero and no E is -0, in every simulation */
-  int mbar_tries;               /* kf_bulk's polls of a box barrier before it reports an error */
   LaunchShape shape;            /* how a step is launched (tuned on the first graph chunks) */
   LaunchShape cand[6];          /* the candidates */
   float cand_ms[6];
   int ncand, tune_next;         /* tuning is over when tune_next == ncand */
   ShapeKey key;
-  unsigned tma_extra;           /* 0; a test sets more (GP_TEST_TMA_SHORTFALL) to make the boxes never complete */
+  unsigned tma_extra[gpd::MAP_KINDS];   /* 0; a test sets more (GP_TEST_TMA_SHORTFALL) to make the boxes never complete */
   int ntiles;                   /* TX x TY tiles over all simulations */
   cudaStream_t stream;
   gpd::SimDesc *d_desc;
@@ -367,8 +366,10 @@ static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   st.partials = b->partials;
   st.want_sums = want_sums;
   st.round_step = (const unsigned *)(b->counters + gpd::CTR_STEP);
-  st.mbar_tries = b->mbar_tries;
-  st.tma_extra = b->tma_extra;
+  for (int k = 0; k < gpd::MAP_KINDS; k++) {
+    st.tma_extra[k] = b->tma_extra[k];
+    st.mbar_tries[k] = b->tma_extra[k] ? 256 : gpd::MBAR_TRIES;
+  }
   st.diag = b->diag ? 1 : 0;
   st.dphi_out = b->dphi_out;
   st.bch_max = b->shape.bch_max;
@@ -1077,13 +1078,14 @@ int gp_batch_create(gp_batch **out, int nsims, const gp_params *params, const do
     if (b->elem == 8 && !(pow2(b->derived[s].dx) && pow2(b->derived[s].dy))) b->mul = false;
   b->diag = true;
   for (int s = 0; s < nsims; s++) b->diag = b->diag && diagonal(b->derived[s]);
-  /* the give-up path of kf_bulk's barrier waits, exercised by a test: the
-   * barriers expect more bytes than a box brings, and the polls are few */
-  b->mbar_tries = gpd::MBAR_TRIES;
-  b->tma_extra = 0;
-  if (const char *v = getenv("GP_TEST_TMA_SHORTFALL")) {
-    b->tma_extra = (unsigned)std::max(0, std::min(4096, atoi(v)));
-    if (b->tma_extra) b->mbar_tries = 256;
+  /* the give-up paths of the box waits, exercised by a test: the barriers expect
+   * more bytes than a box brings, and the polls are few (GP_TEST_TMA_KIND: of the
+   * bulk or of the interface tiles' boxes alone) */
+  {
+    const char *v = getenv("GP_TEST_TMA_SHORTFALL"), *kind = getenv("GP_TEST_TMA_KIND");
+    const unsigned extra = v ? (unsigned)std::max(0, std::min(4096, atoi(v))) : 0;
+    b->tma_extra[gpd::MAP_MU] = kind && strcmp(kind, "interface") == 0 ? 0 : extra;
+    b->tma_extra[gpd::MAP_ALL] = kind && strcmp(kind, "bulk") == 0 ? 0 : extra;
   }
   b->tgrad = false;
   b->shift = false;

@@ -676,7 +676,7 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
     if (lane == 0) {
       ws.meta[b] = en;
       const unsigned bar = smem_addr(&ws.bar[b]);
-      mbar_expect_tx(bar, G::BOX_BYTES + st.tma_extra);
+      mbar_expect_tx(bar, G::BOX_BYTES + st.tma_extra[MAP_MU]);
       tma_load_3d(smem_addr(&ws.st[b]), box_map(maps, tmaps, en.s, buf, MAP_MU, ready), en.y0 - 1 - CO, en.x0 - 1, 0, bar);
     }
   };
@@ -732,11 +732,11 @@ __device__ __noinline__ void bulk_tiles(const SimDesc *__restrict__ sims, const 
       }
     }
     const int b = ci % NST;
-    if (!mbar_wait(smem_addr(&ws.bar[b]), (ci / NST) & 1, st.mbar_tries)) {
+    if (!mbar_wait(smem_addr(&ws.bar[b]), (ci / NST) & 1, st.mbar_tries[MAP_MU])) {
       /* bytes missing: record it, wait (bounded) for the other boxes in
        * flight, step nothing more */
       if (lane == 0) atomicExch(ctr + CTR_ERR, 1);
-      for (int q = ci + 1; q < qi; q++) mbar_wait(smem_addr(&ws.bar[q % NST]), (q / NST) & 1, st.mbar_tries);
+      for (int q = ci + 1; q < qi; q++) mbar_wait(smem_addr(&ws.bar[q % NST]), (q / NST) & 1, st.mbar_tries[MAP_MU]);
       break;
     }
     ci++;
@@ -1244,7 +1244,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
     sm.ent[c] = en;
     if (!DIRECT && en.x >= 0 && en.w) {
       const unsigned bar = smem_addr(&sm.bar[c]);
-      mbar_expect_tx(bar, BOX_BYTES + st.tma_extra);
+      mbar_expect_tx(bar, BOX_BYTES + st.tma_extra[MAP_ALL]);
       tma_load_3d(smem_addr(&sm.F[c]), box_map(maps, tmaps, en.y, buf, MAP_ALL, ready),
                   (en.z & 0xffff) * TY - 2 - CO, (en.z >> 16) * TX - 2, 0, bar);
     }
@@ -1337,7 +1337,7 @@ __device__ __forceinline__ void general_tiles(const StepArgs<R, SOLO> &args, con
       __syncthreads();   /* everyone's cells of this frame; the other slot was last read a tile ago */
       if (nxt < nlist) fetch(nxt, cur ^ 1);
     } else if (en.w) {
-      ok = mbar_wait(smem_addr(&sm.bar[cur]), (parity >> cur) & 1u, st.mbar_tries);
+      ok = mbar_wait(smem_addr(&sm.bar[cur]), (parity >> cur) & 1u, st.mbar_tries[MAP_ALL]);
       parity ^= 1u << cur;
     } else {
       /* rows and columns of the frame after the boundary remap of phi and mu;

@@ -175,14 +175,15 @@ struct StatBufs {
   double *partials;    /* [tiles][2N+2K+1] sums when want_sums */
   int want_sums;
   const unsigned *round_step;  /* FP32 form: device step counter keying the rounding stream */
-  int mbar_tries;      /* polls of a TMA box's barrier before kf_bulk gives up (MBAR_TRIES) */
+  int mbar_tries[2];   /* polls of such a box's barrier before the kernel gives up (MBAR_TRIES) */
   int bch_max, bch_div;  /* bulk chunks: at most bch_max (<= 16) entries, left / (bch_div * warps) */
   int mixed;           /* kf_step: odd CTAs take bulk tiles first, then interface tiles */
   const double *trows; /* non-isothermal simulations: per simulation the temperature of each ghosted column y
                           as the phase-field pass reads it, then as the concentration pass reads it */
   int sweep;           /* kf_bulk: a smoothing sweep's bulk tiles (no step is counted) */
   int diag;            /* every phase's off-diagonal D, c_mu and A are zero and no E is -0 */
-  unsigned tma_extra;  /* bytes a box's barrier expects beyond the box: 0, or more to test the give-up path */
+  unsigned tma_extra[2];  /* bytes that the barrier of a bulk (MAP_MU) and of an interface tile's (MAP_ALL) box expects
+                             beyond it: 0, or more to test the give-up paths */
   double *dphi_out;    /* NULL, or (a batch of one) the step's delta-phi of every interface tile and its ring in
                           the delta-phi layout (Grid dpitch/dplane); cells no interface tile covers are left as
                           they are (their delta-phi is +0.0) */
