@@ -1,5 +1,5 @@
 /*
- * gp_fused.cuh -- the time step as two kernels over classified tiles.
+ * gp_fused.cuh -- the time step as kernels over classified tiles.
  *
  * Every TX x TY tile of every simulation carries a phase flag per state
  * buffer: p >= 0 when each of its cells holds exactly the one-hot phi of phase
@@ -233,12 +233,12 @@ __device__ __forceinline__ int bulk_phase(const ClassifySim &g, const TileFlags 
 /* ------------------------------------------------------------------ */
 
 /* Work-list counters of a batch: [0] interface tiles listed by kf_classify,
- * [1] interface entries taken beyond the CTAs' first, [2] CTAs of kf_bulk and kf_general
+ * [1] interface entries taken beyond the CTAs' first, [2] CTAs of the step's kernels
  * finished, [3] step number (keys the FP32 rounding stream), [4] bulk tiles
- * listed, [5] error flag (a TMA box of kf_bulk did not arrive; the host reads
- * and clears it).  The last CTA of the two kernels resets [0..2] and [4] and
- * advances [3], so a step is exactly the three launches kf_classify, then
- * kf_bulk and kf_general (in either order or side by side). */
+ * listed, [5] error flag (a TMA box did not arrive; the host reads and clears it),
+ * [6] bulk entries taken.  A step is kf_classify, then kf_step or kf_bulk and
+ * kf_general; the last CTA after kf_classify resets [0..2], [4] and [6] and
+ * advances [3]. */
 enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR_ERR = 5, CTR_BHEAD = 6,
        CTR_COUNT = 8 };
 

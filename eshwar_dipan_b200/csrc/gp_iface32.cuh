@@ -96,10 +96,9 @@ __device__ __forceinline__ void ring_face_terms(const CT &D, ItemFrame<R, N, K> 
 /* delta-phi of one ring cell (ring coordinates ri, rj; its phi at P row ri+1,
  * column rj+1) from the staged tile: calculate_divergence_phasefield_2D
  * (calculate_divergence_phasefield.h:4-62).
- * Not inlined: as a call of its own it gets its own register allocation, and
- * the interface tiles spill far less under the 128-register cap of two CTAs
- * per SM (FP64 ternary 3-phase: 732 bytes of spill stores inlined, about 200
- * not; FP32: none), which made whole steps 3-8 % faster. */
+ * Not inlined: as a call of its own it gets its own register allocation. Under
+ * the 128-register cap of two CTAs per SM it spills nothing and the tile's code
+ * around it at most 120 bytes. */
 template <typename R, int N, int K, bool ANISO, typename CT>
 __device__ __noinline__ void ring_dphi(const CT &D, ItemFrame<R, N, K> F, const ItemSmem32<R, N, K> &sm, int ri, int rj,
                                           unsigned mask, R *d, double Tpf) {
@@ -259,6 +258,105 @@ __device__ __noinline__ void ring_dphi(const CT &D, ItemFrame<R, N, K> F, const 
 #pragma unroll
   for (int a = 0; a < N; a++) d[a] = act[a] ? D.dt * (lam[a] - sl) / (tau * D.eps) : R(0.0);
   project<R, N>(ph, act, d);
+}
+
+/* FP32 commit of a pure-phase cell: mu += muc_a * dc in FP64, phi += dphi,
+ * both rounded stochastically. */
+template <typename R, int N, int K>
+__device__ __forceinline__ void bulk_commit_f32(const Consts<R> &D, int a, const R *dc, const R *ph, const R *dp,
+                                                const R *m, R *nph, R *nm, double *dmu, unsigned key) {
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    double s = 0.0;
+#pragma unroll
+    for (int l = 0; l < K; l++) s += D.muc64[a][k][l] * (double)dc[l];
+    dmu[k] = s;
+    nm[k] = (R)round_stochastic((double)m[k] + s, key, N + k);
+  }
+#pragma unroll
+  for (int a2 = 0; a2 < N; a2++) nph[a2] = (R)round_stochastic((double)ph[a2] + (double)dp[a2], key, a2);
+}
+
+/* mu update and phi commit of one tile cell from the tile's face fluxes
+ * (calculate_divergence_concentration.h:24-140): divergences, then the bulk
+ * branch (mu += dmu/dc dc, bulk_commit_f32) or the interface branch (dmu = (dc/dmu)^-1 dc,
+ * inverted in FP64), then phi += delta-phi, all rounded stochastically.  i, j: the
+ * cell's position in the one-cell-halo tile layout; x, y: its interior coordinates. */
+template <typename R, int N, int K, typename CT>
+__device__ __forceinline__ void commit_cell(const CT &D, const R (&FX)[K][K][NXF], const R (&FY)[K][K][NYF],
+                                            const R (&JX)[K][NXF], const R (&JY)[K][NYF], const R (&CM)[N][K][SS],
+                                            const R (&H)[N][SS], int i, int j, int x, int y, const R *ph,
+                                            const R *dp, const R *m, R *nph, R *nm, double *dmu,
+                                            const StatBufs &st) {
+  const R cst = D.obstacle ? D.jat_obst : D.jat_well;
+  const int c = LI(i, j);
+  R divflux[K], divjat[K];
+  const int xf = i * TY + (j - 1), xb = (i - 1) * TY + (j - 1);
+  const int yr = (i - 1) * (TY + 1) + j, yl = (i - 1) * (TY + 1) + (j - 1);
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    divflux[k] = R(0.0);
+#pragma unroll
+    for (int l = 0; l < K; l++) {
+      divflux[k] += divx(FX[k][l][xf] - FX[k][l][xb], D);
+      divflux[k] += divy(FY[k][l][yr] - FY[k][l][yl], D);
+    }
+    divjat[k] = divx((JX[k][xf] - JX[k][xb]) * cst, D);
+    divjat[k] += divy((JY[k][yr] - JY[k][yl]) * cst, D);
+  }
+  int bulk = -1;
+#pragma unroll
+  for (int a = 0; a < N; a++)
+    if (bulk < 0 && ph[a] == R(1.0)) bulk = a;
+  if (bulk >= 0) {
+    R cn[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) cn[k] = D.dt * (divflux[k]) - divjat[k];
+    bulk_commit_f32<R, N, K>(D, bulk, cn, ph, dp, m, nph, nm, dmu, round_key(ld_step(st.round_step), x, y));
+  } else {
+    /* sum_a c_a(mu) sum_b dh_a/dphi_b dphi_b (calculate_divergence_concentration.h:23-31) */
+    R sum[K];
+    double dc[K], dcdmu[K][K];
+#pragma unroll
+    for (int k = 0; k < K; k++) sum[k] = R(0.0);
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      R sdh = R(0.0);
+#pragma unroll
+      for (int b = 0; b < N; b++) sdh += dh<R, N>(ph, a, b) * dp[b];
+#pragma unroll
+      for (int k = 0; k < K; k++) sum[k] += CM[a][k][c] * sdh;
+    }
+    /* non-isothermal (calculate_divergence_concentration.h:85): minus
+     * sum_a dcbdT_phase h_a * dt * (-GRADIENT * velocity); dcbdT_phase is
+     * allocated but never filled by the reference (taken as 0) and the struct
+     * member GRADIENT is never set, so the term is a signed zero */
+    R sdc = R(0.0);
+    if (D.tgrad) {
+#pragma unroll
+      for (int a = 0; a < N; a++) sdc += R(0.0) * H[a][c];
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      if (D.tgrad) dc[k] = (double)(D.dt * (divflux[k]) - divjat[k] - sum[k] - sdc * D.dt * (R(-0.0) * (R)D.tg_vel));
+      else dc[k] = (double)(D.dt * (divflux[k]) - divjat[k] - sum[k]);
+#pragma unroll
+      for (int l = 0; l < K; l++) {
+        dcdmu[k][l] = 0.0;
+#pragma unroll
+        for (int a = 0; a < N; a++) dcdmu[k][l] += D.cmu64[a][k][l] * (double)H[a][c];
+      }
+    }
+    double m64[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) m64[k] = (double)m[k];
+    solve_dmu<R, K>(D, dcdmu, dc, m64, dmu);
+    const unsigned key = round_key(ld_step(st.round_step), x, y);
+#pragma unroll
+    for (int k = 0; k < K; k++) nm[k] = round_stochastic(m64[k], key, N + k);
+#pragma unroll
+    for (int a = 0; a < N; a++) nph[a] = round_stochastic((double)ph[a] + (double)dp[a], key, a);
+  }
 }
 
 /* One staged interface tile (cells (x0+tx, y0+ty)): delta-phi on the tile and its
@@ -459,7 +557,7 @@ __device__ __forceinline__ void tile32(const CT &D, const Grid &g, ItemFrame<R, 
 #pragma unroll
     for (int k = 0; k < K; k++) m[k] = MR(k, c);
     commit_cell<R, N, K>(D, sm.w.u.FX, sm.w.u.FY, sm.w.u.JX, sm.w.u.JY, sm.w.u.CM, sm.w.u.H, i, j, x, y, ph, dp, m,
-                         nph, nm, dmu, st, D.tgrad ? ld_step(tcc + y + 3) : 0.0);
+                         nph, nm, dmu, st);
   }
 #undef PRIJ
 #undef PR

@@ -223,37 +223,6 @@ __device__ __forceinline__ float round_stochastic(double v, unsigned key, int fi
   return fabs(rem) > u * fabs(span) ? hi : lo;
 }
 
-/* a + b rounded to float stochastically without leaving float: TwoSum gives
- * the round-to-nearest sum s and the exact remainder e (s + e = a + b); the
- * neighbour t of s on the side of e is taken with probability |e| / |t - s|,
- * decided by the 16-bit uniform r16 (the probability is exact to 2^-16). */
-__device__ __forceinline__ float add_stochastic(float a, float b, unsigned r16) {
-  const float s = a + b;
-  const float bb = s - a;
-  const float e = (a - (s - bb)) + (b - bb);
-  if (e == 0.0f) return s;
-  const float t = nextafterf(s, e > 0.0f ? INFINITY : -INFINITY);
-  const float u = (float)r16 * (1.0f / 65536.0f);
-  return fabsf(e) > u * fabsf(t - s) ? t : s;
-}
-
-/* FP32 commit of a pure-phase cell: mu += muc_a * dc in FP64, phi += dphi,
- * both rounded stochastically. */
-template <typename R, int N, int K>
-__device__ __forceinline__ void bulk_commit_f32(const Consts<R> &D, int a, const R *dc, const R *ph, const R *dp,
-                                                const R *m, R *nph, R *nm, double *dmu, unsigned key) {
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double s = 0.0;
-#pragma unroll
-    for (int l = 0; l < K; l++) s += D.muc64[a][k][l] * (double)dc[l];
-    dmu[k] = s;
-    nm[k] = (R)round_stochastic((double)m[k] + s, key, N + k);
-  }
-#pragma unroll
-  for (int a2 = 0; a2 < N; a2++) nph[a2] = (R)round_stochastic((double)ph[a2] + (double)dp[a2], key, a2);
-}
-
 /* dmu = (dc/dmu)^-1 dc in FP64 by the simulation's inversion mode, and mu + dmu
  * into m64 (calculate_divergence_concentration.h:96-140) */
 template <typename R, int K, typename CT>
@@ -299,116 +268,6 @@ __device__ __forceinline__ void solve_dmu(const CT &D, double (&dcdmu)[K][K], co
     }
 #pragma unroll
     for (int k = 0; k < K; k++) m64[k] = dmu[k] + m64[k];
-  }
-}
-
-/* mu update and phi commit of one tile cell from the tile's face fluxes
- * (calculate_divergence_concentration.h:24-140): divergences, then the bulk
- * branch (mu = Mu_a(c_a(mu) + dc)) or the interface branch (dmu = (dc/dmu)^-1 dc,
- * inverted in FP64), then phi += delta-phi.  i, j: the cell's position in the
- * one-cell-halo tile layout; x, y: its interior coordinates. */
-template <typename R, int N, int K, typename CT>
-__device__ __forceinline__ void commit_cell(const CT &D, const R (&FX)[K][K][NXF], const R (&FY)[K][K][NYF],
-                                            const R (&JX)[K][NXF], const R (&JY)[K][NYF], const R (&CM)[N][K][SS],
-                                            const R (&H)[N][SS], int i, int j, int x, int y, const R *ph,
-                                            const R *dp, const R *m, R *nph, R *nm, double *dmu,
-                                            const StatBufs &st, double Tc = 0.0) {
-  const R cst = D.obstacle ? D.jat_obst : D.jat_well;
-  const int c = LI(i, j);
-  R divflux[K], divjat[K];
-  const int xf = i * TY + (j - 1), xb = (i - 1) * TY + (j - 1);
-  const int yr = (i - 1) * (TY + 1) + j, yl = (i - 1) * (TY + 1) + (j - 1);
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    divflux[k] = R(0.0);
-#pragma unroll
-    for (int l = 0; l < K; l++) {
-      divflux[k] += divx(FX[k][l][xf] - FX[k][l][xb], D);
-      divflux[k] += divy(FY[k][l][yr] - FY[k][l][yl], D);
-    }
-    divjat[k] = divx((JX[k][xf] - JX[k][xb]) * cst, D);
-    divjat[k] += divy((JY[k][yr] - JY[k][yl]) * cst, D);
-  }
-  int bulk = -1;
-#pragma unroll
-  for (int a = 0; a < N; a++)
-    if (bulk < 0 && ph[a] == R(1.0)) bulk = a;
-  if (bulk >= 0 && sizeof(R) == 4) {
-    R cn[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) cn[k] = D.dt * (divflux[k]) - divjat[k];
-    bulk_commit_f32<R, N, K>(D, bulk, cn, ph, dp, m, nph, nm, dmu, round_key(ld_step(st.round_step), x, y));
-  } else if (bulk >= 0) {
-    R cn[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) cn[k] = CM[bulk][k][c] + D.dt * (divflux[k]) - divjat[k];
-    if (D.tgrad) {
-      R E[N][K];
-      e_at<R, N, K>(D, Tc, E);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        nm[k] = MuE<R, K>(D, E[bulk], cn, bulk, k);
-        dmu[k] = (double)nm[k] - (double)m[k];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        nm[k] = Mu<R, K>(D, cn, bulk, k);
-        dmu[k] = (double)nm[k] - (double)m[k];
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < N; a++) nph[a] = ph[a] + dp[a];
-  } else {
-    /* sum_a c_a(mu) sum_b dh_a/dphi_b dphi_b (calculate_divergence_concentration.h:23-31) */
-    R sum[K];
-    double dc[K], dcdmu[K][K];
-#pragma unroll
-    for (int k = 0; k < K; k++) sum[k] = R(0.0);
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      R sdh = R(0.0);
-#pragma unroll
-      for (int b = 0; b < N; b++) sdh += dh<R, N>(ph, a, b) * dp[b];
-#pragma unroll
-      for (int k = 0; k < K; k++) sum[k] += CM[a][k][c] * sdh;
-    }
-    /* non-isothermal (calculate_divergence_concentration.h:85): minus
-     * sum_a dcbdT_phase h_a * dt * (-GRADIENT * velocity); dcbdT_phase is
-     * allocated but never filled by the reference (taken as 0) and the struct
-     * member GRADIENT is never set, so the term is a signed zero */
-    R sdc = R(0.0);
-    if (D.tgrad) {
-#pragma unroll
-      for (int a = 0; a < N; a++) sdc += R(0.0) * H[a][c];
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      if (D.tgrad) dc[k] = (double)(D.dt * (divflux[k]) - divjat[k] - sum[k] - sdc * D.dt * (R(-0.0) * (R)D.tg_vel));
-      else dc[k] = (double)(D.dt * (divflux[k]) - divjat[k] - sum[k]);
-#pragma unroll
-      for (int l = 0; l < K; l++) {
-        dcdmu[k][l] = 0.0;
-#pragma unroll
-        for (int a = 0; a < N; a++) dcdmu[k][l] += D.cmu64[a][k][l] * (double)H[a][c];
-      }
-    }
-    double m64[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) m64[k] = (double)m[k];
-    solve_dmu<R, K>(D, dcdmu, dc, m64, dmu);
-    if constexpr (sizeof(R) == 8) {
-#pragma unroll
-      for (int k = 0; k < K; k++) nm[k] = (R)m64[k];
-#pragma unroll
-      for (int a = 0; a < N; a++) nph[a] = ph[a] + dp[a];
-    } else {
-      const unsigned key = round_key(ld_step(st.round_step), x, y);
-#pragma unroll
-      for (int k = 0; k < K; k++) nm[k] = round_stochastic(m64[k], key, N + k);
-#pragma unroll
-      for (int a = 0; a < N; a++) nph[a] = round_stochastic((double)ph[a] + (double)dp[a], key, a);
-    }
   }
 }
 
