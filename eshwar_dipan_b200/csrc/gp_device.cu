@@ -387,6 +387,7 @@ static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   l.blist = b->blist;
   l.glist = b->glist;
   l.maps.nsims = b->nsims;
+  l.maps.ahead = gpd::box_fence_ahead(b->nsims, b->ntiles);
   if (b->nsims == 1)
     memcpy(l.maps.m, b->redir_in ? b->redir_map : b->hmaps.data() + in * gpd::MAP_KINDS, sizeof l.maps.m);
   l.tmaps = b->tmaps;

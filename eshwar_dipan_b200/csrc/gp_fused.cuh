@@ -406,17 +406,21 @@ struct alignas(64) TensorMapSlot {
 struct BoxMaps {
   TensorMapSlot m[MAP_KINDS];
   int nsims;
+  int ahead;   /* a batch of several: every block fences all maps before its wait */
 };
 
 /* The copy unit keeps descriptors it has read; one in global memory may be an older
  * one's from the same address until a block has fenced it.  The host writes the maps
- * once, before any step, so in a batch of at most BOX_FENCE_AHEAD simulations every
- * block fences all of them ahead of its wait, while the kernel before finishes; in a
- * larger one a thread fences a map when it moves to its simulation.  Step times,
- * ahead / at each move: 24 simulations of 128^2 to 1024^2 82 / 89 us, 64 of 256^2 50
- * / 54 us, 256 of 256^2 148 / 148 us, 256 of 128^2 110 / 103 us, 1024 of 64^2 443 /
- * 380 us (FP32; FP64 alike). */
-constexpr int BOX_FENCE_AHEAD = 128;
+ * once, before any step.  So every block may fence all of them ahead of its wait,
+ * while the kernel before finishes, which costs by the simulations; or a thread fences
+ * a map when it moves to its simulation, which costs by the tiles.  Step times, ahead /
+ * at each move: 24 simulations of 128^2 to 1024^2 82 / 89 us, 64 of 256^2 50 / 54 us,
+ * 256 of 128^2 to 1024^2 262 / 265 us, 256 of 256^2 148 / 148 us, 256 of 128^2 110 / 103 us,
+ * 1024 of 64^2 443 / 380 us (FP32; FP64 alike): ahead from as many tiles as the
+ * simulations squared (box_fence_ahead). */
+__host__ __device__ __forceinline__ bool box_fence_ahead(long long nsims, long long ntiles) {
+  return nsims > 1 && ntiles >= nsims * nsims;
+}
 __device__ __forceinline__ void box_fence(const TensorMapSlot *m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
 }
@@ -425,10 +429,8 @@ __device__ __forceinline__ void box_fence(const TensorMapSlot *m) {
 template <unsigned KINDS, bool SOLO>
 __device__ __forceinline__ void box_begin(const BoxMaps &maps, const TensorMapSlot *tmaps, int buf) {
   pdl_launch();
-  if (!SOLO && maps.nsims > 1 && maps.nsims <= BOX_FENCE_AHEAD) {
-    static_assert(BOX_FENCE_AHEAD <= NTI, "a thread per simulation");
-    const int s = threadIdx.x;
-    if (s < maps.nsims) {
+  if (!SOLO && maps.ahead) {
+    for (int s = threadIdx.x; s < maps.nsims; s += NTI) {
 #pragma unroll
       for (int k = 0; k < MAP_KINDS; k++)
         if ((KINDS >> k) & 1u) box_fence(tmaps + (2 * s + buf) * MAP_KINDS + k);
@@ -443,7 +445,7 @@ __device__ __forceinline__ const TensorMapSlot *box_map(const BoxMaps &maps, con
                                                         int kind, const TensorMapSlot *&ready) {
   if (maps.nsims == 1) return &maps.m[kind];
   const TensorMapSlot *const m = tmaps + (2 * s + buf) * MAP_KINDS + kind;
-  if (maps.nsims > BOX_FENCE_AHEAD && m != ready) {
+  if (!maps.ahead && m != ready) {
     box_fence(m);
     ready = m;
   }

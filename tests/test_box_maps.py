@@ -1,8 +1,8 @@
 """Tensor maps of the step kernels' boxes: a map in global memory needs an
 acquire fence before a block's first use of it (the copy unit may hold what lay
 at its address before); a batch of one gets its maps as a kernel parameter, one of
-up to 128 fences them all at the start of a block, a larger one where a thread
-moves to a simulation.
+as many tiles as its simulations squared fences them all at the start of a block, any
+other where a thread moves to a simulation.
 
 The GPU tests put different maps at the same addresses one after the other.
 States are compared bit for bit.  Gradients: as in test_gpu_adjoint_ws.py.
@@ -35,9 +35,9 @@ def test_boxes_take_their_map_from_box_map():
     assert "fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" in body("void box_fence(")
     # the kernel parameter's map, else a fence ahead of the wait or here
     assert re.findall(r"return ([^;]*);", body("*box_map(")) == ["&maps.m[kind]", "m"]
-    assert re.search(r"if \(maps.nsims > BOX_FENCE_AHEAD && m != ready\) \{\s*box_fence\(m\);", body("*box_map("))
+    assert re.search(r"if \(!maps.ahead && m != ready\) \{\s*box_fence\(m\);", body("*box_map("))
     ahead = body("void box_begin(")
-    assert "maps.nsims > 1 && maps.nsims <= BOX_FENCE_AHEAD" in ahead
+    assert "if (!SOLO && maps.ahead) {" in ahead
     assert ahead.index("box_fence(") < ahead.index("__syncthreads();") < ahead.index("pdl_wait();")
     for kernel, kinds in (("kf_bulk", "1u << MAP_MU"), ("kf_general", "1u << MAP_ALL"),
                           ("kf_step", "1u << MAP_MU | 1u << MAP_ALL")):
@@ -99,7 +99,8 @@ def test_adjoint_in_one_block_on_several_grids(tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("prec,times", [("FP64", 1), ("FP32", 1), ("FP64", 64), ("FP32", 64), ("FP64", 65)])
+@pytest.mark.parametrize("prec,times", [("FP64", 1), ("FP32", 1), ("FP64", 12), ("FP32", 12), ("FP64", 64),
+                                        ("FP32", 64)])
 def test_batches_one_after_the_other(tmp_path, prec, times):
     """Batches of two grids (`times` of each), each in the memory that the one before gave back, and
     alone: a batch's simulations step as they do alone (maps from global memory
