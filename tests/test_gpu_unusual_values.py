@@ -133,6 +133,41 @@ def test_smooth_by_tile_kinds(tmp_path, system, plant):
     b.close()
 
 
+@pytest.mark.parametrize("system", ["three_aniso", "four_aniso_coupled", "four_iso", "two_aniso"])
+@pytest.mark.parametrize("plant", ["mu_inf", "mu_nan", "mu_huge"])
+def test_bulk_tiles(tmp_path, system, plant):
+    """Values in liquid far from any interface, inside the domain and at its edges:
+    fields, extremes and the two sweeps by tile kinds."""
+    kw, mesh = SYSTEMS[system], (160, 256)
+    ip, fp = write_case(str(tmp_path), "b", dict(kw, mesh=mesh, d_solid=0.0), seeds=[(0, 30, 40, 10.0)])
+    p = gp.load_params(ip)
+    phi, mu = gp.fill(p, fp)
+    values = PLANTS[plant][1]
+    for i, (x, y) in enumerate([(100, 200), (100, 120), (90, 40), (140, 223), (120, 160), (0, 150), (80, 255), (159, 90)]):
+        mu[i % mu.shape[0], x, y] = values[i % len(values)]
+    o = Oracle(p, recip_div=1)
+    o.set(phi, mu)
+    with gp.Simulation(p, phi, mu) as sim:
+        for n in range(2):
+            o.step(1)
+            try:
+                st = sim.step(1)
+            except gp.NonFiniteError as e:
+                st = e.stats
+            for what, a, b in zip(("phi", "mu"), sim.get(), o.get()):
+                assert _same(a, b), "%s after step %d: %s" % (what, n + 1, _diff(a, b))
+            ost = o.stats()
+            for k in ("phi_max", "phi_min", "mu_max", "mu_min"):
+                assert st[k] == ost[k], (k, n)
+    o.set(phi, mu)
+    o.smooth(2)
+    b = gp.Batch([p] * 4, [(phi, mu)] * 4, precision=gp.GP_FP64)
+    b.smooth(2)
+    for what, x, y in zip(("phi", "mu"), b.get(1), o.get()):
+        assert _same(x, y), "sweep, %s: %s" % (what, _diff(x, y))
+    b.close()
+
+
 @pytest.mark.parametrize("name", ["bin_iso_antitrap", "ternary3_aniso_periodic", "dilute_three_phase"])
 @pytest.mark.parametrize("dx", [3e-20, 5e20, 0.5 ** 64])
 def test_spacings_beyond_the_quick_range(tmp_path, name, dx):
