@@ -20,6 +20,7 @@ struct StepLaunch {
   cudaStream_t stream;
   int grid;
   bool mul, diag, tg;
+  bool ahead;                   /* the kernels may start while the one before them runs */
   const void *solo;
   const SimDesc *sims;
   const void *consts;
@@ -41,7 +42,7 @@ struct BatchLaunch {
   cudaError_t (*prepare)(const StepLaunch &l, int *bulk, int *general, int *step);
   /* the bulk and interface lists of a step; flag_out: the flags of the buffer it
    * writes (copied into the bulk entries) */
-  cudaError_t (*classify)(int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts, const int *tsim,
+  cudaError_t (*classify)(bool ahead, int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts, const int *tsim,
                           const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist, int4 *blist, int *ctr);
   cudaError_t (*bulk)(const StepLaunch &l);
   cudaError_t (*general)(const StepLaunch &l);
@@ -73,10 +74,11 @@ struct BatchLaunch {
   size_t elem;
 };
 
-/* A launch that may start while the kernel before it on the stream still runs: the
- * kernel waits by itself (pdl_begin) before it touches what that one writes. */
+/* A launch that may (ahead) start while the kernel before it on the stream still runs:
+ * the kernel waits by itself (pdl_begin) before it touches what that one writes. */
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, const A &...args) {
+cudaError_t launch_dependent(bool ahead, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                             const A &...args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)grid);
   c.blockDim = dim3((unsigned)block);
@@ -84,7 +86,7 @@ cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, 
   c.stream = s;
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = ahead ? 1 : 0;
   c.attrs = &at;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
@@ -156,7 +158,7 @@ struct BatchKernels {
   static cudaError_t step(const StepLaunch &l) {
     cudaError_t e = cudaSuccess;
     with_step(l, [&](auto k, const auto &args) {
-      e = launch_dependent(k, l.grid, NTI, step_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.blist,
+      e = launch_dependent(l.ahead, k, l.grid, NTI, step_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.blist,
                            l.glist, l.maps, l.tmaps, l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
     return e;
@@ -164,7 +166,7 @@ struct BatchKernels {
   static cudaError_t bulk(const StepLaunch &l) {
     cudaError_t e = cudaSuccess;
     with_bulk(l, l.st.want_sums != 0, [&](auto k) {
-      e = launch_dependent(k, l.grid, NTI, bulk_smem, l.stream, l.sims, (const Consts<R> *)l.consts, l.blist, l.maps, l.tmaps,
+      e = launch_dependent(l.ahead, k, l.grid, NTI, bulk_smem, l.stream, l.sims, (const Consts<R> *)l.consts, l.blist, l.maps, l.tmaps,
                            l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.ctr, l.ndone, l.st);
     });
     return e;
@@ -172,7 +174,7 @@ struct BatchKernels {
   static cudaError_t general(const StepLaunch &l) {
     cudaError_t e = cudaSuccess;
     with_general(l, [&](auto k, const auto &args) {
-      e = launch_dependent(k, l.grid, NTI, item_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.maps, l.tmaps,
+      e = launch_dependent(l.ahead, k, l.grid, NTI, item_smem, l.stream, args, l.sims, (const Consts<R> *)l.consts, l.maps, l.tmaps,
                            l.buf, (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.ctr, l.ndone, l.st);
     });
     return e;
@@ -204,10 +206,10 @@ struct BatchKernels {
     with_step(l, [&](auto k, const auto &) { set(k, step_smem, bs); });
     return e;
   }
-  static cudaError_t classify(int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts,
+  static cudaError_t classify(bool ahead, int ntiles, cudaStream_t s, const ClassifySim &solo, const SimDesc *sims, const void *consts,
                               const int *tsim, const TileFlags *flag_in, const TileFlags *flag_out, int4 *glist,
                               int4 *blist, int *ctr) {
-    return launch_dependent(kf_classify<R>, (ntiles + NTC - 1) / NTC, NTC, 0, s, solo, sims, (const Consts<R> *)consts,
+    return launch_dependent(ahead, kf_classify<R>, (ntiles + NTC - 1) / NTC, NTC, 0, s, solo, sims, (const Consts<R> *)consts,
                             tsim, ntiles, flag_in, flag_out, glist, blist, ctr);
   }
   static cudaError_t flags(int ntiles, cudaStream_t s, const SimDesc *sims, const int *tsim, const void *state,
@@ -218,7 +220,7 @@ struct BatchKernels {
   static cudaError_t sweep(const StepLaunch &l, int *blocks) {
     if constexpr (sizeof(R) == 8) {
       if (blocks) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, ks_tiles<R, N, K, A>, NT, 0);
-      return launch_dependent(ks_tiles<R, N, K, A>, l.grid, NT, 0, l.stream, l.sims, (const Consts<R> *)l.consts,
+      return launch_dependent(l.ahead, ks_tiles<R, N, K, A>, l.grid, NT, 0, l.stream, l.sims, (const Consts<R> *)l.consts,
                               (const R *)l.state, (R *)l.next, l.flag_out, l.glist, l.st.trows, l.ctr, l.ndone);
     } else {
       return cudaErrorNotSupported;

@@ -357,6 +357,16 @@ static int bfail(gp_batch *b, int code, const char *fmt, ...) {
     if (e_ != cudaSuccess) return bfail(b, GP_ECUDA, "%s: %s", #call, cudaGetErrorString(e_));  \
   } while (0)
 
+/* From this many tiles the steps of a batch of one are ordinary launches inside a
+ * graph.  Starting ahead hides a graph's launch gap, which counts in a short step; in
+ * a longer one the waiting CTAs take room from the running ones.  us per 200 steps and
+ * their transfers, ahead / ordinary: binary 128^2 4605 / 4945, 256^2 5066 / 5207, 512^2
+ * (1024 tiles) 5627 / 5783, 1024^2 (4096) 5926 / 5986 and with 8 larger seeds 6550 /
+ * 6300, 2048^2 12526 / 12338; ternary three-phase 256^2 6647 / 6738, 512^2 7578 / 7480,
+ * 1024^2 10627 / 10100, 4096^2 87360 / 86910.  Outside a graph and in batches of several
+ * (whose fences it hides) they always start ahead. */
+static constexpr int GP_PLAIN_TILES = 4096;
+
 /* What the kernels of the next step (or sweep) from the current buffer are launched with. */
 static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   gpd::StepLaunch l;
@@ -378,6 +388,9 @@ static gpd::StepLaunch batch_launch_args(gp_batch *b, int want_sums) {
   st.bch_div = b->shape.bch_div;
   const int in = b->cur, out = b->cur ^ 1;
   l.stream = b->stream;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (b->nsims == 1 && b->ntiles >= GP_PLAIN_TILES) cudaStreamIsCapturing(b->stream, &capture);
+  l.ahead = capture == cudaStreamCaptureStatusNone;
   l.mul = b->mul;
   l.diag = b->diag;
   l.tg = b->tgrad;
@@ -406,7 +419,7 @@ static int batch_step_once(gp_batch *b, int want_sums, cudaEvent_t *ev) {
   const int in = b->cur, out = b->cur ^ 1;
   if (ev) BK(cudaEventRecord(ev[0], b->stream));
   if (b->tgrad) BK(b->L.trows(b->nsims, b->stream, b->d_desc, b->d_consts, b->counters, b->dyn, b->trows));
-  BK(b->L.classify(b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
+  BK(b->L.classify(l.ahead, b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[in],
                    b->redir_in ? b->redir_have : b->flags[out], b->glist, b->blist, b->counters));
   if (!want_sums && b->grid_s > 0 && b->shape.fused && (!ev || ev[3] == nullptr)) {
     /* one launch for both kinds of tile; ev (with ev[3] null): events after
@@ -1247,7 +1260,7 @@ int gp_batch_smooth(gp_batch *b, long nsteps) {
       l.st.ext = nullptr;   /* the sweeps keep no progress record */
       l.st.sweep = 1;
       l.ndone = b->grid_b + b->grid_w;
-      BK(b->L.classify(b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[b->cur], b->flags[b->cur ^ 1],
+      BK(b->L.classify(l.ahead, b->ntiles, b->stream, b->csim, b->d_desc, b->d_consts, b->d_tsim, b->flags[b->cur], b->flags[b->cur ^ 1],
                        b->glist, b->blist, b->counters));
       l.grid = b->grid_b;
       BK(b->L.bulk(l));

@@ -64,7 +64,7 @@ def _dependent(funcs):
 
 def test_every_dependent_launch_waits():
     src = _sources()["gp_batch_impl.cuh"]
-    launched = set(re.findall(r"launch_dependent\((k\w+)<", src)) | set(re.findall(r"\bf\((k\w+)<", src))
+    launched = set(re.findall(r"launch_dependent\([\w.]+, (k\w+)<", src)) | set(re.findall(r"\bf\((k\w+)<", src))
     kernels, _ = _dependent(_all())
     assert {"kf_classify", "kf_bulk", "kf_general", "kf_step", "ks_tiles"} == launched == kernels
 
