@@ -245,8 +245,8 @@ enum { CTR_LIST = 0, CTR_HEAD = 1, CTR_DONE = 2, CTR_STEP = 3, CTR_BULK = 4, CTR
 /* Programmatic dependent launch: the kernels of a step are launched while their
  * predecessor still runs (every one of its CTAs has started) and wait here, before
  * they read anything it writes (with ld_step only), until it has completed.  A launch gap of a graph
- * is about 1 us; a step has two.  Graph time of a step, before and after: 256^2 20.7
- * to 18.4 us, 1024^2 34.0 to 30.7; large grids within 2 % (2048^2 119.7 to 121.6). */
+ * is about 1 us; a step has two.  Large single grids lose by it and launch in order
+ * (GP_PLAIN_TILES, gp_device.cu, has both sides' times); the wait is then no wait. */
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
